@@ -79,6 +79,90 @@ __device__ __forceinline__ f3 project(const Mat4& M, f3 p) {
   return mk3(x * 0.5f + 0.5f, y * 0.5f + 0.5f, z);
 }
 
+// ---- Packed pairs of fp32 values --------------------------------------------
+// p2: two fp32 values (lo, hi) in one 64-bit register pair; an operation is one
+// instruction (f32x2) and rounds each half as the scalar instruction does, so a
+// kernel bound by issue slots gets two results a slot with the same bits (measured
+// on a chain of fused multiply-adds: half the instructions, the same pipe time; a
+// scalar operand in both halves costs nothing).  ptxas contracts mul.rn.f32x2 into
+// a following add or sub even where scalar contraction is off, which would round
+// once instead of twice; pmul is therefore the fused form with an addend of -0 read
+// from constant memory (a * b + -0 is a * b rounded, the sign of zero included).
+struct p2 {
+  unsigned long long v;
+};
+__constant__ unsigned long long kNegZero2 = 0x8000000080000000ull;
+
+__device__ __forceinline__ p2 pk(float lo, float hi) {
+  p2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ p2 pk(float s) { return pk(s, s); }
+__device__ __forceinline__ p2 pk(float2 v) { return pk(v.x, v.y); }
+__device__ __forceinline__ float lo_(p2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return x;
+}
+__device__ __forceinline__ float hi_(p2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return y;
+}
+__device__ __forceinline__ p2 padd(p2 a, p2 b) {
+  p2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ p2 psub(p2 a, p2 b) {
+  p2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ p2 pfma(p2 a, p2 b, p2 c) {
+  p2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ p2 pmul(p2 a, p2 b) { return pfma(a, b, p2{kNegZero2}); }
+// a0 * b0 + a1 * b1 + a2 * b2 of both halves, left to right, each operation rounded.
+__device__ __forceinline__ p2 pdot3(p2 a0, p2 b0, p2 a1, p2 b1, p2 a2, p2 b2) {
+  return padd(padd(pmul(a0, b0), pmul(a1, b1)), pmul(a2, b2));
+}
+
+// A 3-vector with x and y packed; the same operations in the same order as f3's.
+struct v3 {
+  p2 xy;
+  float z;
+};
+__device__ __forceinline__ v3 mkv3(float x, float y, float z) { return v3{pk(x, y), z}; }
+__device__ __forceinline__ f3 unpack3(v3 a) { return mk3(lo_(a.xy), hi_(a.xy), a.z); }
+__device__ __forceinline__ v3 add3(v3 a, v3 b) { return v3{padd(a.xy, b.xy), a.z + b.z}; }
+__device__ __forceinline__ v3 sub3(v3 a, v3 b) { return v3{psub(a.xy, b.xy), a.z - b.z}; }
+__device__ __forceinline__ v3 mul3s(v3 a, float s) { return v3{pmul(a.xy, pk(s)), a.z * s}; }
+__device__ __forceinline__ float dot3(v3 a, v3 b) {
+  const p2 m = pmul(a.xy, b.xy);
+  return lo_(m) + hi_(m) + a.z * b.z;
+}
+__device__ __forceinline__ v3 normalize3(v3 v) { return mul3s(v, rcp_(sqrtf(dot3(v, v)))); }
+
+// A point from its homogeneous rows (x, y) and (z, w).
+__device__ __forceinline__ v3 from_rows(p2 xy, p2 zw) {
+  const float r = rcp_(hi_(zw));
+  return v3{pmul(xy, pk(r)), lo_(zw) * r};
+}
+// unproject (above) with its matrix rows in pairs.
+__device__ __forceinline__ v3 unproject_p(const Mat4& M, float sx, float sy, float sz) {
+  const p2 t = pfma(pk(sx, sy), pk(2.0f), pk(-1.0f));  // the doubling is exact: one rounding as before
+  const p2 X = pk(lo_(t)), Y = pk(hi_(t)), Z = pk(sz);
+  const p2 xy = padd(padd(pmul(pk(M.m[0], M.m[1]), X), pmul(pk(M.m[4], M.m[5]), Y)),
+                     padd(pmul(pk(M.m[8], M.m[9]), Z), pk(M.m[12], M.m[13])));
+  const p2 zw = padd(padd(pmul(pk(M.m[2], M.m[3]), X), pmul(pk(M.m[6], M.m[7]), Y)),
+                     padd(pmul(pk(M.m[10], M.m[11]), Z), pk(M.m[14], M.m[15])));
+  return from_rows(xy, zw);
+}
+
 // ---- Fast evaluation (march precision GI_MARCH_FAST) ----------------------
 // Explicit fused multiply-adds, the hardware reciprocal square root and
 // reciprocal, and a fitted atan, used only inside the fast march's step loop;
@@ -102,14 +186,26 @@ __device__ __forceinline__ f3 funproject(const Mat4& inv, float sx, float sy, fl
   const float r = __fdividef(1.0f, v.w);
   return mk3(v.x * r, v.y * r, v.z * r);
 }
+// The hardware's approximate division and reciprocal square root without the
+// scaling that subnormal operands would need.
+__device__ __forceinline__ float div_approx(float a, float b) {
+  float r;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float a) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
 // atan2 by octant reduction to t = min(|x|,|y|) / max(|x|,|y|) in [0, 1] and
 // atan(t) = t P(t^2), P of degree 8 fitted to atan(t)/t by iteratively reweighted
 // least squares on 6000 Chebyshev nodes of [0, 1] (max error 9.4e-8 rad in fp32,
 // about one ulp of the result; the quotient's approximate division adds ~2 ulp).
 __device__ __forceinline__ float fast_atan2(float y, float x) {
   const float ax = fabsf(x), ay = fabsf(y);
-  const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-  const float t = mx > 0.0f ? __fdividef(mn, mx) : 0.0f;
+  const float mx = fmaxf(fmaxf(ax, ay), 1e-37f), mn = fminf(ax, ay);  // (0, 0): t = 0
+  const float t = div_approx(mn, mx);
   const float z = t * t;
   float p = 0.0024567246437072754f;
   p = fmaf(p, z, -0.014401359483599663f);
@@ -139,6 +235,24 @@ __device__ __forceinline__ void lin_setup_f(float s, float fw, int w, int& i0, i
 
 __device__ __forceinline__ void lin_setup(float s, int w, int& i0, int& i1, float& a) {
   lin_setup_f(s, (float)w, w, i0, i1, a);
+}
+
+// atan2f_ (gi_math.h), the same bits, with its octant reduction as selects and its
+// special cases (both arguments infinite, or NaN) in one cold branch.
+__device__ __forceinline__ float march_atan2(float y, float x) {
+  const float ax = fabsf(x), ay = fabsf(y);
+  const float num = fminf(ax, ay), den = fmaxf(ax, ay);
+  if (!(num < kInf)) return atan2f_(y, x);
+  float t = den == 0.0f ? 0.0f : num * rcp_(den);
+  float base = 0.0f;
+  if (t > kTanPiO12) {
+    t = div_(t * kSqrt3 - 1.0f, t + kSqrt3);
+    base = kPiO6;
+  }
+  float a = base + atan_core(t);
+  if (ay > ax) a = kPiO2 - a;
+  if (signbit_(x)) a = kPi - a;
+  return copysign_(a, y);
 }
 
 struct Bilin {

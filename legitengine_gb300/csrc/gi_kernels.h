@@ -56,6 +56,9 @@ struct MarchArgs {
   int soft;                           // 1: depth-variance horizon (exact contract, standard form, 2-ch depth)
   float ray[12];                      // fast step loop's view-ray basis (set_ray_basis)
   float ray_q[6];                     // |U|^2 of that ray as a quadratic form in (sx, sy) (set_ray_basis)
+  float cam[3];                       // eye position: inv_view * (0, 0, 0, 1) (set_ray_basis)
+  float inv_size[2];                  // rcp_ of width and height (set_ray_basis)
+  float far_col[4];                   // inv_view_proj * (0, 0, 1, 1): an unprojection's terms at depth 1 (set_ray_basis)
   // Recorded geometry of a march (standard form): per pixel and direction the
   // steps that raised the horizon, their horizon contributions and the initial
   // term -- all independent of the light pyramid -- so that a later bounce over
@@ -109,7 +112,7 @@ int launch_march(const MarchArgs& a, cudaStream_t stream);
 // Bytes of the three record arrays of a march of this shape (0 if it cannot record:
 // a table of more than 64 steps).
 size_t march_record_bytes(const MarchArgs& a, size_t* hc_bytes, size_t* mask_bytes, size_t* hc0_bytes);
-void set_ray_basis(MarchArgs& a);  // fills a.ray from a.inv_view_proj and a.inv_view
+void set_ray_basis(MarchArgs& a);  // fills a.ray, ray_q, cam, inv_size and far_col from a.inv_view_proj and a.inv_view
 int autotune_march(const MarchArgs& a, cudaStream_t stream, int* best_rows, int* best_rays_per_warp,
                    float* best_ms);
 int march_table_size(const MarchArgs& a);

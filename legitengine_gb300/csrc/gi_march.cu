@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -30,17 +31,33 @@ using namespace dev;
 
 constexpr int kMarchTx = kMarchTileSubX;  // sub-image pixels per warp row
 constexpr int kMarchTy = kMarchTileSubY;  // warps per CTA
+constexpr int kSplit = 4;               // direction split: threads per pixel
+constexpr int kSplitMaxDirs = 32;
+constexpr int kSplitMinDirs = 4;
 constexpr float kPiRef = 3.1415f;  // indirectLighting.frag:169
 
-struct StepEntry {
-  float off;    // pixel offset of the step (:217)
-  float delta;  // trilinear blend weight of the upper level
-  int lo;       // mip level read first (Vulkan mipmap LINEAR selection)
-  union {
-    int hi;       // software taps: the second level read
-    float level;  // texture taps: lo + delta, the fetch's level of detail
-  };
+// A step of a pattern's table.  Software taps: everything of the two levels the
+// step's trilinear taps read that does not depend on the pixel, as pairs (the level
+// read first, the second one), so that a step takes four 16-byte shared-memory reads
+// instead of shifts, conversions and constant-bank reads, and packed arithmetic
+// works on both levels at once.
+struct __align__(16) TapStep {
+  float off;               // pixel offset of the step (:217)
+  float delta;             // trilinear blend weight of the second level
+  int w1, h1;              // second level's size
+  float fw0, fw1, fh0, fh1;  // both levels' sizes as floats
+  const float* img0;       // both levels' texels: depth moments (march) or light (replay)
+  const float* img1;
+  int w0, h0;              // first level's size (Vulkan mipmap LINEAR selection)
+  int lo, hi;              // the levels
 };
+// Texture taps: the fetch's level of detail is all.
+struct TexStep {
+  float off;
+  float level;
+};
+template <bool TEX> struct StepOf { using T = TapStep; };
+template <> struct StepOf<true> { using T = TexStep; };
 
 __device__ __forceinline__ void hammersley(int i, int n, float& ax, float& ay) {
   uint32_t b = ((uint32_t)i << 16u) | ((uint32_t)i >> 16u);
@@ -52,29 +69,120 @@ __device__ __forceinline__ void hammersley(int i, int n, float& ax, float& ay) {
   ay = div_((float)b, 4294967296.0f);  // float(0xffffffffu)
 }
 
+// Depth of texel idx (the .x of a moments pair).
 template <int DCH> __device__ __forceinline__ float depth_texel(const float* p, int idx) {
-  if (DCH == 2) return __ldg(reinterpret_cast<const float2*>(p) + idx).x;
-  return __ldg(p + idx);
+  return __ldg(p + (size_t)(unsigned)idx * DCH);
 }
 
-template <int DCH> __device__ __forceinline__ float depth_bilin(const float* p, const Bilin& B) {
-  return blend1(B, depth_texel<DCH>(p, B.o00), depth_texel<DCH>(p, B.o10), depth_texel<DCH>(p, B.o01),
-                depth_texel<DCH>(p, B.o11));
+// Bilinear footprints of a step's taps on its two levels (entry 0 the level read
+// first; entry 1 unset when the step reads one level): texel indices and weights.
+// Sample coordinates lie within a few viewports of the image, so the texel
+// coordinate fits an int and an index's + 1 and both clamps are one instruction
+// (the min/max of lin_setup_f with the same result).
+struct TapFoot {
+  int o00[2], o10[2], o01[2], o11[2];
+  float w00[2], w10[2], w01[2], w11[2];
+};
+
+__device__ __forceinline__ void tap_index(TapFoot& t, int k, float fx, float fy, int w, int h) {
+  const int i = (int)fx, j = (int)fy;
+  const int i0 = __vimin_s32_relu(i, w - 1), i1 = __viaddmin_s32_relu(i, 1, w - 1);
+  const int j0 = __vimin_s32_relu(j, h - 1), j1 = __viaddmin_s32_relu(j, 1, h - 1);
+  t.o00[k] = j0 * w + i0;
+  t.o10[k] = j0 * w + i1;
+  t.o01[k] = j1 * w + i0;
+  t.o11[k] = j1 * w + i1;
 }
 
-__device__ __forceinline__ f3 light_bilin(const float* p, const Bilin& B) {
-  float4 a = ld4(p, B.o00), b = ld4(p, B.o10), c = ld4(p, B.o01), d = ld4(p, B.o11);
-  f3 r;
-  r.x = a.x * B.w00 + b.x * B.w10 + c.x * B.w01 + d.x * B.w11;
-  r.y = a.y * B.w00 + b.y * B.w10 + c.y * B.w01 + d.y * B.w11;
-  r.z = a.z * B.w00 + b.z * B.w10 + c.z * B.w01 + d.z * B.w11;
+// The footprint on the first level alone.
+__device__ __forceinline__ void tap_foot1(const TapStep& e, float sx, float sy, TapFoot& t) {
+  const p2 u = psub(pmul(pk(sx, sy), pk(e.fw0, e.fh0)), pk(0.5f));
+  const float fx = floorf(lo_(u)), fy = floorf(hi_(u));
+  const p2 ab = psub(u, pk(fx, fy)), oab = psub(pk(1.0f), ab);
+  const float a = lo_(ab), b = hi_(ab), oa = lo_(oab), ob = hi_(oab);
+  t.w00[0] = oa * ob;
+  t.w10[0] = a * ob;
+  t.w01[0] = oa * b;
+  t.w11[0] = a * b;
+  tap_index(t, 0, fx, fy, e.w0, e.h0);
+}
+
+// The footprints on both levels, a level in each half of the packed operations.
+__device__ __forceinline__ void tap_foot2(const TapStep& e, float sx, float sy, TapFoot& t) {
+  const p2 u = psub(pmul(pk(sx), pk(e.fw0, e.fw1)), pk(0.5f));
+  const p2 v = psub(pmul(pk(sy), pk(e.fh0, e.fh1)), pk(0.5f));
+  const float fx0 = floorf(lo_(u)), fx1 = floorf(hi_(u)), fy0 = floorf(lo_(v)), fy1 = floorf(hi_(v));
+  const p2 a = psub(u, pk(fx0, fx1)), b = psub(v, pk(fy0, fy1));
+  const p2 oa = psub(pk(1.0f), a), ob = psub(pk(1.0f), b);
+  const p2 w00 = pmul(oa, ob), w10 = pmul(a, ob), w01 = pmul(oa, b), w11 = pmul(a, b);
+  t.w00[0] = lo_(w00); t.w00[1] = hi_(w00);
+  t.w10[0] = lo_(w10); t.w10[1] = hi_(w10);
+  t.w01[0] = lo_(w01); t.w01[1] = hi_(w01);
+  t.w11[0] = lo_(w11); t.w11[1] = hi_(w11);
+  tap_index(t, 0, fx0, fy0, e.w0, e.h0);
+  tap_index(t, 1, fx1, fy1, e.w1, e.h1);
+}
+
+// Trilinear depth of a step: the restatement's order, or fused (FAST).
+template <int DCH, bool FAST>
+__device__ __forceinline__ float depth_tap(const TapStep& e, bool two, const TapFoot& t) {
+  const float a00 = depth_texel<DCH>(e.img0, t.o00[0]), a10 = depth_texel<DCH>(e.img0, t.o10[0]);
+  const float a01 = depth_texel<DCH>(e.img0, t.o01[0]), a11 = depth_texel<DCH>(e.img0, t.o11[0]);
+  if (!two) {
+    if (FAST) return fmaf(a11, t.w11[0], fmaf(a01, t.w01[0], fmaf(a10, t.w10[0], a00 * t.w00[0])));
+    return a00 * t.w00[0] + a10 * t.w10[0] + a01 * t.w01[0] + a11 * t.w11[0];
+  }
+  const p2 v00 = pk(a00, depth_texel<DCH>(e.img1, t.o00[1])), v10 = pk(a10, depth_texel<DCH>(e.img1, t.o10[1]));
+  const p2 v01 = pk(a01, depth_texel<DCH>(e.img1, t.o01[1])), v11 = pk(a11, depth_texel<DCH>(e.img1, t.o11[1]));
+  const p2 w00 = pk(t.w00[0], t.w00[1]), w10 = pk(t.w10[0], t.w10[1]);
+  const p2 w01 = pk(t.w01[0], t.w01[1]), w11 = pk(t.w11[0], t.w11[1]);
+  if (FAST) {
+    const p2 d = pfma(v11, w11, pfma(v01, w01, pfma(v10, w10, pmul(v00, w00))));
+    return fmaf(hi_(d) - lo_(d), e.delta, lo_(d));
+  }
+  const p2 d = padd(padd(padd(pmul(v00, w00), pmul(v10, w10)), pmul(v01, w01)), pmul(v11, w11));
+  return lo_(d) * (1.0f - e.delta) + hi_(d) * e.delta;
+}
+
+// Both depth moments (E[d], E[d^2]) of level k's bilinear tap, same weights and order as depth_tap.
+__device__ __forceinline__ float2 moments_bilin(const float* p, const TapFoot& t, int k) {
+  const float2 t00 = ld2(p, t.o00[k]), t10 = ld2(p, t.o10[k]), t01 = ld2(p, t.o01[k]), t11 = ld2(p, t.o11[k]);
+  return make_float2(t00.x * t.w00[k] + t10.x * t.w10[k] + t01.x * t.w01[k] + t11.x * t.w11[k],
+                     t00.y * t.w00[k] + t10.y * t.w10[k] + t01.y * t.w01[k] + t11.y * t.w11[k]);
+}
+
+// cos 2h and sin 2h of h = atan2(y, x) by the double-angle identities (fast precision).
+__device__ __forceinline__ void double_angle(float x, float y, float& c, float& s) {
+  c = 1.0f;
+  s = 0.0f;
+  const float r2 = fmaf(x, x, y * y);
+  if (r2 >= 1.17549435e-38f) {
+    const float ir = div_approx(1.0f, r2);
+    c = (x - y) * (x + y) * ir;
+    s = 2.0f * x * y * ir;
+  }
+}
+
+// A light value, red and green packed.
+struct Light {
+  p2 rg;
+  float b;
+};
+
+// Bilinear light of level k's footprint: the restatement's order, or fused (FAST).
+template <bool FAST> __device__ __forceinline__ Light light_bilin(const float* p, const TapFoot& t, int k) {
+  const float4 a = ld4(p, t.o00[k]), b = ld4(p, t.o10[k]), c = ld4(p, t.o01[k]), d = ld4(p, t.o11[k]);
+  const p2 ra = pk(a.x, a.y), rb = pk(b.x, b.y), rc = pk(c.x, c.y), rd = pk(d.x, d.y);
+  const p2 w00 = pk(t.w00[k]), w10 = pk(t.w10[k]), w01 = pk(t.w01[k]), w11 = pk(t.w11[k]);
+  Light r;
+  if (FAST) {
+    r.rg = pfma(rd, w11, pfma(rc, w01, pfma(rb, w10, pmul(ra, w00))));
+    r.b = fmaf(d.z, t.w11[k], fmaf(c.z, t.w01[k], fmaf(b.z, t.w10[k], a.z * t.w00[k])));
+  } else {
+    r.rg = padd(padd(padd(pmul(ra, w00), pmul(rb, w10)), pmul(rc, w01)), pmul(rd, w11));
+    r.b = a.z * t.w00[k] + b.z * t.w10[k] + c.z * t.w01[k] + d.z * t.w11[k];
+  }
   return r;
-}
-
-// Both depth moments (E[d], E[d^2]) of a bilinear tap, same weights and order as depth_bilin.
-__device__ __forceinline__ float2 moments_bilin(const float* p, const Bilin& B) {
-  const float2 t00 = ld2(p, B.o00), t10 = ld2(p, B.o10), t01 = ld2(p, B.o01), t11 = ld2(p, B.o11);
-  return make_float2(blend1(B, t00.x, t10.x, t01.x, t11.x), blend1(B, t00.y, t10.y, t01.y, t11.y));
 }
 
 // Soft-occlusion horizon: the angle a step lowers the horizon to when the
@@ -100,53 +208,44 @@ __device__ __forceinline__ float soft_horizon(float dmean, float dsq, f3 rn, f3 
   return max_h - (d * cdf + sigma * pdf);
 }
 
-// Fused-multiply-add forms of the two taps for the fast step loop.
-template <int DCH> __device__ __forceinline__ float depth_bilin_fast(const float* p, const Bilin& B) {
-  return fmaf(depth_texel<DCH>(p, B.o11), B.w11,
-              fmaf(depth_texel<DCH>(p, B.o01), B.w01,
-                   fmaf(depth_texel<DCH>(p, B.o10), B.w10, depth_texel<DCH>(p, B.o00) * B.w00)));
-}
-
-__device__ __forceinline__ f3 light_bilin_fast(const float* p, const Bilin& B) {
-  const float4 a = ld4(p, B.o00), b = ld4(p, B.o10), c = ld4(p, B.o01), d = ld4(p, B.o11);
-  return mk3(fmaf(d.x, B.w11, fmaf(c.x, B.w01, fmaf(b.x, B.w10, a.x * B.w00))),
-             fmaf(d.y, B.w11, fmaf(c.y, B.w01, fmaf(b.y, B.w10, a.y * B.w00))),
-             fmaf(d.z, B.w11, fmaf(c.z, B.w01, fmaf(b.z, B.w10, a.z * B.w00))));
-}
-
 // Shared-memory tables of one CTA-tile: n_tab steps, R directions and the
 // levels' sizes (float(width >> l), float(height >> l)), laid out in that order
 // in march_smem_bytes(n_tab, R) bytes.  The single-view kernels take exactly that
 // as dynamic shared memory, so the unified L1/shared storage left to L1 does not
 // shrink for the tables' maxima (GI_MAX_STEPS steps, GI_MAX_DIRS directions: 10 KB
 // a CTA, against 0.6 KB for 22 steps and 16 directions).
-struct MarchSmem {
-  StepEntry* step;
-  float2* dir;
-  float2* lsize;
+template <bool TEX> struct MarchSmem {
+  typename StepOf<TEX>::T* step;
+  float4* dir;  // cos, sin and their reciprocals (rcp_)
 };
 
-__host__ __device__ constexpr int march_smem_bytes(int n_tab, int dirs) {
-  return n_tab * (int)sizeof(StepEntry) + dirs * (int)sizeof(float2) + GI_MAX_LEVELS * (int)sizeof(float2);
+// Entries of a step table: the texture loop fetches one step ahead, so its table
+// repeats the last entry (and is a whole number of 16-byte units).
+template <bool TEX> __host__ __device__ constexpr int padded_steps(int n_tab) { return TEX ? (n_tab + 2) & ~1 : n_tab; }
+
+template <bool TEX> __host__ __device__ constexpr int march_smem_bytes(int n_tab, int dirs) {
+  return padded_steps<TEX>(n_tab) * (int)sizeof(typename StepOf<TEX>::T) + dirs * (int)sizeof(float4);
 }
-constexpr int kMarchSmemMax = march_smem_bytes(GI_MAX_STEPS, GI_MAX_DIRS);
+// Without opting in to more, a launch may take 48 KB: the API's maxima fit beside the
+// direction split's terms.
+static_assert(march_smem_bytes<false>(GI_MAX_STEPS, GI_MAX_DIRS) <= 47 * 1024 &&
+                  march_smem_bytes<false>(GI_MAX_STEPS, kSplitMaxDirs) + kSplitMaxDirs * kMarchTx * 12 <= 47 * 1024,
+              "march tables");
 
 // The replay's tables: a record holds at most 64 steps (its step mask), so the
-// replay keeps fixed-size tables for that many (3.2 KB) -- constant offsets in its
+// replay keeps fixed-size tables for that many (6 KB) -- constant offsets in its
 // per-hit table reads, which the pointer layout above cost it 3 %.
 constexpr int kRecMaxSteps = 64;
 struct ReplaySmem {
-  StepEntry step[kRecMaxSteps];
-  float2 dir[GI_MAX_DIRS];
-  float2 lsize[GI_MAX_LEVELS];
+  TapStep step[kRecMaxSteps];
+  float4 dir[GI_MAX_DIRS];
 };
 
-// The tables' places in `base` (16-byte aligned, march_smem_bytes(n_tab, dirs) bytes).
-__device__ __forceinline__ MarchSmem march_smem(unsigned char* base, int n_tab, int dirs) {
-  MarchSmem m;
-  m.step = reinterpret_cast<StepEntry*>(base);
-  m.dir = reinterpret_cast<float2*>(base + n_tab * sizeof(StepEntry));
-  m.lsize = m.dir + dirs;
+// The tables' places in `base` (16-byte aligned, march_smem_bytes<TEX>(n_tab, dirs) bytes).
+template <bool TEX> __device__ __forceinline__ MarchSmem<TEX> march_smem(unsigned char* base, int n_tab) {
+  MarchSmem<TEX> m;
+  m.step = reinterpret_cast<typename StepOf<TEX>::T*>(base);
+  m.dir = reinterpret_cast<float4*>(base + padded_steps<TEX>(n_tab) * sizeof(typename StepOf<TEX>::T));
   return m;
 }
 
@@ -157,53 +256,58 @@ __host__ __device__ __forceinline__ size_t record_pixels(const MarchArgs& a) {
 }
 
 // The light term of a hit (:254-264): the trilinear light tap at the step's
-// footprint, then dl += (light - ambient) * hc, in the order of the restatement
-// (exact) or as fused multiply-adds (fast).  Shared by the march and the replay.
+// footprint (img0, img1: the light pyramid's two levels), then dl += (light -
+// ambient) * hc, in the order of the restatement (exact) or as fused multiply-adds
+// (fast), red and green packed.  Shared by the march and the replay.
 template <bool FAST>
-__device__ __forceinline__ void add_light(const MarchArgs& a, const StepEntry& e, const Bilin& blo,
-                                          const Bilin& bhi, bool two, float hc, float ambient, f3& dl) {
+__device__ __forceinline__ void add_light(const float* img0, const float* img1, float delta, const TapFoot& t,
+                                          bool two, float hc, float ambient, Light& dl) {
+  Light ls = light_bilin<FAST>(img0, t, 0);
   if (FAST) {
-    f3 ls = light_bilin_fast(a.light[e.lo], blo);
     if (two) {
-      const f3 lh = light_bilin_fast(a.light[e.hi], bhi);
-      ls = mk3(fmaf(lh.x - ls.x, e.delta, ls.x), fmaf(lh.y - ls.y, e.delta, ls.y), fmaf(lh.z - ls.z, e.delta, ls.z));
+      const Light lh = light_bilin<FAST>(img1, t, 1);
+      ls.rg = pfma(psub(lh.rg, ls.rg), pk(delta), ls.rg);
+      ls.b = fmaf(lh.b - ls.b, delta, ls.b);
     }
-    dl = mk3(fmaf(ls.x - ambient, hc, dl.x), fmaf(ls.y - ambient, hc, dl.y), fmaf(ls.z - ambient, hc, dl.z));
+    dl.rg = pfma(psub(ls.rg, pk(ambient)), pk(hc), dl.rg);
+    dl.b = fmaf(ls.b - ambient, hc, dl.b);
   } else {
-    f3 ls = light_bilin(a.light[e.lo], blo);
     if (two) {
-      f3 lh = light_bilin(a.light[e.hi], bhi);
-      ls.x = ls.x * (1.0f - e.delta) + lh.x * e.delta;
-      ls.y = ls.y * (1.0f - e.delta) + lh.y * e.delta;
-      ls.z = ls.z * (1.0f - e.delta) + lh.z * e.delta;
+      const Light lh = light_bilin<FAST>(img1, t, 1);
+      ls.rg = padd(pmul(ls.rg, pk(1.0f - delta)), pmul(lh.rg, pk(delta)));
+      ls.b = ls.b * (1.0f - delta) + lh.b * delta;
     }
-    dl.x = dl.x + ls.x * hc;
-    dl.y = dl.y + ls.y * hc;
-    dl.z = dl.z + ls.z * hc;
-    dl.x = dl.x - ambient * hc;
-    dl.y = dl.y - ambient * hc;
-    dl.z = dl.z - ambient * hc;
+    const float ah = ambient * hc;
+    dl.rg = psub(padd(dl.rg, pmul(ls.rg, pk(hc))), pk(ah));
+    dl.b = dl.b + ls.b * hc;
+    dl.b = dl.b - ah;
   }
 }
 
-// Texture-unit taps (MarchArgs::depth_tex / light_tex): one trilinear fetch at
-// level lo + delta of the step -- the sampler of the reference's textureLod with
-// linear filtering and linear mipmapping, evaluated by the texture units (8-bit
-// sub-texel and level weights) instead of in software.
-__device__ __forceinline__ float tex_level(const StepEntry& e) { return e.level; }
+// Texture-unit taps (MarchArgs::depth_tex / light_tex): one trilinear fetch at the
+// step's level of detail -- the sampler of the reference's textureLod with linear
+// filtering and linear mipmapping, evaluated by the texture units (8-bit sub-texel
+// and level weights) instead of in software.  A hit's fetched light l with its
+// horizon contribution in l.w:
+__device__ __forceinline__ void add_lit(const float4& l, float ambient, Light& dl) {
+  dl.rg = pfma(psub(pk(l.x, l.y), pk(ambient)), pk(l.w), dl.rg);
+  dl.b = fmaf(l.z - ambient, l.w, dl.b);
+}
 
-__device__ __forceinline__ void add_light_tex(const MarchArgs& a, float sx, float sy, float level, float hc,
-                                              float ambient, f3& dl) {
-  const float4 l = tex2DLod<float4>(a.light_tex, sx, sy, level);
-  dl = mk3(fmaf(l.x - ambient, hc, dl.x), fmaf(l.y - ambient, hc, dl.y), fmaf(l.z - ambient, hc, dl.z));
+// sum += 2 dl / R (:269), each operation rounded.
+__device__ __forceinline__ void add_term(Light& sum, const Light& dl, float rR) {
+  sum.rg = padd(sum.rg, pmul(pmul(pk(2.0f), dl.rg), pk(rR)));
+  sum.b = sum.b + 2.0f * dl.b * rR;
 }
 
 // Per-pattern tables of a CTA-tile: the same values as evaluating :170-177,
 // :212, :217, :234-235 per pixel.  Every thread of the CTA calls it; the caller
 // synchronises before use.
-template <bool TEX = false, class Smem>
-__device__ __forceinline__ void march_tables(const MarchArgs& a, int n_tab, int pat, Smem& sm, int tid,
-                                             int nthreads) {
+// `img`: the pyramid the software taps' entries point into (`ch` floats a texel).
+template <class Smem>
+__device__ __forceinline__ void march_tables(const MarchArgs& a, const float* const* img, int n_tab, int pat, Smem& sm,
+                                             int tid, int nthreads) {
+  using Step = std::remove_reference_t<decltype(sm.step[0])>;
   const int P = a.pattern;
   const int R = a.dirs;
   const int SR = a.step_dirs;
@@ -216,24 +320,52 @@ __device__ __forceinline__ void march_tables(const MarchArgs& a, int n_tab, int 
     float sa = pixel_ang + div_(2.0f * kPiRef, (float)R) * (float)d;
     float sn, cs;
     sincosf_(sa, &sn, &cs);
-    sm.dir[d] = make_float2(cs, sn);
+    sm.dir[d] = make_float4(cs, sn, rcp_(cs), rcp_(sn));
   }
   const float q = (float)(a.num_levels - 1);
   const float ln2 = logf_(2.0f);
-  for (int s = tid; s < n_tab; s += nthreads) {
+  constexpr bool kTex = std::is_same<Step, TexStep>::value;
+  for (int t = tid; t < padded_steps<kTex>(n_tab); t += nthreads) {
+    const int s = min(t, n_tab - 1);
     float off = ns * powf_(div_(2.0f * kPiRef, (float)SR) + 1.0f, (float)s + lin) + 1.0f - ns;
     float lod = div_(logf_(gmax(0.0f, div_(2.0f * kPiRef, (float)SR) * (off - 1.0f) * 0.5f)), ln2) + (-2.0f);
     float lam = gmin(gmax(lod, 0.0f), q);
-    float lo = floorf(lam);
-    StepEntry e;
+    Step e;
     e.off = off;
-    e.delta = lam - lo;
-    e.lo = (int)lo;
-    if (TEX) e.level = lam;  // == lo + delta exactly (lam - floor(lam) and the sum back are exact)
-    else e.hi = min(e.lo + 1, a.num_levels - 1);
-    sm.step[s] = e;
+    if constexpr (kTex) {
+      e.level = lam;
+    } else {
+      const float lo = floorf(lam);
+      e.delta = lam - lo;
+      e.lo = (int)lo;
+      e.hi = min(e.lo + 1, a.num_levels - 1);
+      e.w0 = a.width >> e.lo;
+      e.h0 = a.height >> e.lo;
+      e.w1 = a.width >> e.hi;
+      e.h1 = a.height >> e.hi;
+      e.fw0 = (float)e.w0;
+      e.fh0 = (float)e.h0;
+      e.fw1 = (float)e.w1;
+      e.fh1 = (float)e.h1;
+      e.img0 = img[e.lo];
+      e.img1 = img[e.hi];
+    }
+    sm.step[t] = e;
   }
-  if (tid < a.num_levels) sm.lsize[tid] = make_float2((float)(a.width >> tid), (float)(a.height >> tid));
+}
+
+// Place of thread `tid` in its tile of 32 x KY sub-image pixels.  A warp takes 8 x 4
+// pixels (16 x 2 in a tile of two rows): its rays stay closer together than a row of
+// 32, so that its lanes leave a direction and raise their horizon together (measured at
+// 1283 x 721, R = 12: 28.2 active lanes an instruction instead of 25.6, the exact march
+// 1767 -> 1664 us, the fast one 1130 -> 1081 us).  Texture taps serve four neighbouring
+// lanes at once, so there each four are a 2 x 2 block (621 us against 646 with rows of 8
+// and 662 with a row of 32).
+template <int KY, bool TEX> __device__ __forceinline__ int2 tile_place(int tid) {
+  const int w = tid >> 5, l = tid & 31;
+  if (KY == 2) return make_int2((w & 1) * 16 + (l & 15), l >> 4);
+  if (TEX) return make_int2((w & 3) * 8 + ((l & 1) | ((l >> 1) & 6)), (w >> 2) * 4 + (((l >> 1) & 1) | ((l >> 3) & 2)));
+  return make_int2((w & 3) * 8 + (l & 7), (w >> 2) * 4 + (l >> 3));
 }
 
 // One CTA-tile of the march: the pixels of interleave pattern `pat` in march
@@ -242,7 +374,7 @@ __device__ __forceinline__ void march_tables(const MarchArgs& a, int n_tab, int 
 // CTA calls it (it contains one CTA barrier).
 //
 // SPLIT > 1 (the direction-split form for short tile lists): the CTA takes one
-// row `row` of the tile, thread (x, s) marches pixel x's directions s, s + SPLIT,
+// warp's pixels of the tile (`row` of its 4 warps), thread (x, s) marches pixel x's directions s, s + SPLIT,
 // ..., stores each direction's term in `contrib` (at most kSplitMaxDirs
 // directions), and after a barrier thread (x, 0) adds the terms in direction
 // order -- the same sum, in the same order, as one thread marching them all.
@@ -254,15 +386,14 @@ __device__ __forceinline__ void march_tables(const MarchArgs& a, int n_tab, int 
 template <int DCH, bool DEINT, int KY, bool FAST, bool SOFT = false, int SPLIT = 1, bool REC = false,
           bool TEX = false>
 __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pat, int tile, int tiles_x,
-                                           MarchSmem& sm, int row = 0, float* contrib = nullptr) {
+                                           MarchSmem<TEX>& sm, int row = 0, float* contrib = nullptr) {
   static_assert(!SOFT || (DCH == 2 && !FAST), "the soft horizon needs both depth moments, exact contract");
   static_assert(SPLIT == 1 || (!DEINT && !SOFT), "the direction split serves the standard form");
   static_assert(!REC || (SPLIT == 1 && !DEINT && !SOFT), "recording serves the standard form");
   static_assert(!TEX || (FAST && DCH == 2 && !DEINT), "texture depth taps serve the fast standard form");
   constexpr int kThreads = kMarchTx * (SPLIT > 1 ? SPLIT : KY);
-  StepEntry* s_step = sm.step;
-  float2* s_dir = sm.dir;
-  float2* s_lsize = sm.lsize;
+  auto* s_step = sm.step;
+  const float4* s_dir = sm.dir;
   const int P = a.pattern;
   const int kx = pat % P, ky = pat / P;
   const int R = a.dirs;
@@ -271,12 +402,13 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
   const float ns = div_(W, 1000.0f);
 
   const int tid = threadIdx.y * kMarchTx + threadIdx.x;
-  march_tables<TEX>(a, n_tab, pat, sm, tid, kThreads);
+  march_tables(a, a.depth, n_tab, pat, sm, tid, kThreads);
   __syncthreads();
 
   // Pixel of this thread.
-  const int i = (tile % tiles_x) * kMarchTx + threadIdx.x;
-  const int j = (tile / tiles_x) * KY + (SPLIT > 1 ? row : (int)threadIdx.y);
+  const int2 place = SPLIT > 1 ? tile_place<KY, TEX>(32 * row + threadIdx.x) : tile_place<KY, TEX>(tid);
+  const int i = (tile % tiles_x) * kMarchTx + place.x;
+  const int j = (tile / tiles_x) * KY + place.y;
   int px = kx + P * i, py = ky + P * j;
   const bool inside = px < a.width && py < a.height;
   if (SPLIT == 1 && !inside) return;
@@ -285,10 +417,11 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     py = min(ky, a.height - 1);
   }
 
-  const float rW = rcp_(W), rH = rcp_(H);  // x / W == x * rcp(W) under the division contract
+  const p2 rWH = pk(a.inv_size[0], a.inv_size[1]);  // x / W == x * rcp(W) under the division contract
   const float cpx = (float)px + 0.5f, cpy = (float)py + 0.5f;
-  const float cscx = cpx * rW, cscy = cpy * rH;
-  f3 N;
+  const p2 centre = pk(cpx, cpy);
+  const float cscx = cpx * lo_(rWH), cscy = cpy * hi_(rWH);
+  v3 N;
   float cdepth;
   size_t out_idx;
   if (DEINT) {
@@ -296,18 +429,19 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     const int dx = kx * sw + i, dy = ky * sh + j;
     out_idx = (size_t)dy * a.width + dx;
     float4 n = ld4(a.normal, (int)out_idx);
-    N = mk3(n.x, n.y, n.z);
+    N = mkv3(n.x, n.y, n.z);
     cdepth = __ldg(a.ndc + out_idx);
   } else {
     out_idx = (size_t)py * a.width + px;
     float4 n = sample4(a.normal, a.width, a.height, cscx, cscy);
-    N = mk3(n.x, n.y, n.z);
+    N = mkv3(n.x, n.y, n.z);
     cdepth = sample1(a.ndc, a.width, a.height, cscx, cscy);
   }
 
-  const float4 cam4 = mat_vec(a.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
-  const f3 cam = mk3(cam4.x, cam4.y, cam4.z);
-  const f3 cwp = unproject(a.inv_view_proj, cscx, cscy, cdepth);
+  const v3 cam = mkv3(a.cam[0], a.cam[1], a.cam[2]);
+  const v3 cwp = unproject_p(a.inv_view_proj, cscx, cscy, cdepth);
+  // Eye direction (:180); the view ray to the centre, normalize(cwp - cam), is its negative exactly.
+  const v3 ed = normalize3(sub3(cam, cwp));
   const float ambient = 0.01f;
   const float log_base = logf_(div_(2.0f * kPiRef, (float)SR) + 1.0f);
   const float inv_width = div_(1.0f, 0.1f);
@@ -319,7 +453,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
   // in which a warp's 32 pixels are consecutive: coalesced stores and loads.
   const unsigned npix = (unsigned)record_pixels(a);
   const unsigned rec_idx = ((unsigned)pat * ((a.height + P - 1) / P) + j) * ((a.width + P - 1) / P) + i;
-  f3 sum = mk3(0.0f, 0.0f, 0.0f);
+  Light sum{pk(0.0f), 0.0f};
   for (int d = SPLIT > 1 ? (int)threadIdx.y : 0; d < R; d += SPLIT) {
     unsigned long long hits = 0ull;  // REC: steps that raised the horizon
     // REC: the next hc slot; the k-th hit of every pixel is row k of the direction's
@@ -328,171 +462,192 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     // record is written and read once, larger than L2: streaming (evict-first) stores
     // and loads keep the pyramids the taps read resident in L2 (0.4 % of the frame).
     float* rec_next = REC ? a.rec_hc + (size_t)d * a.rec_steps * npix + rec_idx : nullptr;
-    const float2 dir = s_dir[d];
+    const float4 dir4 = s_dir[d];
+    const p2 dir = pk(dir4.x, dir4.y);
+    // Texture taps: the first step's depth, fetched before the direction's frame.
+    TexStep te;
+    p2 tsp;
+    float tdepth = 0.0f;
+    auto fetch = [&](int s) {
+      if constexpr (TEX) {
+        te = s_step[s];
+        tsp = pmul(padd(centre, pmul(dir, pk(te.off))), rWH);
+        tdepth = tex2DLod<float>(a.depth_tex, lo_(tsp), hi_(tsp), te.level);
+      }
+    };
+    fetch(0);
     const float eps = 10e-1f;
-    const float ocx = (cpx + dir.x * eps) * rW, ocy = (cpy + dir.y * eps) * rH;
-    // The direction's frame (:180-199): eye direction ed, tangent et (the
-    // normalised difference of two view rays one pixel apart: a cancelling sum,
-    // kept exact in both precisions), and the initial horizon h0 of the projected
-    // normal.  The fast precision takes h0 from its fitted atan and cos 2h0,
-    // sin 2h0 from the atan's arguments, as its step loop does.
-    const f3 owp = unproject(a.inv_view_proj, ocx, ocy, cdepth);
-    const f3 ed = normalize3(sub3(cam, cwp));
-    const f3 et = normalize3(sub3(normalize3(sub3(owp, cam)), normalize3(sub3(cwp, cam))));
+    const p2 oc = pmul(padd(centre, pmul(dir, pk(eps))), rWH);
+    // The direction's frame (:180-199): tangent et (the normalised difference of two
+    // view rays one pixel apart: a cancelling sum, kept exact in both precisions),
+    // and the initial horizon h0 of the projected normal.  The fast precision takes
+    // h0 from its fitted atan and cos 2h0, sin 2h0 from the atan's arguments, as its
+    // step loop does.
+    const v3 owp = unproject_p(a.inv_view_proj, lo_(oc), hi_(oc), cdepth);
+    const v3 et = normalize3(add3(normalize3(sub3(owp, cam)), ed));
     float max_h, cm, sm;
     {
-      const f3 cr = cross3(et, ed);
-      const f3 dnp = cross3(mk3(-cr.x, -cr.y, -cr.z), N);
+      const f3 cr = cross3(unpack3(et), unpack3(ed));
+      const f3 dnp = cross3(mk3(-cr.x, -cr.y, -cr.z), unpack3(N));
       if (FAST) {
-        const float hy = fdot3(dnp, et), hx = fdot3(dnp, ed);
+        const float hy = fdot3(dnp, unpack3(et)), hx = fdot3(dnp, unpack3(ed));
         max_h = fast_atan2(hy, hx);
-        cm = 1.0f;
-        sm = 0.0f;
-        const float r2 = fmaf(hx, hx, hy * hy);
-        if (r2 > 0.0f) {
-          const float ir = __fdividef(1.0f, r2);
-          cm = (hx - hy) * (hx + hy) * ir;
-          sm = 2.0f * hx * hy * ir;
-        }
+        double_angle(hx, hy, cm, sm);
       } else {
-        max_h = atan2f_(dot3(dnp, et), dot3(dnp, ed));
+        max_h = march_atan2(dot3(dnp, unpack3(et)), dot3(dnp, unpack3(ed)));
         sincosf_(2.0f * max_h, &sm, &cm);
       }
     }
     // BoxRayCast(centre, dir, (0,0), viewport) (:83-99, :202-204).
     float path;
     {
-      float ix = rcp_(dir.x), iy = rcp_(dir.y);
+      const float ix = dir4.z, iy = dir4.w;
       float t1 = (0.0f - cpx) * ix, t2 = (W - cpx) * ix;
       float t3 = (0.0f - cpy) * iy, t4 = (H - cpy) * iy;
       float tmax = gmin(gmax(t1, t2), gmax(t3, t4));
       path = fabsf(tmax);
     }
-    const float qd = 0.25f * (FAST ? fdot3(ed, N) : dot3(ed, N));
-    const float qt = 0.25f * (FAST ? fdot3(et, N) : dot3(et, N));
-    // FAST: the step's horizon coordinates hy = et . (n d + cam - cwp), hx = ed . (...)
-    // with the sample's view ray n = sign(w) U / |U|, U = A + sx B + sy C (set_ray_basis):
-    // et . U and ed . U are linear in (sx, sy), so the direction's constants are
-    // et . A, et . B, et . C, ed . A, ... and et . (cam - cwp), ed . (cam - cwp).
-    f3 eT = mk3(0.0f, 0.0f, 0.0f), eD = eT;
-    float etc = 0.0f, edc = 0.0f;
-    if (FAST) {
-      const float* rb = a.ray;
-      eT = mk3(fdot3(et, mk3(rb[0], rb[1], rb[2])), fdot3(et, mk3(rb[4], rb[5], rb[6])),
-               fdot3(et, mk3(rb[8], rb[9], rb[10])));
-      eD = mk3(fdot3(ed, mk3(rb[0], rb[1], rb[2])), fdot3(ed, mk3(rb[4], rb[5], rb[6])),
-               fdot3(ed, mk3(rb[8], rb[9], rb[10])));
-      const f3 cc = sub3(cam, cwp);
-      etc = fdot3(et, cc);
-      edc = fdot3(ed, cc);
+    const float qd = 0.25f * (FAST ? fdot3(unpack3(ed), unpack3(N)) : dot3(ed, N));
+    const float qt = 0.25f * (FAST ? fdot3(unpack3(et), unpack3(N)) : dot3(et, N));
+    // The pairs (tangent, eye): FAST: the step's horizon coordinates hy = et . (n d +
+    // cam - cwp), hx = ed . (...) with the sample's view ray n = sign(w) U / |U|, U = A +
+    // sx B + sy C (set_ray_basis): et . U and ed . U are linear in (sx, sy), so the
+    // direction's constants are (et, ed) . A, . B, . C and (et, ed) . (cam - cwp).
+    // Otherwise the components of et and ed themselves.
+    p2 e0, e1, e2, ec = pk(0.0f);
+    {
+      const f3 t = unpack3(et), u = unpack3(ed);
+      e0 = pk(t.x, u.x);
+      e1 = pk(t.y, u.y);
+      e2 = pk(t.z, u.z);
+      if (FAST) {
+        const float* rb = a.ray;
+        auto along = [&](float x, float y, float z) { return pfma(e2, pk(z), pfma(e1, pk(y), pmul(e0, pk(x)))); };
+        const f3 cc = unpack3(sub3(cam, cwp));
+        const p2 A = along(rb[0], rb[1], rb[2]), B = along(rb[4], rb[5], rb[6]), C = along(rb[8], rb[9], rb[10]);
+        ec = along(cc.x, cc.y, cc.z);
+        e0 = A;
+        e1 = B;
+        e2 = C;
+      }
     }
-    float hc0 = qd * (-cm + c0) + qt * (2.0f * max_h - 2.0f * 0.0f - sm + s0);
-    f3 dl = mk3(ambient * hc0, ambient * hc0, ambient * hc0);
+    const float hc0 = qd * (-cm + c0) + qt * (2.0f * max_h - 2.0f * 0.0f - sm + s0);
+    Light dl{pk(ambient * hc0), ambient * hc0};
     int iters = (int)div_(logf_(div_(path, ns)), log_base) + 1;
     if (a.step_cap > 0 && iters > a.step_cap) iters = a.step_cap;
     if (iters > n_tab) iters = n_tab;
-    for (int s = 0; s < iters; s++) {
-      const StepEntry e = s_step[s];
-      const float spx = cpx + dir.x * e.off, spy = cpy + dir.y * e.off;
-      const float sx = spx * rW, sy = spy * rH;
-      const bool two = e.delta != 0.0f;
-      Bilin blo, bhi;           // footprints of the software taps (not TEX)
-      float dsamp, dsq = 0.0f;  // E[d] and, for the soft horizon, E[d^2] of the trilinear tap
-      if (TEX) {
-        dsamp = tex2DLod<float>(a.depth_tex, sx, sy, tex_level(e));
-      } else {
-        const float2 slo = s_lsize[e.lo];
-        blo = bilin_f(sx, sy, slo.x, slo.y, a.width >> e.lo, a.height >> e.lo);
+    // One step: its sample at (sx, sy) with depth dsamp has the horizon coordinates
+    // (hy, hx) in the direction's frame.
+    auto fast_horizon = [&](float sx, float sy, float dsamp) {
+      // The sample's view ray: (unproject(sx, sy, 1) - cam) scaled by the
+      // homogeneous w, which is linear in (sx, sy), normalised (see set_ray_basis),
+      // entering only through the linear forms above and |U|^2.
+      const float* rb = a.ray;
+      const float* q = a.ray_q;
+      const p2 eu = pfma(pk(sy), e2, pfma(pk(sx), e1, e0));
+      const p2 qx = pfma(pk(sx), pk(q[3], q[4]), pk(q[1], q[2]));
+      const float uu = fmaf(sx, lo_(qx), q[0]) + sy * fmaf(sy, q[5], hi_(qx));
+      const float uw = fmaf(sy, rb[11], fmaf(sx, rb[7], rb[3]));
+      const float sd = dsamp * copysignf(rsqrt_approx(uu), uw);
+      return pfma(pk(sd), eu, ec);
+    };
+    // FAST: the horizon contribution of a step that raises the horizon to sh (HC(h,
+    // hmax) of :254-264) times the edge fade, and the new horizon.
+    auto fast_raise = [&](float sx, float sy, float hy, float hx, float sh) {
+      // The fade is the product of saturate((1 - x) / 0.1) and saturate(x / 0.1) over
+      // both axes; at most one of an axis's two is below 1 (that needs x > 0.9 and x <
+      // 0.1), so their product is the smaller one, and saturate of a monotone product
+      // is monotone, so that is the clamp of the smaller argument; the coordinates are
+      // finite and never -0, where the GLSL clamp and the hardware one agree.
+      const float side = __saturatef(fminf(1.0f - sx, sx) * inv_width) * __saturatef(fminf(1.0f - sy, sy) * inv_width);
+      float cs, ss;
+      double_angle(hx, hy, cs, ss);
+      const float hc = fmaf(qd, cs - cm, qt * (fmaf(2.0f, max_h - sh, ss) - sm)) * side;
+      max_h = sh;
+      cm = cs;
+      sm = ss;
+      return hc;
+    };
+    auto record = [&](int s, float hc) {
+      __stcs(rec_next, hc);
+      rec_next += npix;
+      hits |= 1ull << s;
+    };
+    if constexpr (TEX) {
+      // The loop waits on its fetches, so both are taken early: the next step's depth
+      // is fetched before this step's horizon is tested, and a hit's light is added
+      // when the next hit (or the direction's end) comes, in the same order.
+      float4 pend = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // the last hit's light, and its hc
+      pend.x = pend.y = pend.z = ambient;
+#pragma unroll 2
+      for (int s = 0; s < iters; s++) {
+        const float sx = lo_(tsp), sy = hi_(tsp), level = te.level, d0 = tdepth;
+        fetch(s + 1);
+        const p2 h = fast_horizon(sx, sy, d0);
+        const float hy = lo_(h), hx = hi_(h);
+        const float sh = fast_atan2(hy, hx);
+        if (sh < max_h) {
+          add_lit(pend, ambient, dl);
+          const float hc = fast_raise(sx, sy, hy, hx, sh);
+          pend = tex2DLod<float4>(a.light_tex, sx, sy, level);
+          pend.w = hc;
+          if (REC) record(s, hc);
+        }
+      }
+      add_lit(pend, ambient, dl);
+    } else {
+      for (int s = 0; s < iters; s++) {
+        const TapStep e = s_step[s];
+        const p2 sp = pmul(padd(centre, pmul(dir, pk(e.off))), rWH);
+        const float sx = lo_(sp), sy = hi_(sp);
+        const bool two = e.delta != 0.0f;
+        TapFoot foot;
+        if (two) tap_foot2(e, sx, sy, foot);
+        else tap_foot1(e, sx, sy, foot);
+        float dsamp, dsq = 0.0f;  // E[d] and, for the soft horizon, E[d^2] of the trilinear tap
         if (SOFT) {
-          const float2 m = moments_bilin(a.depth[e.lo], blo);
+          const float2 m = moments_bilin(e.img0, foot, 0);
           dsamp = m.x;
           dsq = m.y;
-        } else {
-          dsamp = FAST ? depth_bilin_fast<DCH>(a.depth[e.lo], blo) : depth_bilin<DCH>(a.depth[e.lo], blo);
-        }
-        if (two) {
-          const float2 shi = s_lsize[e.hi];
-          bhi = bilin_f(sx, sy, shi.x, shi.y, a.width >> e.hi, a.height >> e.hi);
-          if (FAST) {
-            const float dhi = depth_bilin_fast<DCH>(a.depth[e.hi], bhi);
-            dsamp = fmaf(dhi - dsamp, e.delta, dsamp);
-          } else if (SOFT) {
-            const float2 mh = moments_bilin(a.depth[e.hi], bhi);
+          if (two) {
+            const float2 mh = moments_bilin(e.img1, foot, 1);
             dsamp = dsamp * (1.0f - e.delta) + mh.x * e.delta;
             dsq = dsq * (1.0f - e.delta) + mh.y * e.delta;
-          } else {
-            float dhi = depth_bilin<DCH>(a.depth[e.hi], bhi);
-            dsamp = dsamp * (1.0f - e.delta) + dhi * e.delta;
           }
-        }
-      }
-      float sh = 0.0f, hy = 0.0f, hx = 0.0f;
-      bool hit;
-      if (FAST) {
-        // The sample's view ray: (unproject(sx, sy, 1) - cam) scaled by the
-        // homogeneous w, which is linear in (sx, sy), normalised (see set_ray_basis),
-        // entering only through the linear forms above and |U|^2.
-        const float* rb = a.ray;
-        const float* q = a.ray_q;
-        const float eu = fmaf(sy, eT.z, fmaf(sx, eT.y, eT.x));
-        const float du = fmaf(sy, eD.z, fmaf(sx, eD.y, eD.x));
-        const float uu = fmaf(sx, fmaf(sx, q[3], q[1]), q[0]) + sy * fmaf(sy, q[5], fmaf(sx, q[4], q[2]));
-        const float uw = fmaf(sy, rb[11], fmaf(sx, rb[7], rb[3]));
-        const float sd = dsamp * copysignf(rsqrtf(uu), uw);
-        hy = fmaf(sd, eu, etc);
-        hx = fmaf(sd, du, edc);
-        sh = fast_atan2(hy, hx);
-        hit = sh < max_h;
-      } else {
-        const f3 q = unproject(a.inv_view_proj, sx, sy, 1.0f);
-        const f3 rn = normalize3(sub3(q, cam));
-        const f3 swp = add3(cam, mul3s(rn, dsamp));
-        const f3 wd = sub3(swp, cwp);
-        sh = atan2f_(dot3(et, wd), dot3(ed, wd));
-        if (SOFT) sh = soft_horizon(dsamp, dsq, rn, cam, cwp, ed, et, sh, max_h);
-        hit = sh < max_h;
-      }
-      if (hit) {
-        // The horizon contribution of the step (HC(h, hmax) of :254-264), then its light.
-        float side = 1.0f;
-        if (FAST) {
-          // The same product in fewer instructions: of saturate((1 - x) / 0.1) and
-          // saturate(x / 0.1) at most one is below 1 (that needs x > 0.9 and x < 0.1),
-          // so their product is the smaller one, and saturate of a monotone product is
-          // monotone, so that is the clamp of the smaller argument; the coordinates are
-          // finite and never -0, where the GLSL clamp and the hardware one agree.
-          side = __saturatef(fminf(1.0f - sx, sx) * inv_width) * __saturatef(fminf(1.0f - sy, sy) * inv_width);
         } else {
-          side = side * saturate((1.0f - sx) * inv_width);
-          side = side * saturate(sx * inv_width);
-          side = side * saturate((1.0f - sy) * inv_width);
-          side = side * saturate(sy * inv_width);
+          dsamp = depth_tap<DCH, FAST>(e, two, foot);
         }
-        float hc, ss, cs;
+        float hc;
         if (FAST) {
-          ss = 0.0f;
-          cs = 1.0f;
-          const float r2 = fmaf(hx, hx, hy * hy);
-          if (r2 > 0.0f) {
-            const float ir = __fdividef(1.0f, r2);
-            cs = (hx - hy) * (hx + hy) * ir;
-            ss = 2.0f * hx * hy * ir;
-          }
-          hc = fmaf(qd, cs - cm, qt * (fmaf(2.0f, max_h - sh, ss) - sm)) * side;
+          const p2 h = fast_horizon(sx, sy, dsamp);
+          const float sh = fast_atan2(lo_(h), hi_(h));
+          if (!(sh < max_h)) continue;
+          hc = fast_raise(sx, sy, lo_(h), hi_(h), sh);
         } else {
+          // unproject(sx, sy, 1) with its depth terms from the launch.
+          const Mat4& M = a.inv_view_proj;
+          const p2 t = pfma(sp, pk(2.0f), pk(-1.0f));
+          const p2 X = pk(lo_(t)), Y = pk(hi_(t));
+          const p2 qxy = padd(padd(pmul(pk(M.m[0], M.m[1]), X), pmul(pk(M.m[4], M.m[5]), Y)), pk(a.far_col[0], a.far_col[1]));
+          const p2 qzw = padd(padd(pmul(pk(M.m[2], M.m[3]), X), pmul(pk(M.m[6], M.m[7]), Y)), pk(a.far_col[2], a.far_col[3]));
+          const v3 rn = normalize3(sub3(from_rows(qxy, qzw), cam));
+          const v3 wd = sub3(add3(cam, mul3s(rn, dsamp)), cwp);
+          const p2 h = pdot3(e0, pk(lo_(wd.xy)), e1, pk(hi_(wd.xy)), e2, pk(wd.z));
+          float sh = march_atan2(lo_(h), hi_(h));
+          if (SOFT)
+            sh = soft_horizon(dsamp, dsq, unpack3(rn), unpack3(cam), unpack3(cwp), unpack3(ed), unpack3(et), sh, max_h);
+          if (!(sh < max_h)) continue;
+          const p2 lo = pmul(sp, pk(inv_width)), up = pmul(psub(pk(1.0f), sp), pk(inv_width));
+          const float side = saturate(lo_(up)) * saturate(lo_(lo)) * saturate(hi_(up)) * saturate(hi_(lo));
+          float ss, cs;
           sincosf_(2.0f * sh, &ss, &cs);
           hc = (qd * (-cm + cs) + qt * (2.0f * max_h - 2.0f * sh - sm + ss)) * side;
+          max_h = sh;
+          cm = cs;
+          sm = ss;
         }
-        if (TEX) add_light_tex(a, sx, sy, tex_level(e), hc, ambient, dl);
-        else add_light<FAST>(a, e, blo, bhi, two, hc, ambient, dl);
-        max_h = sh;
-        cm = cs;
-        sm = ss;
-        if (REC) {
-          __stcs(rec_next, hc);
-          rec_next += npix;
-          hits |= 1ull << s;
-        }
+        add_light<FAST>(a.light[e.lo], two ? a.light[e.hi] : nullptr, e.delta, foot, two, hc, ambient, dl);
+        if (REC) record(s, hc);
       }
     }
     if (REC) {
@@ -501,13 +656,11 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     }
     if (SPLIT > 1) {
       float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
-      c[0] = 2.0f * dl.x * rR;
-      c[1] = 2.0f * dl.y * rR;
-      c[2] = 2.0f * dl.z * rR;
+      c[0] = 2.0f * lo_(dl.rg) * rR;
+      c[1] = 2.0f * hi_(dl.rg) * rR;
+      c[2] = 2.0f * dl.b * rR;
     } else {
-      sum.x = sum.x + 2.0f * dl.x * rR;
-      sum.y = sum.y + 2.0f * dl.y * rR;
-      sum.z = sum.z + 2.0f * dl.z * rR;
+      add_term(sum, dl, rR);
     }
   }
   if (SPLIT > 1) {
@@ -515,12 +668,11 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     if (threadIdx.y != 0 || !inside) return;
     for (int d = 0; d < R; d++) {
       const float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
-      sum.x = sum.x + c[0];
-      sum.y = sum.y + c[1];
-      sum.z = sum.z + c[2];
+      sum.rg = padd(sum.rg, pk(c[0], c[1]));
+      sum.b = sum.b + c[2];
     }
   }
-  reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(sum.x, sum.y, sum.z, 1.0f);
+  reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(lo_(sum.rg), hi_(sum.rg), sum.b, 1.0f);
 }
 
 // The march of a pixel re-lit from its record (MarchArgs::rec = 2): the same
@@ -534,70 +686,59 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
   const int P = a.pattern;
   const int kx = pat % P, ky = pat / P;
   const int R = a.dirs;
-  const float W = (float)a.width, H = (float)a.height;
-  march_tables(a, n_tab, pat, sm, threadIdx.y * kMarchTx + threadIdx.x, kThreads);
+  march_tables(a, a.light, n_tab, pat, sm, threadIdx.y * kMarchTx + threadIdx.x, kThreads);
   __syncthreads();
-  const int i = (tile % tiles_x) * kMarchTx + threadIdx.x;
-  const int j = (tile / tiles_x) * KY + threadIdx.y;
+  const int2 place = tile_place<KY, false>(threadIdx.y * kMarchTx + threadIdx.x);
+  const int i = (tile % tiles_x) * kMarchTx + place.x;
+  const int j = (tile / tiles_x) * KY + place.y;
   const int px = kx + P * i, py = ky + P * j;
   if (px >= a.width || py >= a.height) return;
-  const float rW = rcp_(W), rH = rcp_(H);
-  const float cpx = (float)px + 0.5f, cpy = (float)py + 0.5f;
+  const p2 rWH = pk(a.inv_size[0], a.inv_size[1]);
+  const p2 centre = pk((float)px + 0.5f, (float)py + 0.5f);
   const size_t out_idx = (size_t)py * a.width + px;
   const unsigned npix = (unsigned)record_pixels(a);
   const unsigned rec_idx = ((unsigned)pat * ((a.height + P - 1) / P) + j) * ((a.width + P - 1) / P) + i;
   const float ambient = 0.01f;
   const float rR = rcp_((float)R);
-  f3 sum = mk3(0.0f, 0.0f, 0.0f);
+  Light sum{pk(0.0f), 0.0f};
   for (int d = 0; d < R; d++) {
-    const float2 dir = sm.dir[d];
+    const float4 dir4 = sm.dir[d];
+    const p2 dir = pk(dir4.x, dir4.y);
     const float hc0 = __ldcs(a.rec_hc0 + (size_t)d * npix + rec_idx);
     // Bits index the 64-entry table (ReplaySmem): in bounds whatever the mask holds.
     unsigned long long hits = __ldcs(a.rec_mask + (size_t)d * npix + rec_idx);
     const float* rec_next = a.rec_hc + (size_t)d * a.rec_steps * npix + rec_idx;
-    f3 dl = mk3(ambient * hc0, ambient * hc0, ambient * hc0);
+    Light dl{pk(ambient * hc0), ambient * hc0};
     while (hits) {
       const int s = __ffsll((long long)hits) - 1;
       hits &= hits - 1ull;
-      const StepEntry e = sm.step[s];
-      const float spx = cpx + dir.x * e.off, spy = cpy + dir.y * e.off;
-      const float sx = spx * rW, sy = spy * rH;
+      const TapStep& e = sm.step[s];
+      const p2 sp = pmul(padd(centre, pmul(dir, pk(e.off))), rWH);
       const float hc = __ldcs(rec_next);
       rec_next += npix;
-      const float2 slo = sm.lsize[e.lo];
-      const Bilin blo = bilin_f(sx, sy, slo.x, slo.y, a.width >> e.lo, a.height >> e.lo);
-      Bilin bhi;
       const bool two = e.delta != 0.0f;
-      if (two) {
-        const float2 shi = sm.lsize[e.hi];
-        bhi = bilin_f(sx, sy, shi.x, shi.y, a.width >> e.hi, a.height >> e.hi);
-      }
-      add_light<FAST>(a, e, blo, bhi, two, hc, ambient, dl);
+      TapFoot foot;
+      if (two) tap_foot2(e, lo_(sp), hi_(sp), foot);
+      else tap_foot1(e, lo_(sp), hi_(sp), foot);
+      add_light<FAST>(e.img0, e.img1, e.delta, foot, two, hc, ambient, dl);
     }
-    sum.x = sum.x + 2.0f * dl.x * rR;
-    sum.y = sum.y + 2.0f * dl.y * rR;
-    sum.z = sum.z + 2.0f * dl.z * rR;
+    add_term(sum, dl, rR);
   }
-  reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(sum.x, sum.y, sum.z, 1.0f);
+  reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(lo_(sum.rg), hi_(sum.rg), sum.b, 1.0f);
 }
 
-// Register budget: 64 per thread (8 CTAs of 128 threads per SM).  The software
-// step loop is issue-bound with more ready warps than issue slots, and a measured
-// 80-register build of the fast loop (6 CTAs per SM, fewer spills) ran 9 % slower.
-// The texture loop (TEX) waits on its texture fetches instead: 40 registers (12
-// CTAs per SM, a few spills) measured 4.6 % faster on the whole frame than 64, and
-// 48 registers (10 CTAs) 4.2 %; 32 registers (16 CTAs) spill in the step loop and
-// made the recording march 38 % slower.  The persistent batch kernel keeps 64: at 40
-// it spills in its work loop and the batched frame ran 24 % slower.
-template <bool FAST, int KY, bool TEX = false> constexpr int march_min_blocks() {
-  return (TEX ? 1536 : 1024) / (kMarchTx * KY);
-}
+// Register budget: 64 per thread (1024 threads per SM) everywhere.  Measured on the
+// present loops (1283 x 721, R = 12; two-bounce texture frame at 1080p, R = 16): 72 and
+// 80 registers spill less and run slower (fast march 1160 and 1177 us against 1130,
+// frame 4038 and 4062 us against 3924); for the texture loop 48 registers (1280 threads)
+// 704 us against 686, for the replay 48 and 40 registers 4248 and 4671 us a frame.
+template <int KY> constexpr int march_min_blocks() { return 1024 / (kMarchTx * KY); }
 
 template <int DCH, bool DEINT, int KY, bool FAST, bool SOFT = false, bool REC = false, bool TEX = false>
-__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY, TEX>())
+__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<KY>())
     march_kernel(const __grid_constant__ MarchArgs a, int n_tab, int tiles_x, int tiles_total) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];  // march_smem_bytes(n_tab, a.dirs)
-  MarchSmem sm = march_smem(dyn_smem, n_tab, a.dirs);
+  extern __shared__ __align__(16) unsigned char dyn_smem[];  // march_smem_bytes<TEX>(n_tab, a.dirs)
+  MarchSmem<TEX> sm = march_smem<TEX>(dyn_smem, n_tab);
   // Pattern is the fastest-varying block index: the P*P CTAs that share a
   // screen tile run together and share its texels in L1/L2.
   const int P = a.pattern;
@@ -608,7 +749,7 @@ __global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY, TEX>(
 }
 
 template <int KY, bool FAST>
-__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY>())
+__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<KY>())
     march_replay_kernel(const __grid_constant__ MarchArgs a, int n_tab, int tiles_x) {
   __shared__ ReplaySmem sm;  // n_tab <= kRecMaxSteps (checked at launch)
   const int P = a.pattern;
@@ -620,15 +761,12 @@ __global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY>())
 // CTAs -- or of the whole frame (a.tiles null; the autotuner's four-threads-per-
 // pixel layout): each CTA one row of a tile, each thread a quarter of a pixel's
 // directions.
-constexpr int kSplit = 4;
-constexpr int kSplitMaxDirs = 32;
-constexpr int kSplitMinDirs = 4;
 
 template <bool FAST, bool TEX>
 __global__ void __launch_bounds__(kMarchTx* kSplit, 1024 / (kMarchTx * kSplit))
     march_split_kernel(const __grid_constant__ MarchArgs a, int n_tab, int tiles_x, int tiles_total) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];  // march_smem_bytes(n_tab, a.dirs)
-  MarchSmem sm = march_smem(dyn_smem, n_tab, a.dirs);
+  extern __shared__ __align__(16) unsigned char dyn_smem[];  // march_smem_bytes<TEX>(n_tab, a.dirs)
+  MarchSmem<TEX> sm = march_smem<TEX>(dyn_smem, n_tab);
   __shared__ float contrib[kSplitMaxDirs * kMarchTx * 3];
   const int P2 = a.pattern * a.pattern;
   const int pat = blockIdx.x % P2;
@@ -645,7 +783,7 @@ __global__ void __launch_bounds__(kMarchTx* kSplit, 1024 / (kMarchTx * kSplit))
 // step loop reads them as the single-view kernel reads its own, where a copy in
 // shared memory cost registers, spills and 3 % of the batched frame.
 template <int KY, bool FAST, bool TEX>
-__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY>())
+__global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<KY>())
     march_batch_kernel(const __grid_constant__ BatchTable t, const int2* __restrict__ items, int num_items,
                        int* __restrict__ counter) {
   // The views' tables differ in size: dynamic shared memory of the largest
@@ -660,7 +798,7 @@ __global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<FAST, KY>())
     if (it >= num_items) return;
     const int2 w = __ldg(items + it);
     const BatchView& v = t.v[w.x];
-    MarchSmem sm = march_smem(tab_smem, v.n_tab, v.a.dirs);
+    MarchSmem<TEX> sm = march_smem<TEX>(tab_smem, v.n_tab);
     march_tile<2, false, KY, FAST, false, 1, false, TEX>(v.a, v.n_tab, w.y & 63, w.y >> 6, v.tiles_x, sm);
     __syncthreads();  // the tables and s_item are rewritten for the next item
   }
@@ -856,6 +994,12 @@ int PyramidTexture::Pack(const float* const* levels, int src_channels, cudaStrea
 // precisions scale the far-plane point alike and the fast rays track the exact ones.
 void set_ray_basis(MarchArgs& a) {
   const float* m = a.inv_view_proj.m;
+  const float* iv = a.inv_view.m;
+  // In the kernels' order and precision: M * (0, 0, 0, 1), and the depth and translation terms at depth 1.
+  for (int r = 0; r < 3; r++) a.cam[r] = (iv[r] * 0.0f + iv[4 + r] * 0.0f) + (iv[8 + r] * 0.0f + iv[12 + r] * 1.0f);
+  a.inv_size[0] = rcp_((float)a.width);
+  a.inv_size[1] = rcp_((float)a.height);
+  for (int r = 0; r < 4; r++) a.far_col[r] = m[8 + r] * 1.0f + m[12 + r] * 1.0f;
   const double cam[3] = {a.inv_view.m[12], a.inv_view.m[13], a.inv_view.m[14]};
   const float w_far = m[11] + m[15];
   double U[3][3];  // A, B, C: the ray's constant part and its derivatives in sx, sy
@@ -885,13 +1029,13 @@ void set_ray_basis(MarchArgs& a) {
 // Rays a warp marches: 32 pixels x the directions of each thread.
 static int rays_per_warp(int dirs, int split) { return kMarchTx * ((dirs + split - 1) / split); }
 
-// Untuned shapes: 4 rows, or 8 for the texture-tap loop (at 1920x1080, R = 16 its
-// recording march ran 1.8 % faster in 8-row CTAs and the two-bounce frame 0.8 %).
+// Untuned shapes: 4 rows (two-bounce texture frame at 1920x1080, R = 16: 3753 us
+// against 3781 with 8 and 3905 with 2; exact march at 1283x721: 1666 us against 1698
+// and 1713).
 static TunedLayout tuned_layout(const MarchArgs& a) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tuned.find(key_of(a));
-  const int rows = (a.fast && a.depth_tex) ? 8 : kMarchTy;
-  return it == g_tuned.end() ? TunedLayout{rows, 1} : it->second;
+  return it == g_tuned.end() ? TunedLayout{kMarchTy, 1} : it->second;
 }
 
 int march_table_size(const MarchArgs& a) {
@@ -961,7 +1105,7 @@ static void launch_tables(void (*kernel)(P...), dim3 grid, dim3 block, int smem,
 template <bool FAST, bool REC, bool TEX>
 static void launch_standard(const MarchArgs& a, int rows, dim3 grid, int n_tab, int tiles_x, int total,
                             cudaStream_t s) {
-  const int smem = march_smem_bytes(n_tab, a.dirs);
+  const int smem = march_smem_bytes<TEX>(n_tab, a.dirs);
   if (rows == 2)
     launch_tables(march_kernel<2, false, 2, FAST, false, REC, TEX>, grid, dim3(kMarchTx, 2), smem, s, a, n_tab,
                   tiles_x, total);
@@ -1013,7 +1157,7 @@ static int launch_march_rows(const MarchArgs& args, int rows, int split, cudaStr
     // The direction-split form (same result).
     grid.x *= kMarchTy;
     const dim3 block(kMarchTx, kSplit);
-    const int smem = march_smem_bytes(n_tab, a.dirs);
+    const int smem = tex ? march_smem_bytes<true>(n_tab, a.dirs) : march_smem_bytes<false>(n_tab, a.dirs);
     if (tex) launch_tables(march_split_kernel<true, true>, grid, block, smem, stream, a, n_tab, tiles_x, total);
     else if (a.fast) launch_tables(march_split_kernel<true, false>, grid, block, smem, stream, a, n_tab, tiles_x, total);
     else launch_tables(march_split_kernel<false, false>, grid, block, smem, stream, a, n_tab, tiles_x, total);
@@ -1040,7 +1184,7 @@ static int launch_march_rows(const MarchArgs& args, int rows, int split, cudaStr
     count_launches(1);
     return GI_OK;
   }
-  const int smem = march_smem_bytes(n_tab, a.dirs);
+  const int smem = march_smem_bytes<false>(n_tab, a.dirs);
   const dim3 b4(kMarchTx, 4);
   if (a.soft) {  // exact contract, standard form, 2-channel moments (checked by the caller)
     launch_tables(march_kernel<2, false, 4, false, true>, grid, b4, smem, stream, a, n_tab, tiles_x, total);
@@ -1156,7 +1300,7 @@ int launch_march_batch(const BatchTable& views, const int2* items, int num_items
     const BatchView& bv = views.v[v];
     if (bv.n_tab < 0 || bv.n_tab > GI_MAX_STEPS || bv.a.dirs < 0 || bv.a.dirs > GI_MAX_DIRS)
       return fail(GI_ERR_INVALID_ARGUMENT, "march batch: view tables out of range");
-    smem = std::max(smem, march_smem_bytes(bv.n_tab, bv.a.dirs));
+    smem = std::max(smem, tex ? march_smem_bytes<true>(bv.n_tab, bv.a.dirs) : march_smem_bytes<false>(bv.n_tab, bv.a.dirs));
   }
   auto go = [&](auto kernel) { launch_tables(kernel, dim3(grid), block, smem, stream, views, items, num_items, counter); };
   if (tex) {

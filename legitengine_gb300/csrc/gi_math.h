@@ -262,13 +262,11 @@ GI_HD void sincosf_(float x, float* s, float* c) {
   r = fma_(-k, kPiO2_3, r);
   float sr, cr;
   sincos_core(r, &sr, &cr);
-  int q = ((int)k) & 3;
-  switch (q) {
-    case 0: *s = sr; *c = cr; break;
-    case 1: *s = cr; *c = -sr; break;
-    case 2: *s = -sr; *c = -cr; break;
-    default: *s = -cr; *c = sr; break;
-  }
+  // Quadrant q: (sin, cos) = (s, c), (c, -s), (-s, -c), (-c, s) for q = 0..3.
+  const uint32_t q = (uint32_t)(int)k;
+  const float a = (q & 1u) ? cr : sr, b = (q & 1u) ? sr : cr;
+  *s = u2f(f2u(a) ^ ((q & 2u) << 30));
+  *c = u2f(f2u(b) ^ (((q + 1u) & 2u) << 30));
 }
 
 GI_HD float sinf_(float x) { float s, c; sincosf_(x, &s, &c); return s; }
