@@ -1,8 +1,8 @@
 // gi_inputs.cu -- the passes that feed the GI path (SSVGIRenderer.h:61-205):
 // G-buffer, shadow map and direct light.  The reference rasterises meshes; here
-// the scene is ray cast through the pixel centres, one thread per pixel: the
-// procedural primitives (boxes and spheres inside a room) staged in shared
-// memory, then the triangle meshes of a loaded scene, object by object behind a
+// the scene is ray cast through the pixel centres, one thread per pixel: those of the
+// procedural primitives (boxes and spheres inside a room) that the bounds of a warp's
+// rays meet, then the triangle meshes of a loaded scene, object by object behind a
 // bounds test.
 #include "gi_device.cuh"
 #include "gi_internal.h"
@@ -13,7 +13,9 @@ namespace {
 
 using namespace dev;
 
-constexpr int kTx = 32, kTy = 4;
+constexpr int kTx = 32, kTy = 4;         // direct light: one row of 32 pixels a warp
+constexpr int kCastX = 32, kCastY = 8;   // ray casts: tile of a CTA, in warps of 8 x 4 pixels
+constexpr int kCastThreads = kCastX * kCastY;
 constexpr int kPrimStage = 256;  // primitives staged per shared-memory batch
 
 struct ViewArgs {
@@ -36,7 +38,6 @@ ViewArgs view_args(const gi_view& v) {
 
 struct Hit {
   float t;
-  f3 n;
   int prim;  // analytic primitive hit, or -1
   int tri;   // triangle hit (when prim == -1), or -1
   int obj;   // the triangle's object
@@ -96,104 +97,290 @@ __device__ void cast_mesh(const MeshSet& m, f3 o, f3 d, const float (&iv)[3], Hi
   }
 }
 
+// A staged primitive: what its ray tests read that is the same for every ray of the
+// camera.  Room, box: its corners minus the origin.  Sphere: origin - centre, and
+// |origin - centre|^2 - r^2.  Two 16-byte reads.
+struct __align__(16) PrimTest {
+  float a[3];
+  int kind;  // gi_prim_kind, | kFinite
+  float b[3];
+  float pad;
+};
+constexpr int kFinite = 0x100;  // every value is finite
+
+__device__ __forceinline__ bool finite(float v) { return v - v == 0.0f; }
+
+__device__ __forceinline__ PrimTest prim_test(const gi_prim& p, f3 o) {
+  PrimTest r;
+  const float ov[3] = {o.x, o.y, o.z};
+  r.kind = p.kind;
+  if (p.kind == GI_PRIM_SPHERE) {
+    const f3 oc = sub3(o, mk3(p.a[0], p.a[1], p.a[2]));
+    r.a[0] = oc.x;
+    r.a[1] = oc.y;
+    r.a[2] = oc.z;
+    r.b[0] = dot3(oc, oc) - p.b[0] * p.b[0];
+    r.b[1] = r.b[2] = 0.0f;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      r.a[k] = p.a[k] - ov[k];
+      r.b[k] = p.b[k] - ov[k];
+    }
+  }
+  bool all = true;
+#pragma unroll
+  for (int k = 0; k < 3; k++) all = all && finite(r.a[k]) && finite(r.b[k]);
+  if (all) r.kind |= kFinite;
+  r.pad = 0.0f;
+  return r;
+}
+
+// Componentwise bounds of the warp's ray directions; NaN if a lane's is NaN.
+struct RayBounds {
+  float dlo[3], dhi[3];
+  float ilo[3], ihi[3];  // bounds of their reciprocals
+  bool open[3];          // an axis whose directions lie about zero: no bounds
+  bool closed;           // no axis is open, no direction NaN
+};
+
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm("redux.sync.min.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+__device__ __forceinline__ RayBounds ray_bounds(const float (&d)[3]) {
+  RayBounds r;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    r.dlo[k] = warp_min(d[k]);
+    r.dhi[k] = warp_max(d[k]);
+    r.open[k] = !(r.dlo[k] >= 1e-37f || r.dhi[k] <= -1e-37f);
+    // The rounded reciprocal decreases with d on each side of zero.
+    r.ilo[k] = rcp_(r.dhi[k]);
+    r.ihi[k] = rcp_(r.dlo[k]);
+  }
+  r.closed = !(r.open[0] || r.open[1] || r.open[2]);
+  return r;
+}
+
+// A lower bound of the distance at which the warp's rays can hit the primitive, +inf
+// if none can.  Rounding is monotone, so the bounds of a ray test's intermediate
+// values are the same operations on the bounds of its operands, without a margin.
+__device__ __forceinline__ float nearest_entry(const PrimTest& p, const RayBounds& r) {
+  if (p.kind == (GI_PRIM_BOX | kFinite)) {
+    float tn = -kInf, tf = kInf;  // lower bound of the entry, upper bound of the exit
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float a0 = p.a[k] * r.ilo[k], a1 = p.a[k] * r.ihi[k], b0 = p.b[k] * r.ilo[k], b1 = p.b[k] * r.ihi[k];
+      tn = r.open[k] ? tn : fmaxf(tn, fminf(fminf(a0, a1), fminf(b0, b1)));
+      tf = r.open[k] ? tf : fminf(tf, fmaxf(fmaxf(a0, a1), fmaxf(b0, b1)));
+    }
+    // An entry needs tn <= tf and tn > 0.
+    return tn > tf || tf <= 0.0f ? kInf : tn;
+  }
+  if (p.kind == (GI_PRIM_SPHERE | kFinite)) {
+    float lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float u = p.a[k] * r.dlo[k], v = p.a[k] * r.dhi[k];
+      lo[k] = fminf(u, v);
+      hi[k] = fmaxf(u, v);
+    }
+    const float blo = lo[0] + lo[1] + lo[2], bhi = hi[0] + hi[1] + hi[2];
+    // A hit needs disc = b^2 - cc >= 0 and t = -b - sqrt(disc) > 0.
+    const float disc = fmaxf(blo * blo, bhi * bhi) - p.b[0];
+    return disc < 0.0f || -blo <= 0.0f ? kInf : fmaxf(-bhi - sqrtf(disc), -kInf);  // NaN: no bound
+  }
+  return -kInf;
+}
+
+// Slab distances of a staged room or box.  NUMBERS: no product is NaN, and the minimum
+// and maximum are one instruction (they differ from GLSL's in the sign of a zero, which
+// no hit has).
+template <bool NUMBERS>
+__device__ __forceinline__ void slabs(const PrimTest& p, const float (&iv)[3], float (&t1)[3], float (&t2)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const float a = p.a[k] * iv[k], b = p.b[k] * iv[k];
+    t1[k] = NUMBERS ? fminf(a, b) : gmin(a, b);
+    t2[k] = NUMBERS ? fmaxf(a, b) : gmax(a, b);
+  }
+}
+__device__ __forceinline__ float room_exit(const float (&t2)[3], int& ax) {
+  ax = 0;
+  float tf = t2[0];
+  if (t2[1] < tf) { ax = 1; tf = t2[1]; }
+  if (t2[2] < tf) { ax = 2; tf = t2[2]; }
+  return tf;
+}
+__device__ __forceinline__ float box_entry(const float (&t1)[3], int& ax) {
+  ax = 0;
+  float tn = t1[0];
+  if (t1[1] > tn) { ax = 1; tn = t1[1]; }
+  if (t1[2] > tn) { ax = 2; tn = t1[2]; }
+  return tn;
+}
+
+// Distance of a ray's hit on a staged primitive; not > 0 if there is none.
+template <bool NUMBERS>
+__device__ __forceinline__ float prim_hit(const PrimTest& p, f3 d, const float (&iv)[3]) {
+  const int kind = p.kind & ~kFinite;
+  if (kind == GI_PRIM_SPHERE) {
+    const float b = p.a[0] * d.x + p.a[1] * d.y + p.a[2] * d.z;
+    const float disc = b * b - p.b[0];
+    return disc >= 0.0f ? -b - sqrtf(disc) : -1.0f;
+  }
+  if (kind != GI_PRIM_ROOM && kind != GI_PRIM_BOX) return -1.0f;
+  float t1[3], t2[3];
+  int ax;
+  slabs<NUMBERS>(p, iv, t1, t2);
+  if (NUMBERS) {
+    const float tf = fminf(fminf(t2[0], t2[1]), t2[2]);
+    if (kind == GI_PRIM_ROOM) return tf;
+    const float tn = fmaxf(fmaxf(t1[0], t1[1]), t1[2]);
+    return tn <= tf ? tn : -1.0f;
+  }
+  if (kind == GI_PRIM_ROOM) return room_exit(t2, ax);
+  const float tn = box_entry(t1, ax);
+  return tn <= gmin(gmin(t2[0], t2[1]), t2[2]) ? tn : -1.0f;
+}
+
 // Nearest hit: room interior (exit face), box exterior (entry face), sphere
 // (near root), ties kept by the earlier primitive.
+//
+// The cast was bound by its arithmetic, every ray testing every primitive.  Now each
+// lane of a warp bounds one primitive's distance to the warp's 8 x 4 pixels of rays
+// (32 primitives in the time of one test), and the rays test the primitives in order
+// of that bound until it passes their farthest hit: the same nearest hit, bit for
+// bit.  Measured with 64 boxes and 16 spheres: the G-buffer at 1920 x 1080 319 -> 67 us, a
+// shadow map of 1024 x 1024 171 -> 27 us (87 and 35 us in index order, without the
+// order by distance).
 __device__ void cast_ray(const gi_prim* __restrict__ prims, int np, const MeshSet& mesh, f3 o, f3 d, Hit& h,
-                         gi_prim* s_prims) {
-  h.t = __int_as_float(0x7f800000);
+                         PrimTest* s_prims) {
+  h.t = kInf;
   h.prim = -1;
   h.tri = -1;
   h.obj = -1;
   h.u = h.v = 0.0f;
-  h.n = mk3(0.0f, 0.0f, 0.0f);
   const float iv[3] = {rcp_(d.x), rcp_(d.y), rcp_(d.z)};
-  const float ov[3] = {o.x, o.y, o.z};
   const float dv[3] = {d.x, d.y, d.z};
+  const RayBounds bounds = ray_bounds(dv);
+  const int lane = threadIdx.x & 31;
+  float farthest = kInf;  // of the warp's hits so far
   for (int base = 0; base < np; base += kPrimStage) {
     const int cnt = min(kPrimStage, np - base);
     __syncthreads();
-    for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < cnt; i += blockDim.x * blockDim.y)
-      s_prims[i] = prims[base + i];
+    for (int i = threadIdx.x; i < cnt; i += kCastThreads) s_prims[i] = prim_test(prims[base + i], o);
     __syncthreads();
-    for (int ii = 0; ii < cnt; ii++) {
-      const gi_prim& p = s_prims[ii];
-      const int i = base + ii;
-      if (p.kind == GI_PRIM_ROOM || p.kind == GI_PRIM_BOX) {
-        float t1[3], t2[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          float a = (p.a[k] - ov[k]) * iv[k];
-          float b = (p.b[k] - ov[k]) * iv[k];
-          t1[k] = gmin(a, b);
-          t2[k] = gmax(a, b);
+    for (int first = 0; first < cnt; first += 32) {
+      const int own = first + lane;
+      float entry = own < cnt ? nearest_entry(s_prims[own], bounds) : kInf;
+      for (;;) {
+        const float next = warp_min(entry);
+        if (next == kInf || next > farthest) break;
+        const int from = __ffs((int)__ballot_sync(0xffffffffu, entry == next)) - 1;
+        if (lane == from) entry = kInf;
+        const PrimTest p = s_prims[first + from];
+        const int prim = base + first + from;
+        const float t = bounds.closed && (p.kind & kFinite) ? prim_hit<true>(p, d, iv) : prim_hit<false>(p, d, iv);
+        if (t > 0.0f && (t < h.t || (t == h.t && prim < h.prim))) {
+          h.t = t;
+          h.prim = prim;
         }
-        if (p.kind == GI_PRIM_ROOM) {
-          int ax = 0;
-          float tf = t2[0];
-          if (t2[1] < tf) { ax = 1; tf = t2[1]; }
-          if (t2[2] < tf) { ax = 2; tf = t2[2]; }
-          if (tf > 0.0f && tf < h.t) {
-            h.t = tf;
-            h.prim = i;
-            float nv[3] = {0.0f, 0.0f, 0.0f};
-            nv[ax] = dv[ax] > 0.0f ? -1.0f : 1.0f;
-            h.n = mk3(nv[0], nv[1], nv[2]);
-          }
-        } else {
-          int ax = 0;
-          float tn = t1[0];
-          if (t1[1] > tn) { ax = 1; tn = t1[1]; }
-          if (t1[2] > tn) { ax = 2; tn = t1[2]; }
-          float tf = gmin(gmin(t2[0], t2[1]), t2[2]);
-          if (tn <= tf && tn > 0.0f && tn < h.t) {
-            h.t = tn;
-            h.prim = i;
-            float nv[3] = {0.0f, 0.0f, 0.0f};
-            nv[ax] = dv[ax] > 0.0f ? -1.0f : 1.0f;
-            h.n = mk3(nv[0], nv[1], nv[2]);
-          }
-        }
-      } else if (p.kind == GI_PRIM_SPHERE) {
-        const f3 c = mk3(p.a[0], p.a[1], p.a[2]);
-        const float r = p.b[0];
-        const f3 oc = sub3(o, c);
-        const float b = dot3(oc, d);
-        const float cc = dot3(oc, oc) - r * r;
-        const float disc = b * b - cc;
-        if (disc >= 0.0f) {
-          const float t = -b - sqrtf(disc);
-          if (t > 0.0f && t < h.t) {
-            h.t = t;
-            h.prim = i;
-            h.n = normalize3(sub3(add3(o, mul3s(d, t)), c));
-          }
-        }
+        farthest = warp_max(h.t);
       }
     }
   }
   if (mesh.num_objects > 0) cast_mesh(mesh, o, d, iv, h);
 }
 
-// gBufferBuilder.frag:28-38 at the primary hit.
-__global__ void __launch_bounds__(kTx* kTy) gbuffer_kernel(const __grid_constant__ ViewArgs v,
-                                                           const gi_prim* __restrict__ prims, int np, MeshSet mesh,
-                                                           float* __restrict__ albedo, float* __restrict__ emissive,
-                                                           float* __restrict__ normal, float* __restrict__ moments,
-                                                           float* __restrict__ ndc) {
-  __shared__ gi_prim s_prims[kPrimStage];
-  const int x = blockIdx.x * kTx + threadIdx.x, y = blockIdx.y * kTy + threadIdx.y;
-  const bool live = x < v.width && y < v.height;
-  const int xc = live ? x : 0, yc = live ? y : 0;
-  const float sx = div_((float)xc + 0.5f, (float)v.width), sy = div_((float)yc + 0.5f, (float)v.height);
-  const float4 cam4 = mat_vec(v.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
-  const f3 cam = mk3(cam4.x, cam4.y, cam4.z);
-  const f3 farp = unproject(v.inv_view_proj, sx, sy, 1.0f);
-  const f3 dir = normalize3(sub3(farp, cam));
+// The surface normal at the hit of an analytic primitive.
+__device__ __forceinline__ f3 prim_normal(const gi_prim& g, f3 o, f3 d, float t) {
+  if (g.kind == GI_PRIM_SPHERE) return normalize3(sub3(add3(o, mul3s(d, t)), mk3(g.a[0], g.a[1], g.a[2])));
+  const PrimTest p = prim_test(g, o);
+  const float iv[3] = {rcp_(d.x), rcp_(d.y), rcp_(d.z)}, dv[3] = {d.x, d.y, d.z};
+  float t1[3], t2[3];
+  slabs<false>(p, iv, t1, t2);
+  int ax;
+  if (g.kind == GI_PRIM_ROOM) room_exit(t2, ax);
+  else box_entry(t1, ax);
+  float nv[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) nv[k] = k == ax ? (dv[k] > 0.0f ? -1.0f : 1.0f) : 0.0f;
+  return mk3(nv[0], nv[1], nv[2]);
+}
+
+// A thread's pixel and ray.  Threads past the image take its last row or column (they
+// join the warp's votes) and store nothing.
+struct CastPixel {
+  int x, y;
+  bool live;
+  f3 org, dir;
+};
+__device__ __forceinline__ CastPixel cast_pixel(const ViewArgs& v) {
+  CastPixel c;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  c.x = blockIdx.x * kCastX + (w & 3) * 8 + (l & 7);
+  c.y = blockIdx.y * kCastY + (w >> 2) * 4 + (l >> 3);
+  c.live = c.x < v.width && c.y < v.height;
+  c.x = min(c.x, v.width - 1);
+  c.y = min(c.y, v.height - 1);
+  const float sx = div_((float)c.x + 0.5f, (float)v.width), sy = div_((float)c.y + 0.5f, (float)v.height);
+  const float4 o4 = mat_vec(v.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
+  c.org = mk3(o4.x, o4.y, o4.z);
+  c.dir = normalize3(sub3(unproject(v.inv_view_proj, sx, sy, 1.0f), c.org));
+  return c;
+}
+
+// gBufferBuilder.frag:28-38 at the primary hit.  The eight powers of a surface's
+// colours are the same for every pixel that shows it: a warp evaluates them once for
+// each of the surfaces it hits, four surfaces at a time, a lane per channel.
+__global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_constant__ ViewArgs v,
+                                                               const gi_prim* __restrict__ prims, int np, MeshSet mesh,
+                                                               float* __restrict__ albedo,
+                                                               float* __restrict__ emissive,
+                                                               float* __restrict__ normal,
+                                                               float* __restrict__ moments, float* __restrict__ ndc) {
+  __shared__ PrimTest s_prims[kPrimStage];
+  __shared__ __align__(16) float s_colour[kCastThreads / 32][32][8];  // a warp's surfaces: albedo, emissive
+  const CastPixel c = cast_pixel(v);
   Hit h;
-  cast_ray(prims, np, mesh, cam, dir, h, s_prims);  // every thread joins the staging barriers
-  if (!live) return;
-  const size_t i = (size_t)y * v.width + x;
-  if (h.prim < 0 && h.tri < 0) {
+  cast_ray(prims, np, mesh, c.org, c.dir, h, s_prims);
+  const int lane = threadIdx.x & 31;
+  auto& colour = s_colour[threadIdx.x >> 5];
+  const int surface = h.prim >= 0 ? h.prim : (h.tri >= 0 ? np + h.obj : -1);
+  int slot = 0;
+  {
+    unsigned todo = __ballot_sync(0xffffffffu, surface >= 0);
+    for (int n = 0; todo; n += 4) {  // four surfaces a round: lanes 8 k .. 8 k + 7 take the k-th
+      int mine = -1;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (!todo) break;
+        const int id = __shfl_sync(0xffffffffu, surface, __ffs((int)todo) - 1);
+        todo &= ~__ballot_sync(0xffffffffu, surface == id);
+        if (surface == id) slot = n + k;
+        if ((lane >> 3) == k) mine = id;
+      }
+      if (mine >= 0) {
+        const int ch = lane & 3;
+        const float* al = mine < np ? prims[mine].albedo : mesh.objects[mine - np].albedo;
+        const float* em = mine < np ? prims[mine].emissive : mesh.objects[mine - np].emissive;
+        colour[n + (lane >> 3)][lane & 7] = powf_((lane & 4) ? em[ch] : al[ch], 2.2f);
+      }
+    }
+    __syncwarp();
+  }
+  if (!c.live) return;
+  const size_t i = (size_t)c.y * v.width + c.x;
+  if (surface < 0) {
     reinterpret_cast<float4*>(albedo)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     reinterpret_cast<float4*>(emissive)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     reinterpret_cast<float4*>(normal)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -201,57 +388,37 @@ __global__ void __launch_bounds__(kTx* kTy) gbuffer_kernel(const __grid_constant
     ndc[i] = 1.0f;
     return;
   }
-  const f3 hit = add3(cam, mul3s(dir, h.t));
-  const f3 dl = sub3(hit, cam);
+  const f3 hit = add3(c.org, mul3s(c.dir, h.t));
+  const f3 dl = sub3(hit, c.org);
   const float delta_len = sqrtf(dot3(dl, dl));
-  const float* src_al;
-  const float* src_em;
+  f3 n;
   if (h.prim >= 0) {
-    src_al = prims[h.prim].albedo;
-    src_em = prims[h.prim].emissive;
+    n = prim_normal(prims[h.prim], c.org, c.dir, h.t);
   } else {
-    src_al = mesh.objects[h.obj].albedo;
-    src_em = mesh.objects[h.obj].emissive;
     // Barycentric blend of the vertex normals, (1 - u - v) n0 + u n1 + v n2.
     const gi_triangle& tr = mesh.tris[h.tri];
     const float w0 = 1.0f - h.u - h.v;
     const f3 n0 = ld3(tr.n[0]), n1 = ld3(tr.n[1]), n2 = ld3(tr.n[2]);
-    h.n = add3(add3(mul3s(n0, w0), mul3s(n1, h.u)), mul3s(n2, h.v));
+    n = add3(add3(mul3s(n0, w0), mul3s(n1, h.u)), mul3s(n2, h.v));
   }
-  float4 al, em;
-  al.x = powf_(src_al[0], 2.2f);
-  al.y = powf_(src_al[1], 2.2f);
-  al.z = powf_(src_al[2], 2.2f);
-  al.w = powf_(src_al[3], 2.2f);
-  em.x = powf_(src_em[0], 2.2f);
-  em.y = powf_(src_em[1], 2.2f);
-  em.z = powf_(src_em[2], 2.2f);
-  em.w = powf_(src_em[3], 2.2f);
-  reinterpret_cast<float4*>(albedo)[i] = al;
-  reinterpret_cast<float4*>(emissive)[i] = em;
-  reinterpret_cast<float4*>(normal)[i] = make_float4(h.n.x, h.n.y, h.n.z, 1.0f);
+  reinterpret_cast<float4*>(albedo)[i] = *reinterpret_cast<const float4*>(&colour[slot][0]);
+  reinterpret_cast<float4*>(emissive)[i] = *reinterpret_cast<const float4*>(&colour[slot][4]);
+  reinterpret_cast<float4*>(normal)[i] = make_float4(n.x, n.y, n.z, 1.0f);
   reinterpret_cast<float2*>(moments)[i] = make_float2(delta_len, delta_len * delta_len);
   ndc[i] = project(v.view_proj, hit).z;
 }
 
-__global__ void __launch_bounds__(kTx* kTy) shadow_kernel(const __grid_constant__ ViewArgs v,
-                                                          const gi_prim* __restrict__ prims, int np, MeshSet mesh,
-                                                          float* __restrict__ out) {
-  __shared__ gi_prim s_prims[kPrimStage];
-  const int x = blockIdx.x * kTx + threadIdx.x, y = blockIdx.y * kTy + threadIdx.y;
-  const bool live = x < v.width && y < v.height;
-  const int xc = live ? x : 0, yc = live ? y : 0;
-  const float sx = div_((float)xc + 0.5f, (float)v.width), sy = div_((float)yc + 0.5f, (float)v.height);
-  const float4 o4 = mat_vec(v.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
-  const f3 org = mk3(o4.x, o4.y, o4.z);
-  const f3 farp = unproject(v.inv_view_proj, sx, sy, 1.0f);
-  const f3 dir = normalize3(sub3(farp, org));
+__global__ void __launch_bounds__(kCastThreads) shadow_kernel(const __grid_constant__ ViewArgs v,
+                                                              const gi_prim* __restrict__ prims, int np, MeshSet mesh,
+                                                              float* __restrict__ out) {
+  __shared__ PrimTest s_prims[kPrimStage];
+  const CastPixel c = cast_pixel(v);
   Hit h;
-  cast_ray(prims, np, mesh, org, dir, h, s_prims);
-  if (!live) return;
+  cast_ray(prims, np, mesh, c.org, c.dir, h, s_prims);
+  if (!c.live) return;
   float z = 1.0f;
-  if (h.prim >= 0 || h.tri >= 0) z = project(v.view_proj, add3(org, mul3s(dir, h.t))).z;
-  out[(size_t)y * v.width + x] = z;
+  if (h.prim >= 0 || h.tri >= 0) z = project(v.view_proj, add3(c.org, mul3s(c.dir, h.t))).z;
+  out[(size_t)c.y * v.width + c.x] = z;
 }
 
 // directLighting.frag:45-79.
@@ -309,6 +476,7 @@ __global__ void __launch_bounds__(kTx* kTy) direct_kernel(const __grid_constant_
 }
 
 dim3 grid2d(int w, int h) { return dim3((w + kTx - 1) / kTx, (h + kTy - 1) / kTy); }
+dim3 cast_grid(int w, int h) { return dim3((w + kCastX - 1) / kCastX, (h + kCastY - 1) / kCastY); }
 
 }  // namespace
 }  // namespace gi
@@ -323,7 +491,7 @@ extern "C" int gi_gbuffer(const gi_view* view, const gi_prim* prims, int num_pri
   GI_CHECK_ARG(aligned16(albedo) && aligned16(emissive) && aligned16(normal) && aligned16(depth_moments),
                "gi_gbuffer: unaligned buffer");
   ViewArgs v = view_args(*view);
-  gbuffer_kernel<<<grid2d(v.width, v.height), dim3(kTx, kTy), 0, (cudaStream_t)stream>>>(
+  gbuffer_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
       v, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, albedo, emissive, normal, depth_moments, ndc_depth);
   GI_CHECK_LAUNCH("gbuffer_kernel");
   count_launches(1);
@@ -352,7 +520,7 @@ extern "C" int gi_gbuffer_mesh(const gi_view* view, const gi_prim* prims, int nu
   GI_CHECK_ARG(aligned16(albedo) && aligned16(emissive) && aligned16(normal) && aligned16(depth_moments),
                "gi_gbuffer_mesh: unaligned buffer");
   ViewArgs v = view_args(*view);
-  gbuffer_kernel<<<grid2d(v.width, v.height), dim3(kTx, kTy), 0, (cudaStream_t)stream>>>(
+  gbuffer_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
       v, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, albedo, emissive, normal, depth_moments, ndc_depth);
   GI_CHECK_LAUNCH("gbuffer_kernel");
   count_launches(1);
@@ -367,7 +535,7 @@ extern "C" int gi_shadow_map_mesh(const gi_view* light_view, const gi_prim* prim
   if (st) return st;
   GI_CHECK_ARG(cull == GI_CULL_NONE || cull == GI_CULL_BACK, "gi_shadow_map_mesh: unknown cull mode");
   ViewArgs v = view_args(*light_view);
-  shadow_kernel<<<grid2d(v.width, v.height), dim3(kTx, kTy), 0, (cudaStream_t)stream>>>(
+  shadow_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
       v, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, shadow);
   GI_CHECK_LAUNCH("shadow_kernel");
   count_launches(1);
@@ -379,7 +547,7 @@ extern "C" int gi_shadow_map(const gi_view* light_view, const gi_prim* prims, in
   GI_CHECK_ARG(light_view && prims && shadow, "gi_shadow_map: null");
   GI_CHECK_ARG(num_prims >= 1 && num_prims <= GI_MAX_PRIMS, "gi_shadow_map: bad primitive count");
   ViewArgs v = view_args(*light_view);
-  shadow_kernel<<<grid2d(v.width, v.height), dim3(kTx, kTy), 0, (cudaStream_t)stream>>>(
+  shadow_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
       v, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, shadow);
   GI_CHECK_LAUNCH("shadow_kernel");
   count_launches(1);
