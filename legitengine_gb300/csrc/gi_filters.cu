@@ -23,32 +23,63 @@ template <int DCH> __device__ __forceinline__ float depth_at(const float* p, int
 // exponential of the summed exponents; out = sum / (sumW + 1e-7).  The block's
 // (32+4) x (16+4) halo of light, depth and normal is staged in shared memory
 // (clamp-to-edge applied while staging), so every tap is a shared-memory read.
-// Each thread filters kBilRows vertically adjacent pixels: their windows share
-// tap rows, so a thread reads kBilRows + 4 rows of taps for kBilRows outputs
-// instead of 5 kBilRows (the kernel is bound by the shared-memory reads); each
-// output still sums its taps in the order above.  Two rows measured best at 1080p:
-// 88.7 us against 96.9 (three) and 101.0 (four; larger halo tiles and registers).
+// Each thread filters two vertically adjacent pixels: their windows share tap rows,
+// so a thread reads 6 rows of taps for its two outputs instead of 10, and the two
+// pixels' weights and sums are the halves of packed operations; each output still
+// sums its taps in the order above, with the same roundings.
+//
+// Bound by arithmetic.  The exact weight's exponential (expf_ without its branches:
+// here the argument is never positive) rounds and scales by packed adds and multiplies
+// instead of conversions and integer arithmetic: 3840 x 2160 315 -> 241 us (362 M
+// instructions before); the fast weights at 1920 x 1080 49.7 -> 47.5 us.
 constexpr int kBilRows = 2;
 constexpr int kHx = kTx + 4, kHy = kTy * kBilRows + 4;
 
-// FAST (the march's fast precision): the weights by the hardware exponential
-// (__expf) and the sums by fused multiply-adds.
-template <bool FAST>
-__device__ __forceinline__ void bilateral_tap(const float4& col, const float4& n, const float4& c, float4& acc) {
-  const float ndx = n.x - c.x, ndy = n.y - c.y, ndz = n.z - c.z;
+// expf_(-s) of both halves for s >= 0 or NaN, bit for bit.
+__device__ __forceinline__ p2 exp_neg(p2 s) {
+  // From 104 on expf_ gives 0, as 105 does here.
+  float a, b;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(lo_(s)), "f"(105.0f));
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(b) : "f"(hi_(s)), "f"(105.0f));
+  const p2 x = pk(a, b);
+  // n = the nearest integer to -s log2 e (ties to even): the sum's spacing is 1 and its
+  // low 8 bits are n + 192, in [40, 192].
+  constexpr float kRound = 12582912.0f + 192.0f;
+  const p2 t = padd(pmul(x, pk(-kLog2e)), pk(kRound));
+  const p2 n = psub(t, pk(kRound));
+  // q = -r of expf_, and its series with the signs of the odd terms turned.
+  p2 q = pfma(n, pk(kLn2Hi), x);
+  q = pfma(n, pk(kLn2Lo), q);
+  p2 p = pfma(q, pk(-(1.0f / 40320.0f)), pk(1.0f / 5040.0f));
+  p = pfma(q, p, pk(-(1.0f / 720.0f)));
+  p = pfma(q, p, pk(1.0f / 120.0f));
+  p = pfma(q, p, pk(-(1.0f / 24.0f)));
+  p = pfma(q, p, pk(1.0f / 6.0f));
+  p = pfma(q, p, pk(-0.5f));
+  p = pfma(q, p, pk(1.0f));
+  p = pfma(q, p, pk(-1.0f));
+  // -p 2^n as (p 2^(n + 65)) 2^-65: one rounding, in the subnormal range, as in ldexp_.
+  const p2 scale = pk(__uint_as_float(__float_as_uint(lo_(t)) << 23), __uint_as_float(__float_as_uint(hi_(t)) << 23));
+  return pmul(pmul(p, scale), pk(-2.7105054312137611e-20f));
+}
+
+// The weights of a tap of each pixel from the differences to their centres.  FAST (the
+// march's fast precision): by fused multiply-adds and the hardware exponential.
+template <bool FAST> __device__ __forceinline__ p2 bilateral_weights(p2 x, p2 y, p2 z, p2 d) {
   if (FAST) {
-    const float wt = __expf(-fmaf(fabsf(n.w - c.w), 10.5f, fmaf(ndz, ndz, fmaf(ndy, ndy, ndx * ndx)) * 20.0f));
-    acc.x = fmaf(col.x, wt, acc.x);
-    acc.y = fmaf(col.y, wt, acc.y);
-    acc.z = fmaf(col.z, wt, acc.z);
-    acc.w = acc.w + wt;
-  } else {
-    const float wt = expf_(-(fabsf(n.w - c.w) * 10.5f + (ndx * ndx + ndy * ndy + ndz * ndz) * 20.0f));
-    acc.x = acc.x + col.x * wt;
-    acc.y = acc.y + col.y * wt;
-    acc.z = acc.z + col.z * wt;
-    acc.w = acc.w + wt;
+    const p2 m = pmul(pfma(z, z, pfma(y, y, pmul(x, x))), pk(20.0f));
+    return pk(__expf(-fmaf(fabsf(lo_(d)), 10.5f, lo_(m))), __expf(-fmaf(fabsf(hi_(d)), 10.5f, hi_(m))));
   }
+  const p2 m = pmul(padd(padd(pmul(x, x), pmul(y, y)), pmul(z, z)), pk(20.0f));
+  d = pmul(d, pk(10.5f));
+  return exp_neg(pk(fabsf(lo_(d)) + lo_(m), fabsf(hi_(d)) + hi_(m)));
+}
+
+template <bool FAST> __device__ __forceinline__ float weigh(float sum, float v, float w) {
+  return FAST ? fmaf(v, w, sum) : sum + v * w;
+}
+template <bool FAST> __device__ __forceinline__ p2 weigh(p2 sum, float v, p2 w) {
+  return FAST ? pfma(pk(v), w, sum) : padd(sum, pmul(pk(v), w));
 }
 
 template <int DCH, bool FAST>
@@ -68,35 +99,58 @@ __global__ void __launch_bounds__(kTx* kTy) bilateral_kernel(const float* __rest
     s_nrm[hy][hx] = n;
   }
   __syncthreads();
-  const int x = blockIdx.x * kTx + threadIdx.x;
-  const int ty = threadIdx.y * kBilRows;  // first of the thread's rows within the tile
-  const int y = blockIdx.y * (kTy * kBilRows) + ty;
+  const int tx = threadIdx.x, ty = threadIdx.y * kBilRows;  // the thread's first tap within the tile
+  const int x = blockIdx.x * kTx + tx, y = blockIdx.y * (kTy * kBilRows) + ty;
   if (x >= w || y >= h) return;
-  float4 c[kBilRows], acc[kBilRows];
+  const float4 c0 = s_nrm[ty + 2][tx + 2], c1 = s_nrm[ty + 3][tx + 2];
+  // Row 0 belongs to the upper pixel alone and row 5 to the lower one: their weights
+  // make a pair, and the lower pixel's wait for its last row.
+  float sx = 0.0f, sy = 0.0f, sz = 0.0f, sw = 0.0f, last[5];
 #pragma unroll
-  for (int k = 0; k < kBilRows; k++) {
-    c[k] = s_nrm[ty + 2 + k][threadIdx.x + 2];
-    acc[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int dx = 0; dx < 5; dx++) {
+    const float4 col = s_col[ty][tx + dx], n = s_nrm[ty][tx + dx], m = s_nrm[ty + 5][tx + dx];
+    const p2 wt = bilateral_weights<FAST>(pk(n.x - c0.x, m.x - c1.x), pk(n.y - c0.y, m.y - c1.y),
+                                          pk(n.z - c0.z, m.z - c1.z), pk(n.w - c0.w, m.w - c1.w));
+    sx = weigh<FAST>(sx, col.x, lo_(wt));
+    sy = weigh<FAST>(sy, col.y, lo_(wt));
+    sz = weigh<FAST>(sz, col.z, lo_(wt));
+    sw = sw + lo_(wt);
+    last[dx] = hi_(wt);
   }
+  const p2 cx = pk(c0.x, c1.x), cy = pk(c0.y, c1.y), cz = pk(c0.z, c1.z), cd = pk(c0.w, c1.w);
+  p2 ax = pk(sx, 0.0f), ay = pk(sy, 0.0f), az = pk(sz, 0.0f), aw = pk(sw, 0.0f);
 #pragma unroll
-  for (int r = 0; r < 5 + kBilRows - 1; r++) {  // tap rows of the windows, top to bottom
+  for (int r = 1; r < 5; r++) {
 #pragma unroll
     for (int dx = 0; dx < 5; dx++) {
-      const float4 col = s_col[ty + r][threadIdx.x + dx];
-      const float4 n = s_nrm[ty + r][threadIdx.x + dx];
-#pragma unroll
-      for (int k = 0; k < kBilRows; k++)  // output k's window holds tap rows k .. k + 4
-        if (r >= k && r < k + 5) bilateral_tap<FAST>(col, n, c[k], acc[k]);
+      const float4 col = s_col[ty + r][tx + dx], n = s_nrm[ty + r][tx + dx];
+      const p2 wt = bilateral_weights<FAST>(psub(pk(n.x), cx), psub(pk(n.y), cy), psub(pk(n.z), cz), psub(pk(n.w), cd));
+      ax = weigh<FAST>(ax, col.x, wt);
+      ay = weigh<FAST>(ay, col.y, wt);
+      az = weigh<FAST>(az, col.z, wt);
+      aw = padd(aw, wt);
     }
   }
-  float4* o = reinterpret_cast<float4*>(out);
+  float4* o = reinterpret_cast<float4*>(out) + (size_t)y * w + x;
+  auto store = [](float4* at, float vx, float vy, float vz, float vw) {
+    const float d = vw + 1e-7f;
+    *at = make_float4(div_(vx, d), div_(vy, d), div_(vz, d), 1.0f);
+  };
+  store(o, lo_(ax), lo_(ay), lo_(az), lo_(aw));
+  if (y + 1 >= h) return;
+  sx = hi_(ax);
+  sy = hi_(ay);
+  sz = hi_(az);
+  sw = hi_(aw);
 #pragma unroll
-  for (int k = 0; k < kBilRows; k++) {
-    if (y + k < h) {
-      const float d = acc[k].w + 1e-7f;
-      o[(size_t)(y + k) * w + x] = make_float4(div_(acc[k].x, d), div_(acc[k].y, d), div_(acc[k].z, d), 1.0f);
-    }
+  for (int dx = 0; dx < 5; dx++) {
+    const float4 col = s_col[ty + 5][tx + dx];
+    sx = weigh<FAST>(sx, col.x, last[dx]);
+    sy = weigh<FAST>(sy, col.y, last[dx]);
+    sz = weigh<FAST>(sz, col.z, last[dx]);
+    sw = sw + last[dx];
   }
+  store(o + w, sx, sy, sz, sw);
 }
 
 // denoiser.frag:72-184 with radius 2: 16 equations [depth, 1] -> colour over
