@@ -465,90 +465,114 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
 //
 // mlp_train_tc_kernel: forward with saved activations, the head's loss gradient,
 // backward through every layer and the weight gradients, for 128-pixel tiles
-// (persistent: one CTA of 128 threads per SM walks the batch's tiles).  Thread i
-// owns pixel i of a tile: row i of every layer's A operand and lane i of the
-// accumulators.  Products of a tile (A = M x K, B = N x K, both K-major without
-// swizzle, D in tensor memory, M = 128):
+// (persistent: one CTA of 256 threads per SM walks the batch's tiles).  Threads i
+// and i + 128 own pixel i of a tile -- row i of every layer's operand and lane i of
+// the accumulators -- and half of its columns each.  Products of a tile (D in tensor
+// memory, M = 128):
 //   forward   Z = A_l W_l             A = X / H1 / H2 / H3 (pixels x features)
-//   backward  dH = dZ_l W_l^T         A = dZ (pixels x outputs), B = W_l as (in x out)
-//   gradient  dW_l += H_{l-1}^T dZ_l  A = H^T (features x pixels), B = dZ^T
-//                                     (outputs x pixels): the pixels are the
-//                                     reduction, and dW accumulates over every
-//                                     tile of the CTA in tensor memory (M = 128:
-//                                     rows past the layer's inputs read the
-//                                     next buffer and are never read back).
-// Epilogues (one thread per pixel, its own accumulator lane): bias and ReLU to
-// bf16 (forward; the transposed copy H^T written beside the row), the head's
-// loss gradient (layer 4), the ReLU mask of the backward (dZ = dH where H > 0).
-// Bias gradients are the column sums of the bf16 dZ (shared memory).  At the end
-// each CTA adds its gradient sums to `grads` (atomic FP32 additions) and its loss.
+//   backward  dH = dZ_l W_l^T         A = dZ (pixels x outputs)
+//   gradient  dW_l += H_{l-1}^T dZ_l  the pixels are the reduction, and dW
+//                                     accumulates over every tile of the CTA in
+//                                     tensor memory (M = 128: rows past the layer's
+//                                     inputs read the next bytes and are never read
+//                                     back)
+//             db_l += 1^T dZ_l        a constant operand of ones
+// Every operand is stored once, as 8 x 8 core matrices of rows (pixels, or a weight's
+// inputs) by 8 consecutive columns, and the descriptors name its K axis: along the
+// columns (K-major: forward and backward A, backward B) or along the rows (MN-major:
+// forward B, both gradient operands).
+// Epilogues (two threads per pixel): bias and ReLU to bf16 (forward), the head's loss
+// gradient (layer 4), the ReLU mask of the backward (dZ = dH where H > 0).  A layer's
+// gradient products run behind the next epilogue: only the layer's accumulator is
+// waited for, and each layer has its own dZ.  At the end each CTA adds its gradient
+// sums to `grads` (16-byte reductions) and its loss.
 // Arithmetic: bf16 operands (inputs, weights, hidden activations, the logits'
 // gradient and the masked hidden gradients), FP32 accumulation, FP32 bias and
 // head; the sums run in the tensor cores' order.
-constexpr int kTrThreads = 128;
-constexpr int uF1 = 0;                            // W1 as 64 x 32 (out x in)
-constexpr int uF2 = uF1 + kHid * kIn * 2;          // W2 as 64 x 64
-constexpr int uF3 = uF2 + kHid * kHid * 2;
-constexpr int uF4 = uF3 + kHid * kHid * 2;         // W4 as 16 x 64 (rows 3-15 zero)
-constexpr int uB2 = uF4 + kOutPad * kHid * 2;      // W2 as 64 x 64 (in x out)
-constexpr int uB3 = uB2 + kHid * kHid * 2;
-constexpr int uB4 = uB3 + kHid * kHid * 2;         // W4 as 64 x 16 (in x out, outputs 3-15 zero)
-constexpr int uX = uB4 + kHid * kOutPad * 2;       // 128 x 32
+//
+// Bound by latency: a tile is a chain of 8 products and epilogues, and batches to
+// 19 456 pixels are one tile per SM.  16 384 rows: 71.7 -> 18.5 us against 128 threads a tile, transposed
+// copies of every operand, column sums in a loop and one addition per value.
+constexpr int kTrThreads = 256;
+constexpr int uW1 = 0;                             // weights, inputs x outputs
+constexpr int uW2 = uW1 + kHid * kIn * 2;
+constexpr int uW3 = uW2 + kHid * kHid * 2;
+constexpr int uW4 = uW3 + kHid * kHid * 2;         // 64 x 16 (outputs 3-15 zero)
+constexpr int uX = uW4 + kHid * kOutPad * 2;       // 128 x 32
 constexpr int uH1 = uX + kRows * kIn * 2;          // 128 x 64 each
 constexpr int uH2 = uH1 + kRows * kHid * 2;
 constexpr int uH3 = uH2 + kRows * kHid * 2;
-constexpr int uDY = uH3 + kRows * kHid * 2;        // 128 x 16
-constexpr int uDZ = uDY + kRows * kOutPad * 2;     // 128 x 64
-constexpr int uXt = uDZ + kRows * kHid * 2;        // 32 x 128 (features x pixels)
-constexpr int uH1t = uXt + kIn * kRows * 2;        // 64 x 128 each
-constexpr int uH2t = uH1t + kHid * kRows * 2;
-constexpr int uH3t = uH2t + kHid * kRows * 2;
-constexpr int uDZt = uH3t + kHid * kRows * 2;      // 64 x 128 (outputs x pixels)
-constexpr int uDYt = uDZt + kHid * kRows * 2;      // 16 x 128
-constexpr int uBar = uDYt + kOutPad * kRows * 2;
-constexpr int uFail = uBar + 8;
+constexpr int uDY = uH3 + kRows * kHid * 2;        // 128 x 16 (outputs 3-15 zero)
+constexpr int uZ1 = uDY + kRows * kOutPad * 2;     // 128 x 64 each: dZ
+constexpr int uZ2 = uZ1 + kRows * kHid * 2;
+constexpr int uZ3 = uZ2 + kRows * kHid * 2;
+constexpr int uOne = uZ3 + kRows * kHid * 2;       // one core matrix of ones
+constexpr int uBias = uOne + 128;                  // b1, b2, b3 (64 floats each), b4
+constexpr int uBar = uBias + (3 * kHid + 4) * 4;   // two mbarriers: the layer's accumulator; a tile's gradients
+constexpr int uFail = uBar + 16;
 constexpr int uTmem = uFail + 4;
 constexpr int kSmemTrainTc = uTmem + 4;
-// A 128-row gradient operand reads 128 rows of 256 bytes from its start: the
-// buffers after Xt (24 KB) and after each H^T (16 KB) stay inside the allocation.
-static_assert(uXt + kRows * kRows * 2 <= kSmemTrainTc && uH3t + kRows * kRows * 2 <= kSmemTrainTc,
-              "gradient operand reads stay in shared memory");
-static_assert(uX % 128 == 0 && uDY % 128 == 0 && uXt % 128 == 0 && uDYt % 128 == 0 && uBar % 8 == 0, "alignment");
-// Tensor-memory columns: the layer accumulator and the four weight-gradient sums.
-constexpr uint32_t cZ = 0, cW1 = 64, cW2 = 128, cW3 = 192, cW4 = 256, kTrTmemCols = 512;
+// A gradient operand of M = 128 rows reads 16 core matrices (2 KB) from each of its
+// pixel groups' starts.
+static_assert(uH3 + kRows * kHid * 2 + 2048 <= kSmemTrainTc, "gradient operand reads stay in shared memory");
+static_assert(uX % 128 == 0 && uDY % 128 == 0 && uZ1 % 128 == 0 && uOne % 128 == 0 && uBias % 16 == 0 &&
+                  uBar % 8 == 0,
+              "alignment");
+static_assert(ob1 % 4 == 0 && oW2 % 4 == 0 && ob2 % 4 == 0 && oW3 % 4 == 0 && ob3 % 4 == 0 && oW4 % 4 == 0,
+              "16-byte reductions");
+// Tensor-memory columns: the layer accumulator, the weight-gradient sums and the
+// bias-gradient sums (every row the same).
+constexpr uint32_t cZ = 0, cW1 = 64, cW2 = 128, cW3 = 192, cW4 = 256, cB3 = 288, cB2 = 352, cB1 = 416, cB4 = 480,
+                   kTrTmemCols = 512;
 
-// Element (r, k) of an R x K K-major operand, as bf16 at smem + base.
-__device__ __forceinline__ void st_bf16(unsigned char* smem, int base, int r, int k, int K, bf16 v) {
-  *reinterpret_cast<bf16*>(smem + base + cm_off(r, k, K)) = v;
-}
-
-// Row `m` of a 128 x K operand from 8-value packs (v4 stores).
-template <int K>
-__device__ __forceinline__ void st_row(uint32_t sbase, int base, int m, const uint32_t (&packs)[K / 2]) {
-#pragma unroll
-  for (int c = 0; c < K; c += 8)
-    st_shared_v4(sbase + base + cm_off(m, c, K), packs[c / 2], packs[c / 2 + 1], packs[c / 2 + 2], packs[c / 2 + 3]);
-}
-
-// Column `m` of the transposed K x 128 operand (one bf16 per feature).
-template <int K>
-__device__ __forceinline__ void st_col(unsigned char* smem, int base, int m, const uint32_t (&packs)[K / 2]) {
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const uint32_t w = packs[k / 2];
-    const unsigned short h = (k & 1) ? (unsigned short)(w >> 16) : (unsigned short)(w & 0xFFFFu);
-    *reinterpret_cast<unsigned short*>(smem + base + cm_off(k, m, kRows)) = h;
-  }
-}
+// An operand in shared memory: its start, the distances of core matrices adjacent along
+// K and along M (or N), and whether K runs along the rows (MN-major).  An MMA consumes
+// two core matrices along K.
+struct Operand {
+  uint32_t at, k, mn;
+  bool rows;
+};
+template <int W> __device__ __forceinline__ Operand along_columns(uint32_t at) { return Operand{at, 128, W * 16, false}; }
+template <int W> __device__ __forceinline__ Operand along_rows(uint32_t at) { return Operand{at, W * 16, 128, true}; }
 
 // K/16 MMAs of A (M = 128 x K) and B (N x K) into D; `first` clears D.
 template <int K, int N>
-__device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint32_t b, bool first) {
-  constexpr uint32_t idesc = idesc_bf16(kRows, N);
+__device__ __forceinline__ void mma_chain(uint32_t d, const Operand& a, const Operand& b, bool first) {
+  const uint32_t idesc = idesc_bf16(kRows, N) | (a.rows ? 1u << 15 : 0u) | (b.rows ? 1u << 16 : 0u);
 #pragma unroll
   for (int j = 0; j < K / 16; j++)
-    mma_bf16(d, smem_desc(a + j * 256, 128, K * 16), smem_desc(b + j * 256, 128, K * 16), idesc,
+    mma_bf16(d, smem_desc(a.at + 2 * j * a.k, a.k, a.mn), smem_desc(b.at + 2 * j * b.k, b.k, b.mn), idesc,
              (first && j == 0) ? 0u : 1u);
+}
+
+// A K x N weight matrix (bf16, row-major, N columns) as core matrices of 8 rows x 8 columns.
+template <int K, int N>
+__device__ __forceinline__ void stage_weights(uint32_t dst, const bf16* __restrict__ w) {
+#pragma unroll
+  for (int i = threadIdx.x; i < K * N / 8; i += kTrThreads) {
+    const int k = i / (N / 8), c = i % (N / 8);
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(w) + i);
+    st_shared_v4(dst + cm_off(k, 8 * c, N), q.x, q.y, q.z, q.w);
+  }
+}
+
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 q;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
+               : "r"(addr)
+               : "memory");
+  return q;
+}
+
+// *p += v for four consecutive floats (16-byte aligned), one reduction.
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
+__device__ __forceinline__ void red_add32(float* p, const float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) red_add4(p + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
 }
 
 __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16* __restrict__ feats,
@@ -561,30 +585,24 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t bar = sbase + uBar;
+  const int row = tid & (kRows - 1), half = tid >> 7;  // the thread's pixel, and its half of the columns
+  const uint32_t layer_bar = sbase + uBar, grad_bar = layer_bar + 8;
   volatile int* fail = reinterpret_cast<volatile int*>(smem + uFail);
+  const float* bias = reinterpret_cast<const float*>(smem + uBias);
 
-  // Weights: forward B (out x in) and backward B (in x out), K-major.
-  for (int i = tid; i < kHid * kIn; i += kTrThreads) {  // W1 [32 x 64]
-    const int k = i / kHid, o = i % kHid;
-    st_bf16(smem, uF1, o, k, kIn, wb[qW1 + i]);
+  stage_weights<kIn, kHid>(sbase + uW1, wb + qW1);
+  stage_weights<kHid, kHid>(sbase + uW2, wb + qW2);
+  stage_weights<kHid, kHid>(sbase + uW3, wb + qW3);
+  stage_weights<kHid, kOutPad>(sbase + uW4, wb + qW4);
+  if (tid < 3 * kHid + kOut) {
+    const int l = tid >> 6, at = tid & (kHid - 1);
+    const int from = (l == 0 ? ob1 : l == 1 ? ob2 : l == 2 ? ob3 : ob4) + at;
+    reinterpret_cast<float*>(smem + uBias)[tid] = __ldg(params + from);
   }
-  for (int i = tid; i < kHid * kHid; i += kTrThreads) {
-    const int k = i / kHid, o = i % kHid;
-    st_bf16(smem, uF2, o, k, kHid, wb[qW2 + i]);
-    st_bf16(smem, uF3, o, k, kHid, wb[qW3 + i]);
-    st_bf16(smem, uB2, k, o, kHid, wb[qW2 + i]);
-    st_bf16(smem, uB3, k, o, kHid, wb[qW3 + i]);
-  }
-  for (int i = tid; i < kHid * kOutPad; i += kTrThreads) {  // W4 [64 x 16]
-    const int k = i / kOutPad, o = i % kOutPad;
-    st_bf16(smem, uF4, o, k, kHid, wb[qW4 + i]);
-    st_bf16(smem, uB4, k, o, kOutPad, wb[qW4 + i]);
-  }
-  for (int i = tid; i < kOutPad * kRows; i += kTrThreads)  // dY^T: outputs 3-15 stay zero
-    *reinterpret_cast<bf16*>(smem + uDYt + 2 * i) = __float2bfloat16_rn(0.0f);
+  if (tid < 64) reinterpret_cast<bf16*>(smem + uOne)[tid] = __float2bfloat16_rn(1.0f);
   if (tid == 0) {
-    mbar_init(bar, 1);
+    mbar_init(layer_bar, 1);
+    mbar_init(grad_bar, 1);
     *fail = 0;
   }
   if (warp == 0) {
@@ -597,114 +615,116 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   __syncthreads();
   fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + uTmem);
-  const uint32_t lane = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 accumulator lanes
-  uint32_t phase = 0;
-  bool failed = false, first = true;
-  float lsum = 0.0f, gb1 = 0.0f, gb2 = 0.0f, gb3 = 0.0f, gb4 = 0.0f;
-  const float b40 = params[ob4 + 0], b41 = params[ob4 + 1], b42 = params[ob4 + 2];
+  const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 accumulator lanes
+  const uint32_t mine = lane + 32 * half;                            // and its columns of a 64-column accumulator
+  uint32_t layer_phase = 0, grad_phase = 0;
+  bool first = true;
+  float lsum = 0.0f;
 
-  // Shared-memory writes -> the tensor cores -> `issue` on thread 0 -> commit, wait.
-  auto mma_round = [&](auto issue) {
+  // A bounded wait of every thread.  One that runs out is recorded and the tile goes on
+  // (with values that are not used), so that the threads stay together; the later
+  // waits then return at once.
+  auto wait = [&](uint32_t bar, uint32_t& phase) {
+    if (!*fail && !mbar_wait(bar, phase)) *fail = 1;
+    phase ^= 1u;
+  };
+  // Shared-memory writes -> the tensor cores -> `layer` (the layer's accumulator) and
+  // `grad` (left running) on thread 0 -> wait for the accumulator.
+  auto mma_round = [&](auto layer, auto grad) {
     fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
     if (tid == 0) {
-      issue();
-      mma_commit(bar);
-      if (!mbar_wait(bar, phase)) *fail = 1;
-      fence_before();
+      layer();
+      mma_commit(layer_bar);
+      grad();
     }
-    phase ^= 1u;
-    __syncthreads();
+    wait(layer_bar, layer_phase);
     fence_after();
-    return *fail == 0;
   };
-  // Layer accumulator -> + bias -> ReLU -> bf16 row and column of the next operand.
-  auto forward_epilogue = [&](int row_buf, int col_buf, const float* __restrict__ bias) {
-    uint32_t packs[kHid / 2];
+  auto nothing = [] {};
+  // Layer accumulator -> + bias -> ReLU -> bf16 row of the next operand.
+  auto forward_epilogue = [&](int buf, const float* b) {
+    float v[32];
+    tmem_ld32(mine + cZ, v);
 #pragma unroll
-    for (int c = 0; c < kHid; c += 32) {
-      float v[32];
-      tmem_ld32(lane + cZ + c, v);
-#pragma unroll
-      for (int h = 0; h < 32; h += 2)
-        packs[(c + h) / 2] = pack_relu_bf16(v[h] + __ldg(bias + c + h), v[h + 1] + __ldg(bias + c + h + 1));
+    for (int c = 0; c < 32; c += 8) {
+      const float4 b0 = *reinterpret_cast<const float4*>(b + 32 * half + c);
+      const float4 b1 = *reinterpret_cast<const float4*>(b + 32 * half + c + 4);
+      st_shared_v4(sbase + buf + cm_off(row, 32 * half + c, kHid), pack_relu_bf16(v[c] + b0.x, v[c + 1] + b0.y),
+                   pack_relu_bf16(v[c + 2] + b0.z, v[c + 3] + b0.w),
+                   pack_relu_bf16(v[c + 4] + b1.x, v[c + 5] + b1.y),
+                   pack_relu_bf16(v[c + 6] + b1.z, v[c + 7] + b1.w));
     }
-    st_row<kHid>(sbase, row_buf, tid, packs);
-    st_col<kHid>(smem, col_buf, tid, packs);
   };
-  // dH (accumulator) masked by the ReLU of the layer's output (bf16 row in smem) -> dZ.
-  auto backward_epilogue = [&](int h_buf) {
-    uint32_t packs[kHid / 2];
+  // dH (accumulator) masked by the ReLU of the layer's output H (its bf16 row) -> dZ.
+  auto backward_epilogue = [&](int h_buf, int z_buf) {
+    float v[32];
+    tmem_ld32(mine + cZ, v);
 #pragma unroll
-    for (int c = 0; c < kHid; c += 32) {
-      float v[32];
-      tmem_ld32(lane + cZ + c, v);
+    for (int c = 0; c < 32; c += 8) {
+      const int at = cm_off(row, 32 * half + c, kHid);
+      const uint4 q = ld_shared_v4(sbase + h_buf + at);
+      const uint32_t h[4] = {q.x, q.y, q.z, q.w};
+      uint32_t z[4];
 #pragma unroll
-      for (int h = 0; h < 32; h += 2) {
-        const uint32_t hp =
-            *reinterpret_cast<const uint32_t*>(smem + h_buf + cm_off(tid, c + h, kHid));  // H[tid][c+h], [c+h+1]
-        const float g0 = (hp & 0xFFFFu) && !(hp & 0x8000u) ? v[h] : 0.0f;      // bf16 > 0
-        const float g1 = (hp >> 16) && !(hp & 0x80000000u) ? v[h + 1] : 0.0f;
-        packs[(c + h) / 2] = pack_bf16(g0, g1);
+      for (int k = 0; k < 4; k++) {
+        const float g0 = (h[k] & 0xFFFFu) && !(h[k] & 0x8000u) ? v[c + 2 * k] : 0.0f;  // bf16 > 0
+        const float g1 = (h[k] >> 16) && !(h[k] & 0x80000000u) ? v[c + 2 * k + 1] : 0.0f;
+        z[k] = pack_bf16(g0, g1);
       }
+      st_shared_v4(sbase + z_buf + at, z[0], z[1], z[2], z[3]);
     }
-    st_row<kHid>(sbase, uDZ, tid, packs);
-    st_col<kHid>(smem, uDZt, tid, packs);
   };
-  // Column sum of the bf16 dZ rows (threads 0..cols-1), after the rows are written.
-  auto column_sum = [&](int buf, int K, int cols) {
-    float sum = 0.0f;
-    if (tid < cols)
-      for (int r = 0; r < kRows; r++) sum += __bfloat162float(*reinterpret_cast<const bf16*>(smem + buf + cm_off(r, tid, K)));
-    return sum;
-  };
+  const Operand ones{sbase + uOne, 0, 0, false};
 
   const int tiles = (n + kRows - 1) / kRows;
-  for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
-    const int p = t * kRows + tid;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int p = t * kRows + row;
     const bool valid = p < n;
-    // Features: row and column of X; targets divided by the exposure scale.
-    uint32_t xp[kIn / 2];
-    {
-      const uint4* src = reinterpret_cast<const uint4*>(feats + (size_t)p * kIn);
-#pragma unroll
-      for (int c = 0; c < kIn / 8; c++) {
-        const uint4 q = valid ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-        xp[4 * c] = q.x;
-        xp[4 * c + 1] = q.y;
-        xp[4 * c + 2] = q.z;
-        xp[4 * c + 3] = q.w;
-      }
-    }
-    st_row<kIn>(sbase, uX, tid, xp);
-    st_col<kIn>(smem, uXt, tid, xp);
+    // Half the feature row each; the targets, divided by the exposure scale, of the
+    // threads that evaluate the head.
+    uint4 x[2];
     float T[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (valid) {
-      const float sc = scale ? __ldg(scale + p) : 1.0f;
 #pragma unroll
-      for (int c = 0; c < 3; c++) T[c] = scale ? __ldg(targets + (size_t)p * 4 + c) / sc : __ldg(targets + (size_t)p * 4 + c);
-      T[3] = __ldg(targets + (size_t)p * 4 + 3);
+    for (int c = 0; c < 2; c++)
+      x[c] = valid ? __ldg(reinterpret_cast<const uint4*>(feats + (size_t)p * kIn) + 2 * half + c)
+                   : make_uint4(0u, 0u, 0u, 0u);
+    if (valid && half == 0) {
+      const float sc = scale ? __ldg(scale + p) : 1.0f;
+      const float4 q = __ldg(reinterpret_cast<const float4*>(targets) + p);
+      T[0] = scale ? q.x / sc : q.x;
+      T[1] = scale ? q.y / sc : q.y;
+      T[2] = scale ? q.z / sc : q.z;
+      T[3] = q.w;
     }
-    auto xval = [&](int k) {
-      const uint32_t w = xp[k / 2];
-      return __uint_as_float(((k & 1) ? (w >> 16) : (w & 0xFFFFu)) << 16);
-    };
+    if (!first) wait(grad_bar, grad_phase);  // the previous tile's operands are free
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      st_shared_v4(sbase + uX + cm_off(row, 16 * half + 8 * c, kIn), x[c].x, x[c].y, x[c].z, x[c].w);
 
-    if (!mma_round([&] { mma_chain<kIn, kHid>(tmem + cZ, sbase + uX, sbase + uF1, true); })) break;
-    forward_epilogue(uH1, uH1t, params + ob1);
-    if (!mma_round([&] { mma_chain<kHid, kHid>(tmem + cZ, sbase + uH1, sbase + uF2, true); })) break;
-    forward_epilogue(uH2, uH2t, params + ob2);
-    if (!mma_round([&] { mma_chain<kHid, kHid>(tmem + cZ, sbase + uH2, sbase + uF3, true); })) break;
-    forward_epilogue(uH3, uH3t, params + ob3);
-    if (!mma_round([&] { mma_chain<kHid, kOutPad>(tmem + cZ, sbase + uH3, sbase + uF4, true); })) break;
-    // Head: the loss gradient at the logits -> dY (row and column).
-    {
+    mma_round([&] { mma_chain<kIn, kHid>(tmem + cZ, along_columns<kIn>(sbase + uX), along_rows<kHid>(sbase + uW1), true); },
+              nothing);
+    forward_epilogue(uH1, bias);
+    mma_round([&] { mma_chain<kHid, kHid>(tmem + cZ, along_columns<kHid>(sbase + uH1), along_rows<kHid>(sbase + uW2), true); },
+              nothing);
+    forward_epilogue(uH2, bias + kHid);
+    mma_round([&] { mma_chain<kHid, kHid>(tmem + cZ, along_columns<kHid>(sbase + uH2), along_rows<kHid>(sbase + uW3), true); },
+              nothing);
+    forward_epilogue(uH3, bias + 2 * kHid);
+    mma_round(
+        [&] { mma_chain<kHid, kOutPad>(tmem + cZ, along_columns<kHid>(sbase + uH3), along_rows<kOutPad>(sbase + uW4), true); },
+        nothing);
+    // Head: the loss gradient at the logits -> dY.
+    if (half == 0) {
       float z[16];
       tmem_ld16(lane + cZ, z);
-      const float lo[3] = {z[0] + b40, z[1] + b41, z[2] + b42};
+      const float lo[3] = {z[0] + bias[3 * kHid], z[1] + bias[3 * kHid + 1], z[2] + bias[3 * kHid + 2]};
       float c[3][3], d[3] = {0.0f, 0.0f, 0.0f};
+      auto xval = [&](int k) {
+        return __bfloat162float(*reinterpret_cast<const bf16*>(smem + uX + cm_off(row, k, kIn)));
+      };
 #pragma unroll
       for (int ch = 0; ch < 3; ch++) {
         c[0][ch] = xval(kCand0 + ch);
@@ -714,79 +734,81 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
       const float l = head_loss_grad_logits(lo, c, T, d, loss_kind);
       if (valid) lsum += l;
       else d[0] = d[1] = d[2] = 0.0f;
-      uint32_t dy[kOutPad / 2] = {pack_bf16(d[0], d[1]), pack_bf16(d[2], 0.0f), 0u, 0u, 0u, 0u, 0u, 0u};
-      st_row<kOutPad>(sbase, uDY, tid, dy);
-#pragma unroll
-      for (int o = 0; o < 3; o++)
-        st_bf16(smem, uDYt, o, tid, kRows, __float2bfloat16_rn(d[o]));
+      st_shared_v4(sbase + uDY + cm_off(row, 0, kOutPad), pack_bf16(d[0], d[1]), pack_bf16(d[2], 0.0f), 0u, 0u);
+      st_shared_v4(sbase + uDY + cm_off(row, 8, kOutPad), 0u, 0u, 0u, 0u);
     }
-    // Layer 4: dW4 += H3^T dY, dH3 = dY W4^T.
-    if (!mma_round([&] {
-          mma_chain<kRows, kOutPad>(tmem + cW4, sbase + uH3t, sbase + uDYt, first);
-          mma_chain<kOutPad, kHid>(tmem + cZ, sbase + uDY, sbase + uB4, true);
-        }))
-      break;
-    gb4 += column_sum(uDY, kOutPad, kOut);
-    backward_epilogue(uH3);
-    __syncthreads();
-    gb3 += column_sum(uDZ, kHid, kHid);
-    // Layer 3: dW3 += H2^T dZ3, dH2 = dZ3 W3^T.
-    if (!mma_round([&] {
-          mma_chain<kRows, kHid>(tmem + cW3, sbase + uH2t, sbase + uDZt, first);
-          mma_chain<kHid, kHid>(tmem + cZ, sbase + uDZ, sbase + uB3, true);
-        }))
-      break;
-    backward_epilogue(uH2);
-    __syncthreads();
-    gb2 += column_sum(uDZ, kHid, kHid);
-    // Layer 2: dW2 += H1^T dZ2, dH1 = dZ2 W2^T.
-    if (!mma_round([&] {
-          mma_chain<kRows, kHid>(tmem + cW2, sbase + uH1t, sbase + uDZt, first);
-          mma_chain<kHid, kHid>(tmem + cZ, sbase + uDZ, sbase + uB2, true);
-        }))
-      break;
-    backward_epilogue(uH1);
-    __syncthreads();
-    gb1 += column_sum(uDZ, kHid, kHid);
-    // Layer 1: dW1 += X^T dZ1.
-    if (!mma_round([&] { mma_chain<kRows, kHid>(tmem + cW1, sbase + uXt, sbase + uDZt, first); })) break;
+    // Layer 4: dH3 = dY W4^T; dW4 += H3^T dY.
+    mma_round(
+        [&] { mma_chain<kOutPad, kHid>(tmem + cZ, along_columns<kOutPad>(sbase + uDY), along_columns<kOutPad>(sbase + uW4), true); },
+        [&] {
+          mma_chain<kRows, kOutPad>(tmem + cW4, along_rows<kHid>(sbase + uH3), along_rows<kOutPad>(sbase + uDY), first);
+          mma_chain<kRows, kOutPad>(tmem + cB4, ones, along_rows<kOutPad>(sbase + uDY), first);
+        });
+    backward_epilogue(uH3, uZ3);
+    // Layer 3: dH2 = dZ3 W3^T; dW3 += H2^T dZ3.
+    mma_round(
+        [&] { mma_chain<kHid, kHid>(tmem + cZ, along_columns<kHid>(sbase + uZ3), along_columns<kHid>(sbase + uW3), true); },
+        [&] {
+          mma_chain<kRows, kHid>(tmem + cW3, along_rows<kHid>(sbase + uH2), along_rows<kHid>(sbase + uZ3), first);
+          mma_chain<kRows, kHid>(tmem + cB3, ones, along_rows<kHid>(sbase + uZ3), first);
+        });
+    backward_epilogue(uH2, uZ2);
+    // Layer 2: dH1 = dZ2 W2^T; dW2 += H1^T dZ2.
+    mma_round(
+        [&] { mma_chain<kHid, kHid>(tmem + cZ, along_columns<kHid>(sbase + uZ2), along_columns<kHid>(sbase + uW2), true); },
+        [&] {
+          mma_chain<kRows, kHid>(tmem + cW2, along_rows<kHid>(sbase + uH1), along_rows<kHid>(sbase + uZ2), first);
+          mma_chain<kRows, kHid>(tmem + cB2, ones, along_rows<kHid>(sbase + uZ2), first);
+        });
+    backward_epilogue(uH1, uZ1);
+    // Layer 1: dW1 += X^T dZ1.  The tile's last products: the next tile waits for them.
+    fence_async_smem();
+    fence_before();
+    const bool stop = __syncthreads_or(*fail) != 0;
+    fence_after();
+    if (tid == 0) {
+      mma_chain<kRows, kHid>(tmem + cW1, along_rows<kIn>(sbase + uX), along_rows<kHid>(sbase + uZ1), first);
+      mma_chain<kRows, kHid>(tmem + cB1, ones, along_rows<kHid>(sbase + uZ1), first);
+      mma_commit(grad_bar);
+    }
     first = false;
+    if (stop) break;
   }
-  failed = *fail != 0;
-  if (failed && tid == 0) {
-    atomicAdd(&g_tc_errors, 1);
-    (void)mbar_wait(bar, phase ^ 1u);  // the MMAs in flight, bounded
-  }
+  if (!first && !mbar_wait(grad_bar, grad_phase)) *fail = 1;  // every product in flight, bounded
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const bool failed = *fail != 0;
+  if (failed && tid == 0) atomicAdd(&g_tc_errors, 1);
   if (!failed && !first) {
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((tid & 31) == 0) atomicAdd(loss, lsum);
-    if (tid < kHid) {
-      atomicAdd(grads + ob1 + tid, gb1);
-      atomicAdd(grads + ob2 + tid, gb2);
-      atomicAdd(grads + ob3 + tid, gb3);
-    }
-    if (tid < kOut) atomicAdd(grads + ob4 + tid, gb4);
-    // Weight-gradient rows: lane r of the accumulators = input feature r.
-    if (warp < 2) {
-      auto add_rows = [&](uint32_t col, int rows, int N, float* g) {
-#pragma unroll
-        for (int c = 0; c < kHid; c += 32) {
-          if (c >= N) break;
-          float v[32];
-          tmem_ld32(lane + col + c, v);
-          if (tid < rows)
-            for (int j = 0; j < 32 && c + j < N; j++) atomicAdd(g + tid * N + c + j, v[j]);
-        }
-      };
-      add_rows(cW1, kIn, kHid, grads + oW1);
-      add_rows(cW2, kHid, kHid, grads + oW2);
-      add_rows(cW3, kHid, kHid, grads + oW3);
-      {
-        float v[16];
-        tmem_ld16(lane + cW4, v);
-        if (tid < kHid)
-          for (int j = 0; j < kOut; j++) atomicAdd(grads + oW4 + tid * kOut + j, v[j]);
+    if (half == 0 && (tid & 31) == 0) atomicAdd(loss, lsum);
+    float v[32];
+    if ((warp & 3) < 2) {  // weight-gradient rows: lane r of the accumulators = input feature r
+      if ((warp & 1) == 0) {
+        tmem_ld32(mine + cW1, v);
+        red_add32(grads + oW1 + row * kHid + 32 * half, v);
       }
+      tmem_ld32(mine + cW2, v);
+      red_add32(grads + oW2 + row * kHid + 32 * half, v);
+      tmem_ld32(mine + cW3, v);
+      red_add32(grads + oW3 + row * kHid + 32 * half, v);
+    } else if ((warp & 3) == 2) {  // bias gradients: any row
+      tmem_ld32(mine + cB1, v);
+      if ((tid & 31) == 0) red_add32(grads + ob1 + 32 * half, v);
+      tmem_ld32(mine + cB2, v);
+      if ((tid & 31) == 0) red_add32(grads + ob2 + 32 * half, v);
+      tmem_ld32(mine + cB3, v);
+      if ((tid & 31) == 0) red_add32(grads + ob3 + 32 * half, v);
+    }
+    float u[16];
+    if (half == 0 && (warp & 3) < 2) {
+      tmem_ld16(lane + cW4, u);
+      for (int j = 0; j < kOut; j++) atomicAdd(grads + oW4 + row * kOut + j, u[j]);
+    } else if (half == 0 && (warp & 3) == 2) {
+      tmem_ld16(lane + cB4, u);
+      if ((tid & 31) == 0)
+        for (int j = 0; j < kOut; j++) atomicAdd(grads + ob4 + j, u[j]);
     }
   }
   fence_before();
