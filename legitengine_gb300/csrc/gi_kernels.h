@@ -63,7 +63,7 @@ struct MarchArgs {
   // steps that raised the horizon, their horizon contributions and the initial
   // term -- all independent of the light pyramid -- so that a later bounce over
   // the same depth, normals and view re-lights them instead of marching again.
-  float* rec_hc;                      // [direction][hit ordinal][record pixel]: hc of the k-th raising step
+  float* rec_hc;                      // [direction][step][record pixel]: hc of the steps that raised the horizon
   unsigned long long* rec_mask;       // [direction][record pixel]: bit s set = step s raised the horizon
   float* rec_hc0;                     // [direction][record pixel]
   // (record pixel: the interleaved (pattern, sub-image row, column) index, so that a
