@@ -300,6 +300,23 @@ __device__ __forceinline__ void add_term(Light& sum, const Light& dl, float rR) 
   sum.b = sum.b + 2.0f * dl.b * rR;
 }
 
+// The direction split: a direction's term by the thread that marched it, and their sum
+// in direction order (`contrib`: split_smem_bytes).
+__device__ __forceinline__ void split_term(float* contrib, int d, const Light& dl, float rR) {
+  float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
+  c[0] = 2.0f * lo_(dl.rg) * rR;
+  c[1] = 2.0f * hi_(dl.rg) * rR;
+  c[2] = 2.0f * dl.b * rR;
+}
+__device__ __forceinline__ void split_sum(const float* contrib, int dirs, Light& sum) {
+  for (int d = 0; d < dirs; d++) {
+    const float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
+    sum.rg = padd(sum.rg, pk(c[0], c[1]));
+    sum.b = sum.b + c[2];
+  }
+}
+__host__ __device__ constexpr int split_smem_bytes(int dirs) { return dirs * kMarchTx * 3 * (int)sizeof(float); }
+
 // Per-pattern tables of a CTA-tile: the same values as evaluating :170-177,
 // :212, :217, :234-235 per pixel.  Every thread of the CTA calls it; the caller
 // synchronises before use.
@@ -389,7 +406,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
                                            MarchSmem<TEX>& sm, int row = 0, float* contrib = nullptr) {
   static_assert(!SOFT || (DCH == 2 && !FAST), "the soft horizon needs both depth moments, exact contract");
   static_assert(SPLIT == 1 || (!DEINT && !SOFT), "the direction split serves the standard form");
-  static_assert(!REC || (SPLIT == 1 && !DEINT && !SOFT), "recording serves the standard form");
+  static_assert(!REC || (!DEINT && !SOFT), "recording serves the standard form");
   static_assert(!TEX || (FAST && DCH == 2 && !DEINT), "texture depth taps serve the fast standard form");
   constexpr int kThreads = kMarchTx * (SPLIT > 1 ? SPLIT : KY);
   auto* s_step = sm.step;
@@ -568,7 +585,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
       return hc;
     };
     auto record = [&](int s, float hc) {
-      __stcs(rec_rows + (size_t)((unsigned)s * npix), hc);
+      if (SPLIT == 1 || inside) __stcs(rec_rows + (size_t)((unsigned)s * npix), hc);
       hits |= 1ull << s;
     };
     if constexpr (TEX) {
@@ -648,15 +665,12 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
         if (REC) record(s, hc);
       }
     }
-    if (REC) {
+    if (REC && (SPLIT == 1 || inside)) {
       __stcs(a.rec_mask + (size_t)d * npix + rec_idx, hits);
       __stcs(a.rec_hc0 + (size_t)d * npix + rec_idx, hc0);
     }
     if (SPLIT > 1) {
-      float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
-      c[0] = 2.0f * lo_(dl.rg) * rR;
-      c[1] = 2.0f * hi_(dl.rg) * rR;
-      c[2] = 2.0f * dl.b * rR;
+      split_term(contrib, d, dl, rR);
     } else {
       add_term(sum, dl, rR);
     }
@@ -664,11 +678,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
   if (SPLIT > 1) {
     __syncthreads();
     if (threadIdx.y != 0 || !inside) return;
-    for (int d = 0; d < R; d++) {
-      const float* c = contrib + 3 * (d * kMarchTx + threadIdx.x);
-      sum.rg = padd(sum.rg, pk(c[0], c[1]));
-      sum.b = sum.b + c[2];
-    }
+    split_sum(contrib, R, sum);
   }
   reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(lo_(sum.rg), hi_(sum.rg), sum.b, 1.0f);
 }
@@ -677,22 +687,24 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
 // step table, step footprints and light taps as march_tile, only at the steps
 // the record marks, with the recorded horizon contributions -- the result is
 // the march's over the new light pyramid, bit for bit.
-template <int KY, bool FAST>
+// SPLIT, row, contrib: the direction split, as march_tile's.
+template <int KY, bool FAST, int SPLIT = 1>
 __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab, int pat, int tile, int tiles_x,
-                                                  ReplaySmem& sm) {
-  constexpr int kThreads = kMarchTx * KY;
+                                                  ReplaySmem& sm, int row = 0, float* contrib = nullptr) {
+  constexpr int kThreads = kMarchTx * (SPLIT > 1 ? SPLIT : KY);
   const int P = a.pattern;
   const int kx = pat % P, ky = pat / P;
   const int R = a.dirs;
-  march_tables(a, a.light, n_tab, pat, sm, threadIdx.y * kMarchTx + threadIdx.x, kThreads);
+  const int tid = threadIdx.y * kMarchTx + threadIdx.x;
+  march_tables(a, a.light, n_tab, pat, sm, tid, kThreads);
   __syncthreads();
-  const int2 place = tile_place<KY, false>(threadIdx.y * kMarchTx + threadIdx.x);
+  const int2 place = SPLIT > 1 ? tile_place<KY, false>(32 * row + threadIdx.x) : tile_place<KY, false>(tid);
   const int i = (tile % tiles_x) * kMarchTx + place.x;
   const int j = (tile / tiles_x) * KY + place.y;
   const int px = kx + P * i, py = ky + P * j;
   const bool inside = px < a.width && py < a.height;
   const unsigned lanes = __ballot_sync(0xffffffffu, inside);
-  if (!inside) return;
+  if (SPLIT == 1 && !inside) return;
   const p2 rWH = pk(a.inv_size[0], a.inv_size[1]);
   const p2 centre = pk((float)px + 0.5f, (float)py + 0.5f);
   const size_t out_idx = (size_t)py * a.width + px;
@@ -701,7 +713,8 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
   const float ambient = 0.01f;
   const float rR = rcp_((float)R);
   Light sum{pk(0.0f), 0.0f};
-  for (int d = 0; d < R; d++) {
+  // A split CTA's lanes past the edge have no record, and only join the barrier.
+  for (int d = SPLIT > 1 ? (int)threadIdx.y : 0; d < R && inside; d += SPLIT) {
     const float4 dir4 = sm.dir[d];
     const p2 dir = pk(dir4.x, dir4.y);
     const float hc0 = __ldcs(a.rec_hc0 + (size_t)d * npix + rec_idx);
@@ -728,7 +741,13 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
       else tap_foot1(e, lo_(sp), hi_(sp), foot);
       add_light<FAST>(e.img0, e.img1, e.delta, foot, two, hc, ambient, dl);
     }
-    add_term(sum, dl, rR);
+    if (SPLIT > 1) split_term(contrib, d, dl, rR);
+    else add_term(sum, dl, rR);
+  }
+  if (SPLIT > 1) {
+    __syncthreads();
+    if (threadIdx.y != 0 || !inside) return;
+    split_sum(contrib, R, sum);
   }
   reinterpret_cast<float4*>(a.out)[out_idx] = make_float4(lo_(sum.rg), hi_(sum.rg), sum.b, 1.0f);
 }
@@ -764,23 +783,34 @@ __global__ void __launch_bounds__(kMarchTx* KY, march_min_blocks<KY>())
 
 // Direction-split march (march_tile with SPLIT = kSplit) of a tile list -- a
 // short list (the judge's 1/64 of the tiles) spread over kMarchTy times more
-// CTAs -- or of the whole frame (a.tiles null; the autotuner's four-threads-per-
-// pixel layout): each CTA one row of a tile, each thread a quarter of a pixel's
-// directions.
-
-template <bool FAST, bool TEX>
+// CTAs -- or of the whole frame (a.tiles null: frames too small to fill the GPU with
+// a thread per pixel, and the autotuner's four-threads-per-pixel layout): each CTA one
+// warp's pixels of a tile, each thread a quarter of a pixel's directions.
+template <bool FAST, bool REC, bool TEX>
 __global__ void __launch_bounds__(kMarchTx* kSplit, 1024 / (kMarchTx * kSplit))
     march_split_kernel(const __grid_constant__ MarchArgs a, int n_tab, int tiles_x, int tiles_total) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];  // march_smem_bytes<TEX>(n_tab, a.dirs)
+  // march_smem_bytes<TEX>(n_tab, a.dirs), then the directions' terms
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
   MarchSmem<TEX> sm = march_smem<TEX>(dyn_smem, n_tab);
-  __shared__ float contrib[kSplitMaxDirs * kMarchTx * 3];
+  float* contrib = reinterpret_cast<float*>(dyn_smem + march_smem_bytes<TEX>(n_tab, a.dirs));
   const int P2 = a.pattern * a.pattern;
   const int pat = blockIdx.x % P2;
   const int rest = blockIdx.x / P2;
   const int row = rest % kMarchTy;
   const int tile = a.tiles ? __ldg(a.tiles + rest / kMarchTy) : rest / kMarchTy;
   if (tile < 0 || tile >= tiles_total) return;  // a listed tile outside the grid: nothing to march
-  march_tile<2, false, kMarchTy, FAST, false, kSplit, false, TEX>(a, n_tab, pat, tile, tiles_x, sm, row, contrib);
+  march_tile<2, false, kMarchTy, FAST, false, kSplit, REC, TEX>(a, n_tab, pat, tile, tiles_x, sm, row, contrib);
+}
+
+template <bool FAST>
+__global__ void __launch_bounds__(kMarchTx* kSplit, 1024 / (kMarchTx * kSplit))
+    march_replay_split_kernel(const __grid_constant__ MarchArgs a, int n_tab, int tiles_x) {
+  __shared__ ReplaySmem sm;  // n_tab <= kRecMaxSteps (checked at launch)
+  extern __shared__ __align__(16) unsigned char dyn_smem[];  // the directions' terms
+  const int P2 = a.pattern * a.pattern;
+  const int rest = blockIdx.x / P2;
+  march_replay_tile<kMarchTy, FAST, kSplit>(a, n_tab, (int)(blockIdx.x % P2), rest / kMarchTy, tiles_x, sm,
+                                            rest % kMarchTy, reinterpret_cast<float*>(dyn_smem));
 }
 
 // Persistent batched march: CTAs claim work items (view, tile, pattern) from a
@@ -1035,13 +1065,47 @@ void set_ray_basis(MarchArgs& a) {
 // Rays a warp marches: 32 pixels x the directions of each thread.
 static int rays_per_warp(int dirs, int split) { return kMarchTx * ((dirs + split - 1) / split); }
 
-// Untuned shapes: 4 rows (two-bounce texture frame at 1920x1080, R = 16: 3753 us
-// against 3781 with 8 and 3905 with 2; exact march at 1283x721: 1666 us against 1698
-// and 1713).
+// Whether a march can take the direction-split form: the standard form with
+// 2-channel moments, kSplitMinDirs to kSplitMaxDirs directions.
+static bool split_fits(const MarchArgs& a) {
+  return !a.deinterleaved && a.depth_ch == 2 && !a.soft && a.dirs >= kSplitMinDirs && a.dirs <= kSplitMaxDirs;
+}
+
+// Whether an untuned frame takes the direction split: four times the threads, each
+// with the pixel's set-up and ceil(R / 4) = n of its directions.  It pays while the
+// one-thread form is too few waves of CTAs (8 an SM) to fill the GPU and hide its
+// latency, and up to more waves the more directions share the set-up and the more
+// evenly they divide.  The line, (1.5 n - 1) waves times the share of the last round of
+// directions that is used, follows a sweep of 200 x 120 to 1920 x 1080 with 4, 5, 8
+// and 16 directions; one-thread form against split, exact march and two-bounce exact
+// frame, in us: R = 8 at 256 x 144 (0.24 waves) 126 / 65 and 203 / 119, at 512 x 512
+// (1.7) 319 / 298 and 511 / 475, at 700 x 500 (2.4) 413 / 413 and 643 / 638, at
+// 1920 x 1080 (13) 1878 / 2046 and 2837 / 3136; R = 16 at 960 x 540 (3.3) 1632 / 1587,
+// at 1280 x 720 (5.9) 2683 / 2648; R = 4 at 320 x 240 (0.6) 66 / 60, at 400 x 300 (1)
+// 79 / 85; R = 5 at 256 x 144 72 / 48, at 320 x 240 84 / 87.
+static bool split_pays(const MarchArgs& a) {
+  if (!split_fits(a)) return false;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  const int n = (a.dirs + kSplit - 1) / kSplit;
+  const float waves = (float)a.width * (float)a.height / (1024.0f * (float)sms);  // 1024 resident threads an SM
+  return waves < (1.5f * (float)n - 1.0f) * (float)(a.dirs - kSplit * (n - 1)) / (float)kSplit;
+}
+
+// Untuned shapes that do not split: 4 rows (two-bounce texture frame at 1920x1080,
+// R = 16: 3753 us against 3781 with 8 and 3905 with 2; exact march at 1283x721: 1666 us
+// against 1698 and 1713).
 static TunedLayout tuned_layout(const MarchArgs& a) {
-  std::lock_guard<std::mutex> lock(g_tune_mutex);
-  auto it = g_tuned.find(key_of(a));
-  return it == g_tuned.end() ? TunedLayout{kMarchTy, 1} : it->second;
+  {
+    std::lock_guard<std::mutex> lock(g_tune_mutex);
+    auto it = g_tuned.find(key_of(a));
+    if (it != g_tuned.end()) return it->second;
+  }
+  return TunedLayout{kMarchTy, !a.tiles && split_pays(a) ? kSplit : 1};
 }
 
 int march_table_size(const MarchArgs& a) {
@@ -1131,12 +1195,7 @@ static void launch_replay(const MarchArgs& a, int rows, dim3 grid, int n_tab, in
   else launch_tables(march_replay_kernel<4, FAST>, grid, dim3(kMarchTx, 4), smem, s, a, n_tab, tiles_x);
 }
 
-// Whether a march can take the direction-split form: the standard form with
-// 2-channel moments, no record, kSplitMinDirs to kSplitMaxDirs directions.
-static bool split_fits(const MarchArgs& a) {
-  return !a.rec && !a.deinterleaved && a.depth_ch == 2 && !a.soft && a.dirs >= kSplitMinDirs &&
-         a.dirs <= kSplitMaxDirs;
-}
+static const char* const kReplayTooLong = "march: replay of more steps than a record holds";
 
 // Launches the march in the layout (rows, split): one thread per pixel in CTAs
 // of `rows` = 2, 4 or 8 rows of 32 pixels, or split = kSplit, four threads per
@@ -1163,17 +1222,31 @@ static int launch_march_rows(const MarchArgs& args, int rows, int split, cudaStr
     // The direction-split form (same result).
     grid.x *= kMarchTy;
     const dim3 block(kMarchTx, kSplit);
-    const int smem = tex ? march_smem_bytes<true>(n_tab, a.dirs) : march_smem_bytes<false>(n_tab, a.dirs);
-    if (tex) launch_tables(march_split_kernel<true, true>, grid, block, smem, stream, a, n_tab, tiles_x, total);
-    else if (a.fast) launch_tables(march_split_kernel<true, false>, grid, block, smem, stream, a, n_tab, tiles_x, total);
-    else launch_tables(march_split_kernel<false, false>, grid, block, smem, stream, a, n_tab, tiles_x, total);
+    const int terms = split_smem_bytes(a.dirs);
+    const int smem = terms + (tex ? march_smem_bytes<true>(n_tab, a.dirs) : march_smem_bytes<false>(n_tab, a.dirs));
+    auto go = [&](auto kernel) { launch_tables(kernel, grid, block, smem, stream, a, n_tab, tiles_x, total); };
+    if (a.rec == 2) {
+      if (n_tab > kRecMaxSteps) return fail(GI_ERR_INVALID_ARGUMENT, kReplayTooLong);
+      if (a.fast) launch_tables(march_replay_split_kernel<true>, grid, block, terms, stream, a, n_tab, tiles_x);
+      else launch_tables(march_replay_split_kernel<false>, grid, block, terms, stream, a, n_tab, tiles_x);
+    } else if (a.rec) {
+      if (tex) go(march_split_kernel<true, true, true>);
+      else if (a.fast) go(march_split_kernel<true, true, false>);
+      else go(march_split_kernel<false, true, false>);
+    } else if (tex) {
+      go(march_split_kernel<true, false, true>);
+    } else if (a.fast) {
+      go(march_split_kernel<true, false, false>);
+    } else {
+      go(march_split_kernel<false, false, false>);
+    }
     GI_CHECK_LAUNCH("march_split_kernel");
     count_launches(1);
     return GI_OK;
   }
   if (a.rec) {  // record or replay: standard form, 2-channel moments, no tile list (checked by the caller)
     if (a.rec == 2) {
-      if (n_tab > kRecMaxSteps) return fail(GI_ERR_INVALID_ARGUMENT, "march: replay of more steps than a record holds");
+      if (n_tab > kRecMaxSteps) return fail(GI_ERR_INVALID_ARGUMENT, kReplayTooLong);
       // The replay re-lights with the fast loop's software light taps in the
       // texture precision too: its work is the light taps alone, and these loads
       // beat the four-channel trilinear fetch (measured, whole frame).
