@@ -230,13 +230,12 @@ __device__ __forceinline__ void relu_backward(const float* dH, const bf16* H, bf
   }
 }
 
-__global__ void adam_kernel(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m,
+__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, bf16* __restrict__ wb, float inv_batch, float lr, float b1,
                             float b2, float eps, float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kParams) return;
   float gi_ = g[i] * inv_batch;
-  g[i] = 0.0f;
   if (!isfinite(gi_)) gi_ = 0.0f;  // a non-finite gradient element counts as zero
   const float mi = b1 * m[i] + (1.0f - b1) * gi_;
   const float vi = b2 * v[i] + (1.0f - b2) * gi_ * gi_;
@@ -593,10 +592,9 @@ int launch_judge(float* learned, const float* plain, int W, int H, int P, const 
 
 struct Mlp {
   float* params = nullptr;
-  float* grads = nullptr;
+  float* grads = nullptr;  // gradient sums of a batch, then its loss sum: cleared and read back as one
   float* m = nullptr;
   float* v = nullptr;
-  float* loss = nullptr;
   bf16* wb = nullptr;
   int step = 0;
   int loss_kind = GI_MLP_LOSS_SQUARED;  // training loss (gi_mlp_set_loss)
@@ -605,9 +603,10 @@ struct Mlp {
     dfree(grads);
     dfree(m);
     dfree(v);
-    dfree(loss);
     dfree(wb);
   }
+  float* loss() const { return grads + kParams; }
+  static constexpr size_t kSumBytes = (kParams + 1) * sizeof(float);
 };
 
 // gi_mlp_forward: the fused reconstruction kernel on given feature rows (tcgen05).
@@ -632,16 +631,14 @@ extern "C" int gi_mlp_create(gi_mlp** out) {
   Mlp& M = m->impl;
   int e = GI_OK;
   e = e ? e : check_cuda(dmalloc(&M.params, kParams * 4), "gi_mlp_create");
-  e = e ? e : check_cuda(dmalloc(&M.grads, kParams * 4), "gi_mlp_create");
+  e = e ? e : check_cuda(dmalloc(&M.grads, Mlp::kSumBytes), "gi_mlp_create");
   e = e ? e : check_cuda(dmalloc(&M.m, kParams * 4), "gi_mlp_create");
   e = e ? e : check_cuda(dmalloc(&M.v, kParams * 4), "gi_mlp_create");
-  e = e ? e : check_cuda(dmalloc(&M.loss, 4), "gi_mlp_create");
   e = e ? e : check_cuda(dmalloc(&M.wb, kWbf * 2), "gi_mlp_create");
   if (e) return e;
-  e = check_cuda(cudaMemset(M.grads, 0, kParams * 4), "gi_mlp_create");
+  e = check_cuda(cudaMemset(M.grads, 0, Mlp::kSumBytes), "gi_mlp_create");
   e = e ? e : check_cuda(cudaMemset(M.m, 0, kParams * 4), "gi_mlp_create");
   e = e ? e : check_cuda(cudaMemset(M.v, 0, kParams * 4), "gi_mlp_create");
-  e = e ? e : check_cuda(cudaMemset(M.loss, 0, 4), "gi_mlp_create");
   e = e ? e : check_cuda(cudaMemset(M.params, 0, kParams * 4), "gi_mlp_create");
   e = e ? e : check_cuda(cudaMemset(M.wb, 0, kWbf * 2), "gi_mlp_create");
   if (e) return e;
@@ -684,7 +681,6 @@ extern "C" int gi_mlp_init(gi_mlp* m, uint64_t seed) {
   m->impl.step = 0;
   int e = check_cuda(cudaMemset(m->impl.m, 0, kParams * 4), "gi_mlp_init");
   e = e ? e : check_cuda(cudaMemset(m->impl.v, 0, kParams * 4), "gi_mlp_init");
-  e = e ? e : check_cuda(cudaMemset(m->impl.grads, 0, kParams * 4), "gi_mlp_init");
   if (e) return e;
   return gi_mlp_set_params(m, p.data(), kParams);
 }
@@ -702,8 +698,8 @@ extern "C" int gi_mlp_train_step(gi_mlp* m, const void* features, const float* t
   GI_CHECK_ARG(aligned16(features) && aligned16(targets), "gi_mlp_train_step: unaligned buffer");
   cudaStream_t s = (cudaStream_t)stream;
   Mlp& M = m->impl;
-  int e = check_cuda(cudaMemsetAsync(M.loss, 0, 4, s), "gi_mlp_train_step");
-  e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss,
+  int e = check_cuda(cudaMemsetAsync(M.grads, 0, Mlp::kSumBytes, s), "gi_mlp_train_step");
+  e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss(),
                               M.loss_kind, s);
   if (e) return e;
   M.step++;
@@ -715,7 +711,7 @@ extern "C" int gi_mlp_train_step(gi_mlp* m, const void* features, const float* t
   count_launches(1);
   if (loss_out) {
     float l = 0.0f;
-    e = check_cuda(cudaMemcpyAsync(&l, M.loss, 4, cudaMemcpyDeviceToHost, s), "gi_mlp_train_step: loss");
+    e = check_cuda(cudaMemcpyAsync(&l, M.loss(), 4, cudaMemcpyDeviceToHost, s), "gi_mlp_train_step: loss");
     if (e) return e;
     e = check_cuda(cudaStreamSynchronize(s), "gi_mlp_train_step: sync");
     if (e) return e;
@@ -737,20 +733,16 @@ extern "C" int gi_mlp_gradients(gi_mlp* m, const void* features, const float* ta
   GI_CHECK_ARG(aligned16(features) && aligned16(targets), "gi_mlp_gradients: unaligned buffer");
   cudaStream_t s = (cudaStream_t)stream;
   Mlp& M = m->impl;
-  int e = check_cuda(cudaMemsetAsync(M.loss, 0, 4, s), "gi_mlp_gradients");
-  e = e ? e : check_cuda(cudaMemsetAsync(M.grads, 0, kParams * 4, s), "gi_mlp_gradients");
-  e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss,
+  int e = check_cuda(cudaMemsetAsync(M.grads, 0, Mlp::kSumBytes, s), "gi_mlp_gradients");
+  e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss(),
                               M.loss_kind, s);
   if (e) return e;
-  std::vector<float> g(kParams);
-  float l = 0.0f;
-  e = check_cuda(cudaMemcpyAsync(g.data(), M.grads, kParams * 4, cudaMemcpyDeviceToHost, s), "gi_mlp_gradients");
-  e = e ? e : check_cuda(cudaMemcpyAsync(&l, M.loss, 4, cudaMemcpyDeviceToHost, s), "gi_mlp_gradients");
-  e = e ? e : check_cuda(cudaMemsetAsync(M.grads, 0, kParams * 4, s), "gi_mlp_gradients");
+  std::vector<float> g(kParams + 1);
+  e = check_cuda(cudaMemcpyAsync(g.data(), M.grads, Mlp::kSumBytes, cudaMemcpyDeviceToHost, s), "gi_mlp_gradients");
   e = e ? e : check_cuda(cudaStreamSynchronize(s), "gi_mlp_gradients");
   if (e) return e;
   for (int i = 0; i < kParams; i++) grads_host[i] = g[i] / (float)n;
-  if (loss_host) *loss_host = l / (float)(n * kOut);
+  if (loss_host) *loss_host = g[kParams] / (float)(n * kOut);
   return GI_OK;
 }
 
