@@ -21,11 +21,12 @@
 // the NEXT tile while the current tile runs its MMA rounds; the neighbourhood
 // and mip taps are read from global memory.  (Inputs not 16-byte aligned, and a
 // last partial tile, read everything from global memory.)
-// One thread of a group issues the MMAs of a layer, commits them to the group's
-// mbarrier and waits on it, and waits for the staging copies (bounded: a wait
-// that runs out records an error and the group stops; the CTA then waits for its
-// copies in flight, frees its tensor memory and returns) while the group's other
-// threads block on a hardware barrier.
+// One thread of a group issues the MMAs of a layer and commits them to the group's
+// mbarrier, and every thread waits on it, and for the staging copies (bounded: after a
+// wait that runs out the group stops at its next barrier and records an error; the CTA
+// then waits for its copies in flight, frees its tensor memory and returns).  So a layer
+// takes one hardware barrier of the group, before its MMAs (1920 x 1080: 127.5 -> 124.5
+// us against one waiting thread and a second barrier).
 //
 // Operand layout: K-major without swizzle.  A core matrix is 8 rows x 16 bytes
 // stored as 128 contiguous bytes; core matrices adjacent along K are 128 bytes
@@ -73,8 +74,7 @@ constexpr int sNormal = 0, sAlbedo = 2048, sLight = 4096, sDirect = 6144, sMomen
 constexpr int kStageBytes = 9216;
 constexpr int tStage = tA + kGroups * kABytes;
 constexpr int tBar = tStage + kGroups * kStageBytes;  // per group: MMA mbarrier, staging mbarrier
-constexpr int tFail = tBar + 16 * kGroups;            // one int per group
-constexpr int tTmem = tFail + 4 * kGroups;
+constexpr int tTmem = tBar + 16 * kGroups;
 constexpr int kSmemTc = tTmem + 8;
 static_assert(tStage % 128 == 0 && kStageBytes % 128 == 0, "bulk copy destinations");
 static_assert(tBB % 128 == 0 && tOnes % 128 == 0 && tA % 128 == 0 && kABytes % 128 == 0 && tBar % 8 == 0,
@@ -132,20 +132,27 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 }
 
 // Waits for the phase with the given parity to complete, for at most `limit` SM
-// cycles (by default ~2^31, about a second); false if it did not.
+// cycles (by default ~2^31, about a second); false if it did not.  The first look does
+// not suspend the thread, so that a limit of a few cycles runs out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit = kWaitCycles) {
   const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  while (!done) {
+    if (clock64() - t0 > limit) return false;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (done) return true;
-    if (clock64() - t0 > limit) return false;
   }
+  return true;
 }
 
 // One arrival that also expects `bytes` of asynchronous copies on the barrier.
@@ -219,27 +226,34 @@ __device__ __forceinline__ void stage_b(unsigned char* smem, int off, const bf16
   }
 }
 
-// Barrier of one group's 128 threads (named barrier 1 + group).
-__device__ __forceinline__ void group_sync(int group) {
-  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(kRows) : "memory");
+// Barrier of one group's 128 threads (named barrier 1 + group); whether any of them
+// passed true.
+__device__ __forceinline__ bool group_any(int group, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(1 + group), "r"(kRows), "r"((uint32_t)v)
+      : "memory");
+  return r != 0;
 }
 
 // Makes this group's A operand visible to the tensor cores, issues the layer's
-// bias MMA and its K/16 MMAs from the group's first thread, which alone waits for their
-// completion (the other 127 threads block on the group's hardware barrier instead
-// of spinning); the fence pair around that barrier orders the completion before
-// every thread's accumulator reads.  Returns false (on every thread of the group)
-// if the wait ran out.
+// bias MMA and its K/16 MMAs from the group's first thread and waits for them; the
+// fence after the wait orders their completion before the accumulator reads.  `bad`
+// is set on a thread whose wait runs out; returns false (on every thread of the
+// group) if an earlier one did.
 // The B operand's row-group stride is K * 16 bytes, or 0 when its N = 16 rows
 // re-read the first 8 (the output layer).
 // `first` runs on the issuing thread after the barrier, before the MMAs.
 template <int K, int N, int L, typename First>
 __device__ __forceinline__ bool run_layer(uint32_t sbase, int a_off, int b_off, uint32_t tmem, uint32_t bar,
-                                          uint32_t& phase, int group, volatile int* fail, First first,
+                                          uint32_t& phase, int group, bool& bad, First first,
                                           long long limit = kWaitCycles) {
   fence_async_smem();
   fence_before();
-  group_sync(group);
+  if (group_any(group, bad)) return false;
   fence_after();
   if ((threadIdx.x & (kRows - 1)) == 0) {
     first();
@@ -253,14 +267,12 @@ __device__ __forceinline__ bool run_layer(uint32_t sbase, int a_off, int b_off, 
       mma_bf16(tmem, ad, bd, idesc, 1u);
     }
     mma_commit(bar);
-    if (!mbar_wait(bar, phase, limit)) *fail = 1;
-    fence_before();
   }
+  if (!mbar_wait(bar, phase, limit)) bad = true;
   phase ^= 1u;
-  group_sync(group);
-  const bool failed = *fail != 0;
+  __syncwarp();  // the warp's accumulator loads are one instruction for all its lanes
   fence_after();
-  return !failed;
+  return true;
 }
 
 // Hidden-layer epilogue: accumulator lane (bias included) -> ReLU -> bf16 row
@@ -310,7 +322,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   const uint32_t stage = sbase + tStage + group * kStageBytes;
   const unsigned char* stage_p = smem + tStage + group * kStageBytes;
   const int a_off = tA + group * kABytes;
-  volatile int* fail = reinterpret_cast<volatile int*>(smem + tFail) + group;
 
   stage_b(smem, tB1, wb + qW1, kIn, kHid, kHid);
   stage_b(smem, tB2, wb + qW2, kHid, kHid, kHid);
@@ -336,7 +347,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   if (gtid == 0) {
     mbar_init(bar, 1);
     mbar_init(sbar, 1);
-    *fail = 0;
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + tTmem),
@@ -357,7 +367,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   const int full_tiles = n / kRows;
   const int stride = gridDim.x * kGroups;
   uint32_t phase = 0, sphase = 0;
-  bool failed = false;
+  bool bad = false, failed = false;  // a wait of this thread, of the group ran out
   int t = blockIdx.x * kGroups + group;
   const int first_tile = t;
   bool pending = staged && t < full_tiles;  // a staging copy of tile t in flight
@@ -385,9 +395,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
         for (int i = 0; i < kIn; i++) f[i] = 0.0f;
       }
     } else if (pending) {
-      if (gtid == 0 && !mbar_wait(sbar, sphase)) *fail = 1;
-      group_sync(group);
-      if (*fail) { failed = true; break; }  // the copy stays pending: waited for again before exit
+      if (!mbar_wait(sbar, sphase)) bad = true;
       sphase ^= 1u;
       pending = false;
       const float depth = reinterpret_cast<const float*>(stage_p + sMoments)[2 * gtid];
@@ -405,7 +413,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     // The staging buffer takes the group's next tile once every thread has its
     // features: issued after the first layer's barrier.
     const bool prefetch = staged && t + stride < full_tiles;
-    pending = prefetch;
 #pragma unroll
     for (int c = 0; c < kIn; c += 8)
       st_shared_v4(sbase + a_off + cm_off(gtid, c, kIn), pack_bf16(f[c], f[c + 1]), pack_bf16(f[c + 2], f[c + 3]),
@@ -425,31 +432,34 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     };
     auto nothing = [] {};
     const long long first_limit = t == first_tile ? g_tc_first_wait_cycles : kWaitCycles;
-    if (!run_layer<kIn, kHid, 0>(sbase, a_off, tB1, tmem, bar, phase, group, fail, issue_next, first_limit)) {
+    if (!run_layer<kIn, kHid, 0>(sbase, a_off, tB1, tmem, bar, phase, group, bad, issue_next, first_limit)) {
       failed = true;
       break;
     }
+    pending = prefetch;
     hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kHid, 1>(sbase, a_off, tB2, tmem, bar, phase, group, fail, nothing)) { failed = true; break; }
+    if (!run_layer<kHid, kHid, 1>(sbase, a_off, tB2, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
     hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kHid, 2>(sbase, a_off, tB3, tmem, bar, phase, group, fail, nothing)) { failed = true; break; }
+    if (!run_layer<kHid, kHid, 2>(sbase, a_off, tB3, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
     hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kOutPad, 3>(sbase, a_off, tB4, tmem, bar, phase, group, fail, nothing)) {
+    if (!run_layer<kHid, kOutPad, 3>(sbase, a_off, tB4, tmem, bar, phase, group, bad, nothing)) {
       failed = true;
       break;
     }
     float v[16];
     tmem_ld16(lane_addr, v);
-    if (p < n) {
+    if (p < n && !bad) {
       const float lo[3] = {v[0], v[1], v[2]};
       float w[3], y[3];
       head_forward(lo, cand, w, y);
       reinterpret_cast<float4*>(out)[p] = make_float4(y[0] * scale, y[1] * scale, y[2] * scale, 1.0f);
     }
   }
+  failed = group_any(group, bad) || failed;
   if (failed && gtid == 0) {
     atomicAdd(&g_tc_errors, 1);
-    (void)mbar_wait(bar, phase ^ 1u);  // the group's MMAs in flight, bounded
+    (void)mbar_wait(bar, phase ^ 1u);    // the group's MMAs in flight, bounded
+    (void)mbar_wait(sbar, sphase ^ 1u);  // and a staging copy whose wait ran out
   }
   if (pending && gtid == 0) (void)mbar_wait(sbar, sphase);  // a staging copy in flight, bounded
   fence_before();
