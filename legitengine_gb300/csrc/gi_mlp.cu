@@ -270,6 +270,9 @@ __global__ void sync_bf16_kernel(const float* __restrict__ p, bf16* __restrict__
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) features_kernel(const __grid_constant__ FeatureArgs a) {
   const int P = a.pattern;
+  __shared__ float pattern[2 * 64];
+  if (threadIdx.x < P * P) pattern_features(threadIdx.x, P, pattern[threadIdx.x], pattern[64 + threadIdx.x]);
+  __syncthreads();
   const int tw = kMarchTileSubX * P, th = kMarchTileSubY * P;
   int x, y;
   size_t out_idx;
@@ -299,7 +302,7 @@ __global__ void __launch_bounds__(256) features_kernel(const __grid_constant__ F
   }
   float f[kIn];
   float scale;
-  pixel_features(a, x, y, f, scale);
+  pixel_features(a, x, y, pattern, f, scale);
   a.scale[out_idx] = scale;
   __align__(16) bf16 q[kIn];
 #pragma unroll

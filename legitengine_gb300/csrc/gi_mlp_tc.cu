@@ -3,17 +3,24 @@
 // persistent kernel, with tcgen05.mma (BF16 operands from shared memory, FP32
 // accumulators in tensor memory) and no intermediate buffer in HBM.
 //
-// One CTA per SM = 8 groups of 4 warps sharing one shared-memory copy of the
+// One CTA per SM = 5 groups of 4 warps sharing one shared-memory copy of the
 // weights and the SM's 512 tensor-memory columns; each group works on its own
-// 128-pixel tile with its own A operand, staging buffer, mbarriers, named barrier
-// and 64 columns, so the groups' feature gathers and MMA rounds overlap.  In a
-// group, thread i owns pixel i of the tile, which is row i of every layer's A
-// operand and lane i of the accumulator, so each warp reads back exactly its own
-// 32 lanes.  Per tile:
+// 128-pixel tile with its own staging buffer, mbarriers, named barrier and 96
+// columns, so the groups' feature gathers and MMA rounds overlap.  In a group,
+// thread i owns pixel i of the tile, which is row i of every layer's A operand and
+// lane i of the accumulator, so each warp reads back and writes exactly its own 32
+// lanes.  Per tile:
 //   features (registers) -> A [128 x 32] -> MMA with W1 (+ the bias MMA) ->
 //   tcgen05.ld, ReLU, bf16 -> A [128 x 64] -> MMA with W2 -> ... -> MMA with W4
 //   (N = 16, columns 3-15 unused) -> softmax blend of the candidate estimates,
 //   x exposure scale -> out.
+// The A operands are in tensor memory (bf16 pairs, written by tcgen05.st beside the
+// accumulator).  With A in shared memory the kernel was bound by that memory's
+// bandwidth: an MMA of N = 64 reads twice as many bytes of A as of B, and every
+// layer's rows were stored there first (tensor-core and load/store accesses each kept it
+// 47 % busy; now 32 and 21 %).  1920 x 1080: 124.5 -> 116.5 us; what is left is the
+// latency of a tile's chain, of which tensor memory holds five at once.  Loading the next
+// tile's taps during the MMA rounds spilled (140 us).
 // A tile is 128 consecutive pixels, so its own depth moments, normals, albedo,
 // few-ray light and direct light are five contiguous byte ranges: one thread of
 // the group copies them into the group's staging buffer with bulk asynchronous
@@ -28,7 +35,7 @@
 // takes one hardware barrier of the group, before its MMAs (1920 x 1080: 127.5 -> 124.5
 // us against one waiting thread and a second barrier).
 //
-// Operand layout: K-major without swizzle.  A core matrix is 8 rows x 16 bytes
+// Layout of the operands in shared memory: K-major without swizzle.  A core matrix is 8 rows x 16 bytes
 // stored as 128 contiguous bytes; core matrices adjacent along K are 128 bytes
 // apart (the descriptor's leading byte offset) and those adjacent along M (or N)
 // are K*2*8 bytes apart (its stride byte offset).  One MMA consumes K = 16, so a
@@ -48,9 +55,12 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 constexpr int kRows = 128;  // pixels per tile = MMA M = accumulator lanes
-constexpr int kGroups = 8;  // tiles in flight per CTA (one CTA per SM)
+constexpr int kGroups = 5;  // tiles in flight per CTA (one CTA per SM)
 constexpr int kTcThreads = 128 * kGroups;
-constexpr uint32_t kTmemCols = 64 * kGroups;  // one 128 x 64 FP32 accumulator per group: all 512 columns
+// Tensor-memory columns: per group a 128 x 64 FP32 accumulator and a 128 x 64 bf16 A
+// operand, then the four layers' constant "ones" operands (128 x 16 bf16 each).
+constexpr uint32_t cA = 64, kGroupCols = cA + kHid / 2, cOnes = kGroupCols * kGroups, kOnesCols = 8, kTmemCols = 512;
+static_assert(cOnes + 4 * kOnesCols <= kTmemCols, "tensor memory");
 
 // Shared memory (bytes).  B operands are the weights as N x K (K-major).
 constexpr int kB4Rows = 8;                        // W4 rows 0-7 (3 outputs, zero padding)
@@ -62,23 +72,19 @@ constexpr int tB4 = tB3 + kHid * kHid * 2;        // 8 x 64; the MMA's rows 8-15
 // "ones" operand, B = the bias operand.  Bias row n holds, at k = 2L and 2L + 1,
 // the bf16 high and low parts of layer L's bias b_L[n] (b - hi rounded again), so
 // the MMA adds hi + lo, b to about 2^-16 relative.  Layer L's ones operand has
-// 1 at k = 2L, 2L + 1 in every row: one 8 x 8 core matrix read for all 16 row
-// groups (stride byte offset 0), its k = 8-15 half a zero core matrix.
+// 1 at k = 2L, 2L + 1 in every row and 0 elsewhere; k = 8-15 read the bias rows again.
 constexpr int tBB = tB4 + kB4Rows * kHid * 2;     // 64 rows x 8 k (16 bytes a row)
-constexpr int tOnes = tBB + kHid * 16;            // 4 ones core matrices + 1 zero core matrix
-constexpr int tA = tOnes + 5 * 128;               // per group 128 x 64 (layer 1 uses 128 x 32)
-constexpr int kABytes = kRows * kHid * 2;
-// Staging of a tile's own inputs: normal, albedo, few-ray light, direct light
-// (16 bytes a pixel each) and depth moments (8).
-constexpr int sNormal = 0, sAlbedo = 2048, sLight = 4096, sDirect = 6144, sMoments = 8192;
-constexpr int kStageBytes = 9216;
-constexpr int tStage = tA + kGroups * kABytes;
+// Staging of a tile's own inputs: normal, albedo, few-ray light, direct light, filtered
+// few-ray light (16 bytes a pixel each) and depth moments (8).
+constexpr int sNormal = 0, sAlbedo = 2048, sLight = 4096, sDirect = 6144, sFiltered = 8192, sMoments = 10240;
+constexpr int kStageBytes = 11264;
+constexpr int tStage = tBB + kHid * 16;
 constexpr int tBar = tStage + kGroups * kStageBytes;  // per group: MMA mbarrier, staging mbarrier
-constexpr int tTmem = tBar + 16 * kGroups;
+constexpr int tPattern = tBar + 16 * kGroups;         // features 29 and 30 of an interleave pattern's pixels
+constexpr int tTmem = tPattern + 2 * 64 * 4;
 constexpr int kSmemTc = tTmem + 8;
 static_assert(tStage % 128 == 0 && kStageBytes % 128 == 0, "bulk copy destinations");
-static_assert(tBB % 128 == 0 && tOnes % 128 == 0 && tA % 128 == 0 && kABytes % 128 == 0 && tBar % 8 == 0,
-              "alignment");
+static_assert(tBB % 128 == 0 && tBar % 8 == 0, "alignment");
 
 __device__ int g_tc_errors;  // waits that ran out (kept across launches)
 constexpr long long kWaitCycles = 1ll << 31;  // ~1 s of SM clocks
@@ -114,6 +120,15 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+// The same with A in tensor memory (lane = row, a column = two consecutive k).
+__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
 
@@ -200,6 +215,23 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 32-bit columns of this thread's lane written to tensor memory; tmem_st_wait before the
+// barrier that precedes the MMA that reads them.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
+          taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   const bf16 x = __float2bfloat16_rn(a), y = __float2bfloat16_rn(b);
   return (uint32_t)__bfloat16_as_ushort(x) | ((uint32_t)__bfloat16_as_ushort(y) << 16);
@@ -239,19 +271,19 @@ __device__ __forceinline__ bool group_any(int group, bool v) {
   return r != 0;
 }
 
-// Makes this group's A operand visible to the tensor cores, issues the layer's
-// bias MMA and its K/16 MMAs from the group's first thread and waits for them; the
-// fence after the wait orders their completion before the accumulator reads.  `bad`
-// is set on a thread whose wait runs out; returns false (on every thread of the
-// group) if an earlier one did.
+// Makes this group's A operand (its columns of tensor memory, written by every thread)
+// visible to the tensor cores, issues the layer's bias MMA and its K/16 MMAs from the
+// group's first thread and waits for them; the fence after the wait orders their
+// completion before the accumulator reads.  `bad` is set on a thread whose wait runs
+// out; returns false (on every thread of the group) if an earlier one did.
 // The B operand's row-group stride is K * 16 bytes, or 0 when its N = 16 rows
 // re-read the first 8 (the output layer).
 // `first` runs on the issuing thread after the barrier, before the MMAs.
 template <int K, int N, int L, typename First>
-__device__ __forceinline__ bool run_layer(uint32_t sbase, int a_off, int b_off, uint32_t tmem, uint32_t bar,
+__device__ __forceinline__ bool run_layer(uint32_t sbase, uint32_t ones, int b_off, uint32_t tmem, uint32_t bar,
                                           uint32_t& phase, int group, bool& bad, First first,
                                           long long limit = kWaitCycles) {
-  fence_async_smem();
+  tmem_st_wait();
   fence_before();
   if (group_any(group, bad)) return false;
   fence_after();
@@ -259,13 +291,10 @@ __device__ __forceinline__ bool run_layer(uint32_t sbase, int a_off, int b_off, 
     first();
     constexpr uint32_t idesc = idesc_bf16(kRows, N);
     constexpr uint32_t b_sbo = (N == kOutPad) ? 0u : (uint32_t)(K * 16);
-    mma_bf16(tmem, smem_desc(sbase + tOnes + 128 * L, 512 - 128 * L, 0), smem_desc(sbase + tBB, 0, 128), idesc, 0u);
+    mma_bf16_ts(tmem, ones + kOnesCols * L, smem_desc(sbase + tBB, 0, 128), idesc, 0u);
 #pragma unroll
-    for (int j = 0; j < K / 16; j++) {
-      const uint64_t ad = smem_desc(sbase + a_off + j * 256, 128, K * 16);
-      const uint64_t bd = smem_desc(sbase + b_off + j * 256, 128, b_sbo);
-      mma_bf16(tmem, ad, bd, idesc, 1u);
-    }
+    for (int j = 0; j < K / 16; j++)
+      mma_bf16_ts(tmem, tmem + cA + 8 * j, smem_desc(sbase + b_off + j * 256, 128, b_sbo), idesc, 1u);
     mma_commit(bar);
   }
   if (!mbar_wait(bar, phase, limit)) bad = true;
@@ -277,19 +306,15 @@ __device__ __forceinline__ bool run_layer(uint32_t sbase, int a_off, int b_off, 
 
 // Hidden-layer epilogue: accumulator lane (bias included) -> ReLU -> bf16 row
 // of the next A operand (K = 64).
-__device__ __forceinline__ void hidden_epilogue(uint32_t a_base, uint32_t taddr) {
-  const int m = threadIdx.x & (kRows - 1);
+__device__ __forceinline__ void hidden_epilogue(uint32_t lane_addr) {
 #pragma unroll
   for (int c = 0; c < kHid; c += 32) {
     float v[32];
-    tmem_ld32(taddr + c, v);
+    tmem_ld32(lane_addr + c, v);
+    uint32_t r[16];
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-      const int k = c + 8 * h;
-      st_shared_v4(a_base + cm_off(m, k, kHid), pack_relu_bf16(v[8 * h + 0], v[8 * h + 1]),
-                   pack_relu_bf16(v[8 * h + 2], v[8 * h + 3]), pack_relu_bf16(v[8 * h + 4], v[8 * h + 5]),
-                   pack_relu_bf16(v[8 * h + 6], v[8 * h + 7]));
-    }
+    for (int k = 0; k < 16; k++) r[k] = pack_relu_bf16(v[2 * k], v[2 * k + 1]);
+    tmem_st16(lane_addr + cA + c / 2, r);
   }
 }
 
@@ -302,6 +327,7 @@ __device__ __forceinline__ void stage_tile(const FeatureArgs& a, int t, uint32_t
   bulk_g2s(buf + sAlbedo, a.albedo + 4 * p0, 16 * kRows, bar);
   bulk_g2s(buf + sLight, a.indirect[0] + 4 * p0, 16 * kRows, bar);
   bulk_g2s(buf + sDirect, a.direct + 4 * p0, 16 * kRows, bar);
+  bulk_g2s(buf + sFiltered, a.filtered + 4 * p0, 16 * kRows, bar);
   bulk_g2s(buf + sMoments, a.moments + 2 * p0, 8 * kRows, bar);
 }
 
@@ -321,7 +347,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   const uint32_t sbar = bar + 8;                   // staging copies
   const uint32_t stage = sbase + tStage + group * kStageBytes;
   const unsigned char* stage_p = smem + tStage + group * kStageBytes;
-  const int a_off = tA + group * kABytes;
 
   stage_b(smem, tB1, wb + qW1, kIn, kHid, kHid);
   stage_b(smem, tB2, wb + qW2, kHid, kHid, kHid);
@@ -339,11 +364,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     const bf16 v = (k & 1) ? __float2bfloat16_rn(b - __bfloat162float(hi)) : hi;
     *reinterpret_cast<bf16*>(smem + tBB + n * 16 + k * 2) = v;
   }
-  // Ones operands: core matrix L (8 rows x 8 k) is 1 at k = 2L, 2L + 1; core 4 is zero.
-  for (int i = tid; i < 5 * 64; i += kTcThreads) {
-    const int L = i >> 6, k = i & 7;
-    *reinterpret_cast<bf16*>(smem + tOnes + 2 * i) = __float2bfloat16_rn((L < 4 && (k >> 1) == L) ? 1.0f : 0.0f);
-  }
+  float* pattern = reinterpret_cast<float*>(smem + tPattern);
+  if (!ROWS && tid < a.pattern * a.pattern) pattern_features(tid, a.pattern, pattern[tid], pattern[64 + tid]);
   if (gtid == 0) {
     mbar_init(bar, 1);
     mbar_init(sbar, 1);
@@ -358,9 +380,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   fence_before();
   __syncthreads();
   fence_after();
-  // This group's 64 accumulator columns; this warp's 32 lanes of them.
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + tTmem) + (uint32_t)(64 * group);
-  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  // The ones operands, by the first group; the others' first MMAs wait for them.
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem + tTmem);
+  const uint32_t warp_lanes = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t ones = tmem_base + cOnes;
+  if (group == 0) {
+#pragma unroll
+    for (int L = 0; L < 4; L++) {
+      uint32_t r[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) r[k] = k == L ? 0x3F803F80u : 0u;
+      tmem_st8(ones + kOnesCols * L + warp_lanes, r);
+    }
+    tmem_st_wait();
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  // This group's columns; this warp's 32 lanes of them.
+  const uint32_t tmem = tmem_base + kGroupCols * group;
+  const uint32_t lane_addr = tmem + warp_lanes;
 
   const int W = a.width, n = a.width * a.height;
   const int tiles = (n + kRows - 1) / kRows;
@@ -372,8 +411,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   const int first_tile = t;
   bool pending = staged && t < full_tiles;  // a staging copy of tile t in flight
   if (pending && gtid == 0) stage_tile(a, t, stage, sbar);
+  // The pixel's place, advanced by whole strides instead of divided anew.
+  int x = (t * kRows + gtid) % W, y = (t * kRows + gtid) / W;
+  const int step_x = stride * kRows % W, step_y = stride * kRows / W;
   for (; t < tiles && !failed; t += stride) {
     const int p = t * kRows + gtid;
+    const int px = x, py = y;
+    x += step_x;
+    y += step_y;
+    if (x >= W) {
+      x -= W;
+      y++;
+    }
     float f[kIn];
     float scale = 1.0f;
     if (ROWS) {  // the row's bf16 features (exact in float) and its scale
@@ -403,9 +452,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
       const float4 al = reinterpret_cast<const float4*>(stage_p + sAlbedo)[gtid];
       const float4 li = reinterpret_cast<const float4*>(stage_p + sLight)[gtid];
       const float4 dl = reinterpret_cast<const float4*>(stage_p + sDirect)[gtid];
-      pixel_features_from(a, p % W, p / W, depth, n4, al, li, dl, f, scale);
+      const float4 fl = reinterpret_cast<const float4*>(stage_p + sFiltered)[gtid];
+      pixel_features_from(a, px, py, depth, n4, al, li, dl, fl, pattern, f, scale);
     } else if (p < n) {
-      pixel_features(a, p % W, p / W, f, scale);
+      pixel_features(a, px, py, pattern, f, scale);
     } else {
 #pragma unroll
       for (int i = 0; i < kIn; i++) f[i] = 0.0f;
@@ -413,10 +463,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     // The staging buffer takes the group's next tile once every thread has its
     // features: issued after the first layer's barrier.
     const bool prefetch = staged && t + stride < full_tiles;
+    {
+      uint32_t r[kIn / 2];
 #pragma unroll
-    for (int c = 0; c < kIn; c += 8)
-      st_shared_v4(sbase + a_off + cm_off(gtid, c, kIn), pack_bf16(f[c], f[c + 1]), pack_bf16(f[c + 2], f[c + 3]),
-                   pack_bf16(f[c + 4], f[c + 5]), pack_bf16(f[c + 6], f[c + 7]));
+      for (int k = 0; k < kIn / 2; k++) r[k] = pack_bf16(f[2 * k], f[2 * k + 1]);
+      __syncwarp();
+      tmem_st16(lane_addr + cA, r);
+    }
     // The head blends candidate estimates as the network saw them (bf16).
     float cand[3][3];
 #pragma unroll
@@ -432,17 +485,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     };
     auto nothing = [] {};
     const long long first_limit = t == first_tile ? g_tc_first_wait_cycles : kWaitCycles;
-    if (!run_layer<kIn, kHid, 0>(sbase, a_off, tB1, tmem, bar, phase, group, bad, issue_next, first_limit)) {
+    if (!run_layer<kIn, kHid, 0>(sbase, ones, tB1, tmem, bar, phase, group, bad, issue_next, first_limit)) {
       failed = true;
       break;
     }
     pending = prefetch;
-    hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kHid, 1>(sbase, a_off, tB2, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
-    hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kHid, 2>(sbase, a_off, tB3, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
-    hidden_epilogue(sbase + a_off, lane_addr);
-    if (!run_layer<kHid, kOutPad, 3>(sbase, a_off, tB4, tmem, bar, phase, group, bad, nothing)) {
+    hidden_epilogue(lane_addr);
+    if (!run_layer<kHid, kHid, 1>(sbase, ones, tB2, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
+    hidden_epilogue(lane_addr);
+    if (!run_layer<kHid, kHid, 2>(sbase, ones, tB3, tmem, bar, phase, group, bad, nothing)) { failed = true; break; }
+    hidden_epilogue(lane_addr);
+    if (!run_layer<kHid, kOutPad, 3>(sbase, ones, tB4, tmem, bar, phase, group, bad, nothing)) {
       failed = true;
       break;
     }
@@ -466,7 +519,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   __syncthreads();
   fence_after();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem - (uint32_t)(64 * group)),
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(kTmemCols)
                  : "memory");
 }
@@ -842,15 +895,18 @@ static int reconstruct_grid_cap(int* cap) {
   std::lock_guard<std::mutex> lock(g_tc_mutex);
   if (dev >= 64) return fail(GI_ERR_UNSUPPORTED, "reconstruct: device index");
   if (!g_tc_grid[dev]) {
-    int sms = 0, optin = 0;
+    int sms = 0, optin = 0, per_sm = kSmemTc + 1024;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     if (optin < kSmemTc) return fail(GI_ERR_UNSUPPORTED, "reconstruct: not enough shared memory per block");
     for (auto kernel : {mlp_reconstruct_kernel<false>, mlp_reconstruct_kernel<true>}) {
       e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTc),
                      "reconstruct: smem attribute");
       if (e) return e;
-      e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
+      // Shared memory for the one CTA; the rest of the SM's storage is L1 for the taps.
+      e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          (kSmemTc + 1024) * 100 / per_sm + 1),
                      "reconstruct: carveout");
       if (e) return e;
     }
@@ -872,7 +928,7 @@ int launch_reconstruct(const FeatureArgs& a, const __nv_bfloat16* wb, const floa
   if (grid <= 0) return GI_OK;
   // The staging copies need 16-byte aligned sources.
   const int staged = aligned16(a.normal) && aligned16(a.albedo) && aligned16(a.indirect[0]) && aligned16(a.direct) &&
-                     aligned16(a.moments);
+                     aligned16(a.moments) && aligned16(a.filtered);
   mlp_reconstruct_kernel<false><<<grid, kTcThreads, kSmemTc, stream>>>(a, wb, params, out, staged);
   GI_CHECK_LAUNCH("mlp_reconstruct_kernel");
   count_launches(1);
