@@ -193,35 +193,79 @@ __global__ void __launch_bounds__(kThreads) mip_tail_kernel(const __grid_constan
 
 // ---------------------------------------------------------------------------
 // Blur (blurLayerBuilder.frag:17-35): taps x outer, y inner, over [-r, r).
-constexpr int kBlurTx = 32, kBlurTy = 8;
+constexpr int kBlurTx = 32, kBlurTy = 8;  // threads of a CTA
+constexpr int kBlurRows = 4;              // rows of a thread
+constexpr int kBlurTileY = kBlurTy * kBlurRows;
+
+template <int CH> struct TexelOf;
+template <> struct TexelOf<4> { using T = float4; };
+template <> struct TexelOf<2> { using T = float2; };
+template <> struct TexelOf<1> { using T = float; };
+__device__ __forceinline__ float4 add_texel(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float2 add_texel(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float add_texel(float a, float b) { return a + b; }
+__device__ __forceinline__ float4 scale_texel(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
+__device__ __forceinline__ float2 scale_texel(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+__device__ __forceinline__ float scale_texel(float a, float s) { return a * s; }
+
+// The pyramids' radius 2: four rows of a column a thread, whose windows share 7 rows of
+// texels, so that it reads 28 texels instead of 64; each output sums its 16 in the order
+// above.  Bound by instructions when every output read its own: both pyramids of
+// 1920 x 1080 22.3 -> 11.7 us, the light alone 12.5 -> 9.4, the depth 12.8 -> 6.8.
+template <int CH> __device__ void blur2_tile(const BlurJob& J, int x, int y0) {
+  using T = typename TexelOf<CH>::T;
+  const T* src = reinterpret_cast<const T*>(J.src);
+  int row[kBlurRows + 3];
+#pragma unroll
+  for (int r = 0; r < kBlurRows + 3; r++) row[r] = dev::iclamp(y0 + r - 2, 0, J.h - 1) * J.w;
+  T sum[kBlurRows];
+#pragma unroll
+  for (int dx = -2; dx < 2; dx++) {
+    const int sx = dev::iclamp(x + dx, 0, J.w - 1);
+    T t[kBlurRows + 3];
+#pragma unroll
+    for (int r = 0; r < kBlurRows + 3; r++) t[r] = __ldg(src + row[r] + sx);
+#pragma unroll
+    for (int k = 0; k < kBlurRows; k++)
+#pragma unroll
+      for (int dy = 0; dy < 4; dy++)
+        sum[k] = dx == -2 && dy == 0 ? add_texel(T{}, t[k]) : add_texel(sum[k], t[k + dy]);
+  }
+  T* dst = reinterpret_cast<T*>(J.dst);
+#pragma unroll
+  for (int k = 0; k < kBlurRows; k++)
+    if (y0 + k < J.h) dst[(size_t)(y0 + k) * J.w + x] = scale_texel(sum[k], rcp_(16.0f));
+}
 
 template <int CH> __device__ void blur_tile(const BlurJob& J, int tile) {
   const int tx = tile % J.tiles_x, ty = tile / J.tiles_x;
   const int x = tx * kBlurTx + (threadIdx.x % kBlurTx);
-  const int y = ty * kBlurTy + (threadIdx.x / kBlurTx);
-  if (x >= J.w || y >= J.h) return;
+  const int y0 = ty * kBlurTileY + (threadIdx.x / kBlurTx) * kBlurRows;
+  if (x >= J.w || y0 >= J.h) return;
   const int r = J.radius;
-  float4 out;
-  if (r == 0) {
-    out = load_texel<CH>(J.src, (size_t)y * J.w + x);
-  } else {
-    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float tw = 0.0f;
-    for (int dx = -r; dx < r; dx++) {
-      int sx = dev::iclamp(x + dx, 0, J.w - 1);
-      for (int dy = -r; dy < r; dy++) {
-        int sy = dev::iclamp(y + dy, 0, J.h - 1);
-        float4 t = load_texel<CH>(J.src, (size_t)sy * J.w + sx);
-        s.x = s.x + t.x;
-        s.y = s.y + t.y;
-        s.z = s.z + t.z;
-        s.w = s.w + t.w;
-        tw = tw + 1.0f;
-      }
-    }
-    out = make_float4(div_(s.x, tw), div_(s.y, tw), div_(s.z, tw), div_(s.w, tw));
+  if (r == 2) {
+    blur2_tile<CH>(J, x, y0);
+    return;
   }
-  store_texel<CH>(J.dst, (size_t)y * J.w + x, out);
+  for (int y = y0; y < min(y0 + kBlurRows, J.h); y++) {
+    float4 out;
+    if (r == 0) {
+      out = load_texel<CH>(J.src, (size_t)y * J.w + x);
+    } else {
+      float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float tw = 0.0f;
+      for (int dx = -r; dx < r; dx++) {
+        int sx = dev::iclamp(x + dx, 0, J.w - 1);
+        for (int dy = -r; dy < r; dy++) {
+          int sy = dev::iclamp(y + dy, 0, J.h - 1);
+          s = add_texel(s, load_texel<CH>(J.src, (size_t)sy * J.w + sx));
+          tw = tw + 1.0f;
+        }
+      }
+      out = make_float4(div_(s.x, tw), div_(s.y, tw), div_(s.z, tw), div_(s.w, tw));
+    }
+    store_texel<CH>(J.dst, (size_t)y * J.w + x, out);
+  }
 }
 
 __global__ void __launch_bounds__(kBlurTx * kBlurTy) blur_kernel(const __grid_constant__ BlurJobs jobs) {
@@ -266,7 +310,7 @@ int launch_blur(BlurJobs& jobs, cudaStream_t stream) {
   for (int j = 0; j < jobs.count; j++) {
     BlurJob& J = jobs.job[j];
     J.tiles_x = (J.w + kBlurTx - 1) / kBlurTx;
-    int tiles_y = (J.h + kBlurTy - 1) / kBlurTy;
+    int tiles_y = (J.h + kBlurTileY - 1) / kBlurTileY;
     J.tile_begin = total;
     total += J.tiles_x * tiles_y;
   }
