@@ -218,8 +218,23 @@ class Renderer {
     // Temporal feedback: the previous frame's gathered image is this frame's light.
     float* prev = prev_lit_ ? rg_.ResolveView(prev_lit_->imageViewProxy->Id()).level(0) : nullptr;
     const bool from_prev = prev && have_prev_;
+    // The last bounce's last light stage writes the caller's indirect image in place of
+    // its own buffer, unless that image overlaps one the gather still reads or writes.
+    auto apart = [&](const float* q, int ch) {
+      const char* a0 = reinterpret_cast<const char*>(out_ind);
+      const char* b0 = reinterpret_cast<const char*>(q);
+      const size_t px = (size_t)w * h;
+      return a0 + px * 16 <= b0 || b0 + px * 4 * ch <= a0;
+    };
+    const bool write_ind = out_ind && aligned16(out_ind) && apart(in.albedo, 4) && apart(in.normal, 4) &&
+                           apart(in.depth_moments, 2) && apart(in.ndc_depth, 1) && apart(in.direct, 4) &&
+                           apart(out_lit, 4);
     for (int b = 0; b < p.bounces; b++) {
       const bool first = b == 0, last = b + 1 == p.bounces;
+      const bool to_caller = last && write_ind, filters = p.bilateral && !mlp_, denoises = p.denoise_radius > 0;
+      float* const b_den = to_caller ? out_ind : den;
+      float* const b_filt = to_caller && !denoises ? out_ind : filt;
+      float* const b_ind = to_caller && !denoises && !filters ? out_ind : ind;  // without a network
       std::vector<float*> lvl = ll, lbl = lb;
       lvl[0] = first ? (from_prev ? prev : const_cast<float*>(in.direct)) : lit_tmp;
       lbl[0] = lvl[0];
@@ -291,7 +306,7 @@ class Renderer {
       // for a plain bounce that re-lights the first one's record (the replay
       // takes software light taps).
       const MarchArgs plain_args =
-          mlp_ ? MarchArgs{} : with_record(march_args(p.march.dirs, plain_sd, ind), 0);
+          mlp_ ? MarchArgs{} : with_record(march_args(p.march.dirs, plain_sd, b_ind), 0);
       const bool pack_light = ltex && (mlp_ || plain_args.rec != 2);
       rg_.AddPass(legit::RenderGraph::RenderPassDesc()
                       .SetProfilerInfo(legit::Colors::wisteria, "BlurPass")
@@ -305,7 +320,7 @@ class Renderer {
                         if (first && dtex) legit::Check(dtex->Pack(db.data(), 2, ctx.GetCommandBuffer()), "BlurPass");
                         if (pack_light) legit::Check(ltex->Pack(lbl.data(), 4, ctx.GetCommandBuffer()), "BlurPass");
                       }));
-      const float* cur = ind;
+      const float* cur = b_ind;
       if (!mlp_) {
         const MarchArgs ma = plain_args;
         rg_.AddPass(legit::RenderGraph::RenderPassDesc()
@@ -315,7 +330,7 @@ class Renderer {
                         }));
       } else {
         std::vector<float*> few = levels_of(*few_pyr_, rg_);
-        float* learned = rg_.ResolveView(learned_->imageViewProxy->Id()).level(0);
+        float* learned = to_caller && !denoises ? out_ind : rg_.ResolveView(learned_->imageViewProxy->Id()).level(0);
         float* plain = rg_.ResolveView(plain_->imageViewProxy->Id()).level(0);
         float* few_f = rg_.ResolveView(few_f_->imageViewProxy->Id()).level(0);
         const gi_mlp* mlp = mlp_;
@@ -389,32 +404,32 @@ class Renderer {
       }
       // The learned result is already a filtered estimate (residual over the
       // bilaterally filtered few-ray light), so it is not filtered again.
-      if (p.bilateral && !mlp_) {
+      if (filters) {
         const float* src = cur;
         rg_.AddPass(legit::RenderGraph::RenderPassDesc()
                         .SetProfilerInfo(legit::Colors::greenSea, "BilateralPass")
                         .SetRecordFunc([=](legit::RenderGraph::RenderPassContext ctx) {
-                          legit::Check(launch_bilateral(src, in.depth_moments, 2, in.normal, filt, w, h,
+                          legit::Check(launch_bilateral(src, in.depth_moments, 2, in.normal, b_filt, w, h,
                                                         ctx.GetCommandBuffer(), fast_filters),
                                        "BilateralPass");
                         }));
-        cur = filt;
+        cur = b_filt;
       }
-      if (p.denoise_radius > 0) {
+      if (denoises) {
         const float* src = cur;
         const int r = p.denoise_radius;
         rg_.AddPass(legit::RenderGraph::RenderPassDesc()
                         .SetProfilerInfo(legit::Colors::greenSea, "DenoiserPass")
                         .SetRecordFunc([=](legit::RenderGraph::RenderPassContext ctx) {
-                          legit::Check(gi_denoise(src, in.depth_moments, in.normal, den, w, h, r,
+                          legit::Check(gi_denoise(src, in.depth_moments, in.normal, b_den, w, h, r,
                                                   ctx.GetCommandBuffer()),
                                        "DenoiserPass");
                         }));
-        cur = den;
+        cur = b_den;
       }
       float* dst = last ? out_lit : lit_tmp;
       const float* fin = cur;
-      const bool copy_ind = last && out_ind;
+      const bool copy_ind = last && out_ind && !write_ind;
       rg_.AddPass(legit::RenderGraph::RenderPassDesc()
                       .SetProfilerInfo(legit::Colors::pomegranate, "GatheringPass")
                       .SetRecordFunc([=](legit::RenderGraph::RenderPassContext ctx) {
