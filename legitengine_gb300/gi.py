@@ -193,30 +193,61 @@ def _torch():
     return torch
 
 
-def _stream():
+# The arguments of a call, as integers: a pass of 1920x1080 pyramids takes four calls of
+# up to 20 images, and was bound by building their arguments (an import and a ctypes
+# object each, a stream object a call): 89 us a pass, now 47, about its kernels' time.
+_float32 = None
+_raw_stream = None
+
+
+def _stream() -> int:
+    """The current stream's handle."""
+    if _raw_stream is None:
+        return _first_stream()
+    return _raw_stream(_device())
+
+
+def _first_stream() -> int:
+    """Initialises torch's CUDA side, after which the handle can be asked for by itself."""
+    global _raw_stream, _device
     torch = _torch()
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    handle = torch.cuda.current_stream().cuda_stream
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is not None and dev is not None:
+        _raw_stream, _device = raw, dev
+    return handle
 
 
-def _ptr(t) -> C.c_void_p:
+_device = None
+
+
+def _ptr(t) -> int:
+    global _float32
     if t is None:
-        return C.c_void_p(0)
-    torch = _torch()
-    assert t.is_cuda and t.dtype == torch.float32 and t.is_contiguous(), "expected a contiguous fp32 CUDA tensor"
-    return C.c_void_p(t.data_ptr())
+        return 0
+    if _float32 is None:
+        _float32 = _torch().float32
+    assert t.is_cuda and t.dtype is _float32 and t.is_contiguous(), "expected a contiguous fp32 CUDA tensor"
+    return t.data_ptr()
 
 
-def _dptr(t) -> C.c_void_p:
+def _dptr(t) -> int:
     """Device pointer of any contiguous CUDA tensor (bf16 features, int32 tile lists)."""
     if t is None:
-        return C.c_void_p(0)
+        return 0
     assert t.is_cuda and t.is_contiguous(), "expected a contiguous CUDA tensor"
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_arrays: dict = {}  # ctypes array types by length
 
 
 def _ptrs(ts: Sequence) -> C.Array:
-    arr = (C.c_void_p * len(ts))(*[_ptr(t).value for t in ts])
-    return arr
+    n = len(ts)
+    kind = _arrays.get(n)
+    if kind is None:
+        kind = _arrays[n] = C.c_void_p * n
+    return kind(*map(_ptr, ts))
 
 
 def mip_level_count(w: int, h: int, requested: int = 10) -> int:
@@ -393,8 +424,7 @@ class Renderer:
         _check(lib().gi_renderer_create(w, h, C.byref(p), C.byref(self._h)), "gi_renderer_create")
 
     def render(self, view: GiView, albedo, normal, moments, ndc, direct, out_lit, out_indirect=None):
-        inp = GiFrameInputs(_ptr(albedo).value, _ptr(normal).value, _ptr(moments).value, _ptr(ndc).value,
-                            _ptr(direct).value)
+        inp = GiFrameInputs(_ptr(albedo), _ptr(normal), _ptr(moments), _ptr(ndc), _ptr(direct))
         _check(lib().gi_renderer_render(self._h, C.byref(view), C.byref(inp), _ptr(out_lit), _ptr(out_indirect),
                                         _stream()), "gi_renderer_render")
 
@@ -479,7 +509,7 @@ def features(moments, normal, albedo, direct, indirect_levels, filtered, depth_b
     """indirect_levels: the few-ray indirect at mip levels (0, 2, 4); out: bf16 [pixels, 32];
     scale: fp32 [pixels], the exposure scale the light features are divided by."""
     h, w = normal.shape[0], normal.shape[1]
-    arr = (C.c_void_p * 3)(*[_ptr(t).value for t in indirect_levels])
+    arr = (C.c_void_p * 3)(*[_ptr(t) for t in indirect_levels])
     _check(lib().gi_features(w, h, pattern, _ptr(moments), _ptr(normal), _ptr(albedo), _ptr(direct), arr,
                              _ptr(filtered), _ptr(depth_blur_l2), _dptr(out), _ptr(scale), _dptr(tiles),
                              0 if tiles is None else tiles.numel(), _stream()), "gi_features")
@@ -622,10 +652,10 @@ class Batch:
         for i, v in enumerate(views):
             arr[i].view = v["view"]
             arr[i].march = v["march"]
-            arr[i].albedo, arr[i].normal = _ptr(v["albedo"]).value, _ptr(v["normal"]).value
-            arr[i].depth_moments, arr[i].ndc_depth = _ptr(v["moments"]).value, _ptr(v["ndc"]).value
-            arr[i].direct, arr[i].out_lit = _ptr(v["direct"]).value, _ptr(v["out_lit"]).value
-            arr[i].out_indirect = _ptr(v.get("out_indirect")).value
+            arr[i].albedo, arr[i].normal = _ptr(v["albedo"]), _ptr(v["normal"])
+            arr[i].depth_moments, arr[i].ndc_depth = _ptr(v["moments"]), _ptr(v["ndc"])
+            arr[i].direct, arr[i].out_lit = _ptr(v["direct"]), _ptr(v["out_lit"])
+            arr[i].out_indirect = _ptr(v.get("out_indirect"))
         self._h = C.c_void_p()
         _check(lib().gi_batch_create(arr, len(views), tile_rows, C.byref(self._h)), "gi_batch_create")
 
