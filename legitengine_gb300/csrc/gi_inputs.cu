@@ -13,10 +13,12 @@ namespace {
 
 using namespace dev;
 
-constexpr int kTx = 32, kTy = 4;         // direct light: one row of 32 pixels a warp
-constexpr int kCastX = 32, kCastY = 8;   // ray casts: tile of a CTA, in warps of 8 x 4 pixels
-constexpr int kCastThreads = kCastX * kCastY;
+constexpr int kTx = 32, kTy = 4;          // direct light: one row of 32 pixels a warp
+constexpr int kCastPix = 2;               // ray casts: pixels a thread, 4 rows apart
+constexpr int kCastX = 32, kCastY = 8 * kCastPix;  // tile of a CTA, in warps of 8 x (4 kCastPix) pixels
+constexpr int kCastThreads = kCastX * kCastY / kCastPix;
 constexpr int kPrimStage = 256;  // primitives staged per shared-memory batch
+constexpr int kOwnPrims = 4;     // of them that a lane bounds at a time
 
 struct ViewArgs {
   Mat4 inv_view_proj, inv_view, view_proj, view;
@@ -155,12 +157,29 @@ __device__ __forceinline__ float warp_max(float v) {
   return r;
 }
 
-__device__ __forceinline__ RayBounds ray_bounds(const float (&d)[3]) {
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+__device__ __forceinline__ RayBounds ray_bounds(const float (&d)[kCastPix][3]) {
   RayBounds r;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    r.dlo[k] = warp_min(d[k]);
-    r.dhi[k] = warp_max(d[k]);
+    float lo = d[0][k], hi = d[0][k];
+#pragma unroll
+    for (int q = 1; q < kCastPix; q++) {
+      lo = min_nan(lo, d[q][k]);
+      hi = max_nan(hi, d[q][k]);
+    }
+    r.dlo[k] = warp_min(lo);
+    r.dhi[k] = warp_max(hi);
     r.open[k] = !(r.dlo[k] >= 1e-37f || r.dhi[k] <= -1e-37f);
     // The rounded reciprocal decreases with d on each side of zero.
     r.ilo[k] = rcp_(r.dhi[k]);
@@ -256,21 +275,28 @@ __device__ __forceinline__ float prim_hit(const PrimTest& p, f3 d, const float (
 // (near root), ties kept by the earlier primitive.
 //
 // The cast was bound by its arithmetic, every ray testing every primitive.  Now each
-// lane of a warp bounds one primitive's distance to the warp's 8 x 4 pixels of rays
+// lane of a warp bounds one primitive's distance to the warp's 8 x 8 pixels of rays
 // (32 primitives in the time of one test), and the rays test the primitives in order
 // of that bound until it passes their farthest hit: the same nearest hit, bit for
-// bit.  Measured with 64 boxes and 16 spheres: the G-buffer at 1920 x 1080 319 -> 67 us, a
-// shadow map of 1024 x 1024 171 -> 27 us (87 and 35 us in index order, without the
-// order by distance).
-__device__ void cast_ray(const gi_prim* __restrict__ prims, int np, const MeshSet& mesh, f3 o, f3 d, Hit& h,
-                         PrimTest* s_prims) {
-  h.t = kInf;
-  h.prim = -1;
-  h.tri = -1;
-  h.obj = -1;
-  h.u = h.v = 0.0f;
-  const float iv[3] = {rcp_(d.x), rcp_(d.y), rcp_(d.z)};
-  const float dv[3] = {d.x, d.y, d.z};
+// bit.  Measured with 64 boxes and 16 spheres: the G-buffer at 1920 x 1080 319 -> 53 us, a
+// shadow map of 1024 x 1024 171 -> 20 us (in index order 87 and 35; one pixel a thread and
+// one primitive a lane at a time 67 and 27).
+__device__ __forceinline__ void cast_rays(const gi_prim* __restrict__ prims, int np, const MeshSet& mesh, f3 o,
+                                          const f3 (&d)[kCastPix], Hit (&h)[kCastPix], PrimTest* s_prims) {
+  float iv[kCastPix][3], dv[kCastPix][3];
+#pragma unroll
+  for (int q = 0; q < kCastPix; q++) {
+    h[q].t = kInf;
+    h[q].prim = -1;
+    h[q].tri = -1;
+    h[q].obj = -1;
+    h[q].u = h[q].v = 0.0f;
+    dv[q][0] = d[q].x;
+    dv[q][1] = d[q].y;
+    dv[q][2] = d[q].z;
+#pragma unroll
+    for (int k = 0; k < 3; k++) iv[q][k] = rcp_(dv[q][k]);
+  }
   const RayBounds bounds = ray_bounds(dv);
   const int lane = threadIdx.x & 31;
   float farthest = kInf;  // of the warp's hits so far
@@ -279,26 +305,48 @@ __device__ void cast_ray(const gi_prim* __restrict__ prims, int np, const MeshSe
     __syncthreads();
     for (int i = threadIdx.x; i < cnt; i += kCastThreads) s_prims[i] = prim_test(prims[base + i], o);
     __syncthreads();
-    for (int first = 0; first < cnt; first += 32) {
-      const int own = first + lane;
-      float entry = own < cnt ? nearest_entry(s_prims[own], bounds) : kInf;
+    for (int first = 0; first < cnt; first += 32 * kOwnPrims) {
+      // Each lane's primitives, 32 apart; the nearest of them and its place.
+      float entry[kOwnPrims];
+#pragma unroll
+      for (int k = 0; k < kOwnPrims; k++) {
+        const int own = first + 32 * k + lane;
+        entry[k] = own < cnt ? nearest_entry(s_prims[own], bounds) : kInf;
+      }
       for (;;) {
-        const float next = warp_min(entry);
-        if (next == kInf || next > farthest) break;
-        const int from = __ffs((int)__ballot_sync(0xffffffffu, entry == next)) - 1;
-        if (lane == from) entry = kInf;
-        const PrimTest p = s_prims[first + from];
-        const int prim = base + first + from;
-        const float t = bounds.closed && (p.kind & kFinite) ? prim_hit<true>(p, d, iv) : prim_hit<false>(p, d, iv);
-        if (t > 0.0f && (t < h.t || (t == h.t && prim < h.prim))) {
-          h.t = t;
-          h.prim = prim;
+        float mine = entry[0];
+        int place = 0;
+#pragma unroll
+        for (int k = 1; k < kOwnPrims; k++) {
+          place = entry[k] < mine ? k : place;
+          mine = fminf(mine, entry[k]);
         }
-        farthest = warp_max(h.t);
+        const float next = warp_min(mine);
+        if (next == kInf || next > farthest) break;
+        const int from = __ffs((int)__ballot_sync(0xffffffffu, mine == next)) - 1;
+        const int at = first + 32 * __shfl_sync(0xffffffffu, place, from) + from;
+#pragma unroll
+        for (int k = 0; k < kOwnPrims; k++)
+          if (first + 32 * k + lane == at) entry[k] = kInf;
+        const PrimTest p = s_prims[at];
+        const int prim = base + at;
+        const bool numbers = bounds.closed && (p.kind & kFinite);
+        float far = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kCastPix; q++) {
+          const float t = numbers ? prim_hit<true>(p, d[q], iv[q]) : prim_hit<false>(p, d[q], iv[q]);
+          if (t > 0.0f && (t < h[q].t || (t == h[q].t && prim < h[q].prim))) {
+            h[q].t = t;
+            h[q].prim = prim;
+          }
+          far = fmaxf(far, h[q].t);
+        }
+        farthest = warp_max(far);
       }
     }
   }
-  if (mesh.num_objects > 0) cast_mesh(mesh, o, d, iv, h);
+  if (mesh.num_objects > 0)
+    for (int q = 0; q < kCastPix; q++) cast_mesh(mesh, o, d[q], iv[q], h[q]);
 }
 
 // The surface normal at the hit of an analytic primitive.
@@ -317,47 +365,45 @@ __device__ __forceinline__ f3 prim_normal(const gi_prim& g, f3 o, f3 d, float t)
   return mk3(nv[0], nv[1], nv[2]);
 }
 
-// A thread's pixel and ray.  Threads past the image take its last row or column (they
+// A thread's pixels and rays.  Pixels past the image take its last row or column (they
 // join the warp's votes) and store nothing.
-struct CastPixel {
-  int x, y;
-  bool live;
-  f3 org, dir;
+struct CastPixels {
+  int x, y[kCastPix];
+  bool live[kCastPix];
+  f3 org, dir[kCastPix];
 };
-__device__ __forceinline__ CastPixel cast_pixel(const ViewArgs& v) {
-  CastPixel c;
+__device__ __forceinline__ CastPixels cast_pixels(const ViewArgs& v) {
+  CastPixels c;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  c.x = blockIdx.x * kCastX + (w & 3) * 8 + (l & 7);
-  c.y = blockIdx.y * kCastY + (w >> 2) * 4 + (l >> 3);
-  c.live = c.x < v.width && c.y < v.height;
-  c.x = min(c.x, v.width - 1);
-  c.y = min(c.y, v.height - 1);
-  const float sx = div_((float)c.x + 0.5f, (float)v.width), sy = div_((float)c.y + 0.5f, (float)v.height);
+  const int x = blockIdx.x * kCastX + (w & 3) * 8 + (l & 7);
+  c.x = min(x, v.width - 1);
+  const float sx = div_((float)c.x + 0.5f, (float)v.width);
   const float4 o4 = mat_vec(v.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
   c.org = mk3(o4.x, o4.y, o4.z);
-  c.dir = normalize3(sub3(unproject(v.inv_view_proj, sx, sy, 1.0f), c.org));
+#pragma unroll
+  for (int q = 0; q < kCastPix; q++) {
+    const int y = blockIdx.y * kCastY + ((w >> 2) * kCastPix + q) * 4 + (l >> 3);
+    c.live[q] = x < v.width && y < v.height;
+    c.y[q] = min(y, v.height - 1);
+    const float sy = div_((float)c.y[q] + 0.5f, (float)v.height);
+    c.dir[q] = normalize3(sub3(unproject(v.inv_view_proj, sx, sy, 1.0f), c.org));
+  }
   return c;
 }
 
 // gBufferBuilder.frag:28-38 at the primary hit.  The eight powers of a surface's
 // colours are the same for every pixel that shows it: a warp evaluates them once for
 // each of the surfaces it hits, four surfaces at a time, a lane per channel.
-__global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_constant__ ViewArgs v,
-                                                               const gi_prim* __restrict__ prims, int np, MeshSet mesh,
-                                                               float* __restrict__ albedo,
-                                                               float* __restrict__ emissive,
-                                                               float* __restrict__ normal,
-                                                               float* __restrict__ moments, float* __restrict__ ndc) {
-  __shared__ PrimTest s_prims[kPrimStage];
-  __shared__ __align__(16) float s_colour[kCastThreads / 32][32][8];  // a warp's surfaces: albedo, emissive
-  const CastPixel c = cast_pixel(v);
-  Hit h;
-  cast_ray(prims, np, mesh, c.org, c.dir, h, s_prims);
+__device__ __forceinline__ void shade(const ViewArgs& v, const gi_prim* __restrict__ prims, int np, const MeshSet& mesh,
+                                      int x, int y, bool live, f3 org, f3 dir, const Hit& h, float (&colour)[32][8],
+                                      float* __restrict__ albedo, float* __restrict__ emissive,
+                                      float* __restrict__ normal, float* __restrict__ moments,
+                                      float* __restrict__ ndc) {
   const int lane = threadIdx.x & 31;
-  auto& colour = s_colour[threadIdx.x >> 5];
   const int surface = h.prim >= 0 ? h.prim : (h.tri >= 0 ? np + h.obj : -1);
   int slot = 0;
   {
+    __syncwarp();  // the last pixel's colours have been read
     unsigned todo = __ballot_sync(0xffffffffu, surface >= 0);
     for (int n = 0; todo; n += 4) {  // four surfaces a round: lanes 8 k .. 8 k + 7 take the k-th
       int mine = -1;
@@ -378,8 +424,8 @@ __global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_cons
     }
     __syncwarp();
   }
-  if (!c.live) return;
-  const size_t i = (size_t)c.y * v.width + c.x;
+  if (!live) return;
+  const size_t i = (size_t)y * v.width + x;
   if (surface < 0) {
     reinterpret_cast<float4*>(albedo)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     reinterpret_cast<float4*>(emissive)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -388,12 +434,12 @@ __global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_cons
     ndc[i] = 1.0f;
     return;
   }
-  const f3 hit = add3(c.org, mul3s(c.dir, h.t));
-  const f3 dl = sub3(hit, c.org);
+  const f3 hit = add3(org, mul3s(dir, h.t));
+  const f3 dl = sub3(hit, org);
   const float delta_len = sqrtf(dot3(dl, dl));
   f3 n;
   if (h.prim >= 0) {
-    n = prim_normal(prims[h.prim], c.org, c.dir, h.t);
+    n = prim_normal(prims[h.prim], org, dir, h.t);
   } else {
     // Barycentric blend of the vertex normals, (1 - u - v) n0 + u n1 + v n2.
     const gi_triangle& tr = mesh.tris[h.tri];
@@ -408,17 +454,37 @@ __global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_cons
   ndc[i] = project(v.view_proj, hit).z;
 }
 
+__global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_constant__ ViewArgs v,
+                                                               const gi_prim* __restrict__ prims, int np, MeshSet mesh,
+                                                               float* __restrict__ albedo,
+                                                               float* __restrict__ emissive,
+                                                               float* __restrict__ normal,
+                                                               float* __restrict__ moments, float* __restrict__ ndc) {
+  __shared__ PrimTest s_prims[kPrimStage];
+  __shared__ __align__(16) float s_colour[kCastThreads / 32][32][8];  // a warp's surfaces: albedo, emissive
+  const CastPixels c = cast_pixels(v);
+  Hit h[kCastPix];
+  cast_rays(prims, np, mesh, c.org, c.dir, h, s_prims);
+#pragma unroll
+  for (int q = 0; q < kCastPix; q++)
+    shade(v, prims, np, mesh, c.x, c.y[q], c.live[q], c.org, c.dir[q], h[q], s_colour[threadIdx.x >> 5], albedo, emissive,
+          normal, moments, ndc);
+}
+
 __global__ void __launch_bounds__(kCastThreads) shadow_kernel(const __grid_constant__ ViewArgs v,
                                                               const gi_prim* __restrict__ prims, int np, MeshSet mesh,
                                                               float* __restrict__ out) {
   __shared__ PrimTest s_prims[kPrimStage];
-  const CastPixel c = cast_pixel(v);
-  Hit h;
-  cast_ray(prims, np, mesh, c.org, c.dir, h, s_prims);
-  if (!c.live) return;
-  float z = 1.0f;
-  if (h.prim >= 0 || h.tri >= 0) z = project(v.view_proj, add3(c.org, mul3s(c.dir, h.t))).z;
-  out[(size_t)c.y * v.width + c.x] = z;
+  const CastPixels c = cast_pixels(v);
+  Hit h[kCastPix];
+  cast_rays(prims, np, mesh, c.org, c.dir, h, s_prims);
+#pragma unroll
+  for (int q = 0; q < kCastPix; q++) {
+    if (!c.live[q]) continue;
+    float z = 1.0f;
+    if (h[q].prim >= 0 || h[q].tri >= 0) z = project(v.view_proj, add3(c.org, mul3s(c.dir[q], h[q].t))).z;
+    out[(size_t)c.y[q] * v.width + c.x] = z;
+  }
 }
 
 // directLighting.frag:45-79.
