@@ -20,20 +20,44 @@ template <int DCH> __device__ __forceinline__ float depth_at(const float* p, int
 
 // Bilateral: taps y outer, x inner over [-2, 2]; w = exp(-|d-d0|*10.5) *
 // exp(-|n-n0|^2*20) (weights of denoiser.frag:103,105), evaluated as one
-// exponential of the summed exponents; out = sum / (sumW + 1e-7).  The block's
-// (32+4) x (16+4) halo of light, depth and normal is staged in shared memory
-// (clamp-to-edge applied while staging), so every tap is a shared-memory read.
-// Each thread filters two vertically adjacent pixels: their windows share tap rows,
-// so a thread reads 6 rows of taps for its two outputs instead of 10, and the two
-// pixels' weights and sums are the halves of packed operations; each output still
-// sums its taps in the order above, with the same roundings.
-//
-// Bound by arithmetic.  The exact weight's exponential (expf_ without its branches:
-// here the argument is never positive) rounds and scales by packed adds and multiplies
-// instead of conversions and integer arithmetic: 3840 x 2160 315 -> 241 us (362 M
-// instructions before); the fast weights at 1920 x 1080 49.7 -> 47.5 us.
+// exponential of the summed exponents; out = sum / (sumW + 1e-7).  A block's halo of
+// light, depth and normal is staged in shared memory (clamp-to-edge applied while
+// staging), so every tap is a shared-memory read.  Each thread filters two vertically
+// adjacent pixels: their windows share tap rows, so a thread reads 6 rows of taps for
+// its two outputs instead of 10, and the two pixels' weights and sums are the halves of
+// packed operations; each output still sums its taps in the order above, with the same
+// roundings.  The fast weights (hardware exponential) are cheap and evaluated per tap;
+// the exact ones once for both pixels that share them (bilateral_exact_kernel).
 constexpr int kBilRows = 2;
-constexpr int kHx = kTx + 4, kHy = kTy * kBilRows + 4;
+constexpr int kHx = kTx + 4;
+
+// Texels of a 36 x HY halo from (x0, y0) on; xyz of the normal with the depth in w.
+// CENTRE: in the light's w (not filtered) the pixel's exact weight to itself, 1, or NaN
+// where its normal or depth is not finite.
+template <int DCH, int HY, int THREADS, bool CENTRE>
+__device__ __forceinline__ void stage_halo(const float* __restrict__ ind, const float* __restrict__ depth,
+                                           const float* __restrict__ normal, int w, int h, int x0, int y0,
+                                           float4* s_col, float4* s_nrm) {
+  // Every load out before the first is stored (fast weights at 1920 x 1080 47.6 -> 42.8 us).
+  constexpr int kOwn = (kHx * HY + THREADS - 1) / THREADS;
+  float4 c[kOwn], n[kOwn];
+#pragma unroll
+  for (int k = 0; k < kOwn; k++) {
+    const int i = min((int)(threadIdx.y * kTx + threadIdx.x) + k * THREADS, kHx * HY - 1);
+    const int q = iclamp(y0 + i / kHx, 0, h - 1) * w + iclamp(x0 + i % kHx, 0, w - 1);
+    c[k] = ld4(ind, q);
+    n[k] = ld4(normal, q);
+    n[k].w = depth_at<DCH>(depth, q);
+  }
+#pragma unroll
+  for (int k = 0; k < kOwn; k++) {
+    if (CENTRE)
+      c[k].w = 1.0f + ((n[k].x - n[k].x) + (n[k].y - n[k].y) + (n[k].z - n[k].z) + (n[k].w - n[k].w));
+    const int i = min((int)(threadIdx.y * kTx + threadIdx.x) + k * THREADS, kHx * HY - 1);
+    s_col[i] = c[k];
+    s_nrm[i] = n[k];
+  }
+}
 
 // expf_(-s) of both halves for s >= 0 or NaN, bit for bit.
 __device__ __forceinline__ p2 exp_neg(p2 s) {
@@ -63,54 +87,29 @@ __device__ __forceinline__ p2 exp_neg(p2 s) {
   return pmul(pmul(p, scale), pk(-2.7105054312137611e-20f));
 }
 
-// The weights of a tap of each pixel from the differences to their centres.  FAST (the
-// march's fast precision): by fused multiply-adds and the hardware exponential.
-template <bool FAST> __device__ __forceinline__ p2 bilateral_weights(p2 x, p2 y, p2 z, p2 d) {
-  if (FAST) {
-    const p2 m = pmul(pfma(z, z, pfma(y, y, pmul(x, x))), pk(20.0f));
-    return pk(__expf(-fmaf(fabsf(lo_(d)), 10.5f, lo_(m))), __expf(-fmaf(fabsf(hi_(d)), 10.5f, hi_(m))));
-  }
-  const p2 m = pmul(padd(padd(pmul(x, x), pmul(y, y)), pmul(z, z)), pk(20.0f));
-  d = pmul(d, pk(10.5f));
-  return exp_neg(pk(fabsf(lo_(d)) + lo_(m), fabsf(hi_(d)) + hi_(m)));
+__device__ __forceinline__ void store_filtered(float4* at, float x, float y, float z, float w) {
+  const float d = w + 1e-7f;
+  *at = make_float4(div_(x, d), div_(y, d), div_(z, d), 1.0f);
 }
 
-template <bool FAST> __device__ __forceinline__ float weigh(float sum, float v, float w) {
-  return FAST ? fmaf(v, w, sum) : sum + v * w;
-}
-template <bool FAST> __device__ __forceinline__ p2 weigh(p2 sum, float v, p2 w) {
-  return FAST ? pfma(pk(v), w, sum) : padd(sum, pmul(pk(v), w));
+// The fast weights of a tap of each pixel from the differences to their centres.
+__device__ __forceinline__ p2 fast_weights(p2 x, p2 y, p2 z, p2 d) {
+  const p2 m = pmul(pfma(z, z, pfma(y, y, pmul(x, x))), pk(20.0f));
+  return pk(__expf(-fmaf(fabsf(lo_(d)), 10.5f, lo_(m))), __expf(-fmaf(fabsf(hi_(d)), 10.5f, hi_(m))));
 }
 
-template <int DCH, bool FAST>
-__global__ void __launch_bounds__(kTx* kTy) bilateral_kernel(const float* __restrict__ ind,
-                                                             const float* __restrict__ depth,
-                                                             const float* __restrict__ normal,
-                                                             float* __restrict__ out, int w, int h) {
+// The march's fast precision: the weights by fused multiply-adds and the hardware
+// exponential, the sums by fused multiply-adds.
+template <int DCH>
+__global__ void __launch_bounds__(kTx* kTy) bilateral_fast_kernel(const float* __restrict__ ind,
+                                                                  const float* __restrict__ depth,
+                                                                  const float* __restrict__ normal,
+                                                                  float* __restrict__ out, int w, int h) {
+  constexpr int kHy = kTy * kBilRows + 4;
   __shared__ float4 s_col[kHy][kHx];
   __shared__ float4 s_nrm[kHy][kHx];  // xyz, w = depth
-  const int x0 = blockIdx.x * kTx - 2, y0 = blockIdx.y * (kTy * kBilRows) - 2;
-  {
-    // Three texels a thread, every load out before the first is stored (fast weights at
-    // 1920 x 1080 47.6 -> 42.8 us, exact at 3840 x 2160 241 -> 235).
-    constexpr int kOwn = (kHx * kHy + kTx * kTy - 1) / (kTx * kTy);
-    float4 c[kOwn], n[kOwn];
-#pragma unroll
-    for (int k = 0; k < kOwn; k++) {
-      const int i = min((int)(threadIdx.y * kTx + threadIdx.x) + k * kTx * kTy, kHx * kHy - 1);
-      const int hx = i % kHx, hy = i / kHx;
-      const int q = iclamp(y0 + hy, 0, h - 1) * w + iclamp(x0 + hx, 0, w - 1);
-      c[k] = ld4(ind, q);
-      n[k] = ld4(normal, q);
-      n[k].w = depth_at<DCH>(depth, q);
-    }
-#pragma unroll
-    for (int k = 0; k < kOwn; k++) {
-      const int i = min((int)(threadIdx.y * kTx + threadIdx.x) + k * kTx * kTy, kHx * kHy - 1);
-      (&s_col[0][0])[i] = c[k];
-      (&s_nrm[0][0])[i] = n[k];
-    }
-  }
+  stage_halo<DCH, kHy, kTx * kTy, false>(ind, depth, normal, w, h, blockIdx.x * kTx - 2, blockIdx.y * (kTy * kBilRows) - 2,
+                                  &s_col[0][0], &s_nrm[0][0]);
   __syncthreads();
   const int tx = threadIdx.x, ty = threadIdx.y * kBilRows;  // the thread's first tap within the tile
   const int x = blockIdx.x * kTx + tx, y = blockIdx.y * (kTy * kBilRows) + ty;
@@ -122,11 +121,11 @@ __global__ void __launch_bounds__(kTx* kTy) bilateral_kernel(const float* __rest
 #pragma unroll
   for (int dx = 0; dx < 5; dx++) {
     const float4 col = s_col[ty][tx + dx], n = s_nrm[ty][tx + dx], m = s_nrm[ty + 5][tx + dx];
-    const p2 wt = bilateral_weights<FAST>(pk(n.x - c0.x, m.x - c1.x), pk(n.y - c0.y, m.y - c1.y),
-                                          pk(n.z - c0.z, m.z - c1.z), pk(n.w - c0.w, m.w - c1.w));
-    sx = weigh<FAST>(sx, col.x, lo_(wt));
-    sy = weigh<FAST>(sy, col.y, lo_(wt));
-    sz = weigh<FAST>(sz, col.z, lo_(wt));
+    const p2 wt = fast_weights(pk(n.x - c0.x, m.x - c1.x), pk(n.y - c0.y, m.y - c1.y), pk(n.z - c0.z, m.z - c1.z),
+                               pk(n.w - c0.w, m.w - c1.w));
+    sx = fmaf(col.x, lo_(wt), sx);
+    sy = fmaf(col.y, lo_(wt), sy);
+    sz = fmaf(col.z, lo_(wt), sz);
     sw = sw + lo_(wt);
     last[dx] = hi_(wt);
   }
@@ -137,19 +136,15 @@ __global__ void __launch_bounds__(kTx* kTy) bilateral_kernel(const float* __rest
 #pragma unroll
     for (int dx = 0; dx < 5; dx++) {
       const float4 col = s_col[ty + r][tx + dx], n = s_nrm[ty + r][tx + dx];
-      const p2 wt = bilateral_weights<FAST>(psub(pk(n.x), cx), psub(pk(n.y), cy), psub(pk(n.z), cz), psub(pk(n.w), cd));
-      ax = weigh<FAST>(ax, col.x, wt);
-      ay = weigh<FAST>(ay, col.y, wt);
-      az = weigh<FAST>(az, col.z, wt);
+      const p2 wt = fast_weights(psub(pk(n.x), cx), psub(pk(n.y), cy), psub(pk(n.z), cz), psub(pk(n.w), cd));
+      ax = pfma(pk(col.x), wt, ax);
+      ay = pfma(pk(col.y), wt, ay);
+      az = pfma(pk(col.z), wt, az);
       aw = padd(aw, wt);
     }
   }
   float4* o = reinterpret_cast<float4*>(out) + (size_t)y * w + x;
-  auto store = [](float4* at, float vx, float vy, float vz, float vw) {
-    const float d = vw + 1e-7f;
-    *at = make_float4(div_(vx, d), div_(vy, d), div_(vz, d), 1.0f);
-  };
-  store(o, lo_(ax), lo_(ay), lo_(az), lo_(aw));
+  store_filtered(o, lo_(ax), lo_(ay), lo_(az), lo_(aw));
   if (y + 1 >= h) return;
   sx = hi_(ax);
   sy = hi_(ay);
@@ -158,12 +153,118 @@ __global__ void __launch_bounds__(kTx* kTy) bilateral_kernel(const float* __rest
 #pragma unroll
   for (int dx = 0; dx < 5; dx++) {
     const float4 col = s_col[ty + 5][tx + dx];
-    sx = weigh<FAST>(sx, col.x, last[dx]);
-    sy = weigh<FAST>(sy, col.y, last[dx]);
-    sz = weigh<FAST>(sz, col.z, last[dx]);
+    sx = fmaf(col.x, last[dx], sx);
+    sy = fmaf(col.y, last[dx], sy);
+    sz = fmaf(col.z, last[dx], sz);
     sw = sw + last[dx];
   }
-  store(o + w, sx, sy, sz, sw);
+  store_filtered(o + w, sx, sy, sz, sw);
+}
+
+// The exact weights.  Bound by the arithmetic of the exponentials, of which two pixels
+// that lie in each other's window have the same one (the differences change sign, their
+// squares and magnitudes do not).  So each pixel's weights to the 12 taps after it --
+// (1..2, 0), (-2..2, 1), (-2..2, 2) -- are evaluated once into shared memory, for the
+// tile and the two pixels around it on the left, right and above, and an output reads
+// its other 12 from the pixels before it.  The tile's height keeps the block within 48
+// KB; 8 and 14 rows measured 217 and 209 us against 209 with 12 before the last columns
+// of all rows became one warp's.  3840 x 2160: 315 us with scalar weights per tap, 235
+// with packed ones, 206 shared; bound by shared memory's accesses (85 % busy) now.
+constexpr int kExY = 6;                        // rows of threads
+constexpr int kExTile = kExY * kBilRows;       // rows of outputs
+constexpr int kExHy = kExTile + 4, kExWy = kExTile + 2;  // rows of the halo, and of weights
+
+template <int DCH>
+__global__ void __launch_bounds__(kTx* kExY) bilateral_exact_kernel(const float* __restrict__ ind,
+                                                                    const float* __restrict__ depth,
+                                                                    const float* __restrict__ normal,
+                                                                    float* __restrict__ out, int w, int h) {
+  constexpr int kThreads = kTx * kExY;
+  __shared__ float4 s_col[kExHy][kHx];
+  __shared__ float4 s_nrm[kExHy][kHx];  // xyz, w = depth
+  __shared__ float s_w[12][kExWy][kHx];
+  stage_halo<DCH, kExHy, kThreads, true>(ind, depth, normal, w, h, blockIdx.x * kTx - 2, blockIdx.y * kExTile - 2,
+                                   &s_col[0][0], &s_nrm[0][0]);
+  __syncthreads();
+  // Two rows of a column a lane: a warp takes two rows' first 32 columns, or the last
+  // four of all rows.  Taps past the halo's sides belong to pairs that no output has;
+  // they read its last column.
+  static_assert(kExWy / 2 * 4 <= 32, "the last columns of all rows are one warp's");
+  for (int u = threadIdx.y; u <= kExWy / 2; u += kExY) {
+    const bool body = u < kExWy / 2;
+    const int y = 2 * (body ? u : threadIdx.x / 4), x = body ? threadIdx.x : 32 + threadIdx.x % 4;
+    if (y >= kExWy) break;
+    const float4 c0 = s_nrm[y][x], c1 = s_nrm[y + 1][x];
+    auto weights = [&](int f, const float4& n, const float4& m) {  // taps of the upper and of the lower pixel
+      const p2 ex = pk(n.x - c0.x, m.x - c1.x), ey = pk(n.y - c0.y, m.y - c1.y), ez = pk(n.z - c0.z, m.z - c1.z);
+      const p2 q = pmul(padd(padd(pmul(ex, ex), pmul(ey, ey)), pmul(ez, ez)), pk(20.0f));
+      const p2 d = pmul(pk(n.w - c0.w, m.w - c1.w), pk(10.5f));
+      const p2 wt = exp_neg(pk(fabsf(lo_(d)) + lo_(q), fabsf(hi_(d)) + hi_(q)));
+      s_w[f][y][x] = lo_(wt);
+      s_w[f][y + 1][x] = hi_(wt);
+    };
+#pragma unroll
+    for (int dx = -2; dx <= 2; dx++) {
+      const int sx = iclamp(x + dx, 0, kHx - 1);
+      const float4 n1 = s_nrm[y + 1][sx], n2 = s_nrm[y + 2][sx], n3 = s_nrm[y + 3][sx];
+      if (dx > 0) weights(dx - 1, s_nrm[y][sx], n1);
+      weights(4 + dx, n1, n2);
+      weights(9 + dx, n2, n3);
+    }
+  }
+  __syncthreads();
+  const int tx = threadIdx.x, ty = threadIdx.y * kBilRows;  // the thread's first tap within the tile
+  const int x = blockIdx.x * kTx + tx, y = blockIdx.y * kExTile + ty;
+  if (x >= w || y >= h) return;
+  // Weight of the pixel in halo row py of the thread's column to its tap (dx, dy); to
+  // itself: in its light.
+  auto weight = [&](int py, int dx, int dy) {
+    const int px = tx + 2;
+    if (dy == 0) return dx > 0 ? s_w[dx - 1][py][px] : s_w[-dx - 1][py][px + dx];
+    if (dy > 0) return s_w[5 * dy - 1 + dx][py][px];
+    return s_w[-5 * dy - 1 - dx][py + dy][px + dx];
+  };
+  float sx = 0.0f, sy = 0.0f, sz = 0.0f, sw = 0.0f;
+#pragma unroll
+  for (int dx = 0; dx < 5; dx++) {  // row 0: the upper pixel's alone
+    const float4 col = s_col[ty][tx + dx];
+    const float wt = weight(ty + 2, dx - 2, -2);
+    sx = sx + col.x * wt;
+    sy = sy + col.y * wt;
+    sz = sz + col.z * wt;
+    sw = sw + wt;
+  }
+  p2 ax = pk(sx, 0.0f), ay = pk(sy, 0.0f), az = pk(sz, 0.0f), aw = pk(sw, 0.0f);
+#pragma unroll
+  for (int r = 1; r < 5; r++) {
+#pragma unroll
+    for (int dx = 0; dx < 5; dx++) {
+      const float4 col = s_col[ty + r][tx + dx];
+      const p2 wt = pk(dx == 2 && r == 2 ? col.w : weight(ty + 2, dx - 2, r - 2),
+                       dx == 2 && r == 3 ? col.w : weight(ty + 3, dx - 2, r - 3));
+      ax = padd(ax, pmul(pk(col.x), wt));
+      ay = padd(ay, pmul(pk(col.y), wt));
+      az = padd(az, pmul(pk(col.z), wt));
+      aw = padd(aw, wt);
+    }
+  }
+  float4* o = reinterpret_cast<float4*>(out) + (size_t)y * w + x;
+  store_filtered(o, lo_(ax), lo_(ay), lo_(az), lo_(aw));
+  if (y + 1 >= h) return;
+  sx = hi_(ax);
+  sy = hi_(ay);
+  sz = hi_(az);
+  sw = hi_(aw);
+#pragma unroll
+  for (int dx = 0; dx < 5; dx++) {  // row 5: the lower pixel's
+    const float4 col = s_col[ty + 5][tx + dx];
+    const float wt = weight(ty + 3, dx - 2, 2);
+    sx = sx + col.x * wt;
+    sy = sy + col.y * wt;
+    sz = sz + col.z * wt;
+    sw = sw + wt;
+  }
+  store_filtered(o + w, sx, sy, sz, sw);
 }
 
 // denoiser.frag:72-184 with radius 2: 16 equations [depth, 1] -> colour over
@@ -324,13 +425,15 @@ dim3 grid2d(int w, int h) { return dim3((w + kTx - 1) / kTx, (h + kTy - 1) / kTy
 
 int launch_bilateral(const float* ind, const float* depth, int depth_ch, const float* normal, float* out, int w, int h,
                      cudaStream_t stream, bool fast) {
-  const dim3 grid((w + kTx - 1) / kTx, (h + kTy * kBilRows - 1) / (kTy * kBilRows)), block(kTx, kTy);
+  const int rows = fast ? kTy : kExY;
+  const dim3 grid((w + kTx - 1) / kTx, (h + rows * kBilRows - 1) / (rows * kBilRows)), block(kTx, rows);
+  auto go = [&](auto kernel) { kernel<<<grid, block, 0, stream>>>(ind, depth, normal, out, w, h); };
   if (depth_ch == 2) {
-    if (fast) bilateral_kernel<2, true><<<grid, block, 0, stream>>>(ind, depth, normal, out, w, h);
-    else bilateral_kernel<2, false><<<grid, block, 0, stream>>>(ind, depth, normal, out, w, h);
+    if (fast) go(bilateral_fast_kernel<2>);
+    else go(bilateral_exact_kernel<2>);
   } else {
-    if (fast) bilateral_kernel<1, true><<<grid, block, 0, stream>>>(ind, depth, normal, out, w, h);
-    else bilateral_kernel<1, false><<<grid, block, 0, stream>>>(ind, depth, normal, out, w, h);
+    if (fast) go(bilateral_fast_kernel<1>);
+    else go(bilateral_exact_kernel<1>);
   }
   GI_CHECK_LAUNCH("bilateral_kernel");
   count_launches(1);
