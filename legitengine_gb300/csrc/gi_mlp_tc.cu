@@ -35,11 +35,13 @@
 // takes one hardware barrier of the group, before its MMAs (1920 x 1080: 127.5 -> 124.5
 // us against one waiting thread and a second barrier).
 //
-// Layout of the operands in shared memory: K-major without swizzle.  A core matrix is 8 rows x 16 bytes
-// stored as 128 contiguous bytes; core matrices adjacent along K are 128 bytes
-// apart (the descriptor's leading byte offset) and those adjacent along M (or N)
-// are K*2*8 bytes apart (its stride byte offset).  One MMA consumes K = 16, so a
-// layer of depth K is K/16 MMAs whose descriptors advance by 256 bytes.
+// Layout of the operands in shared memory: core matrices of 8 rows x 16 bytes, stored as
+// 128 contiguous bytes, without swizzle.  Weights are stored as they lie in memory,
+// inputs x outputs, a core matrix 8 inputs by 8 consecutive outputs: K runs along the rows
+// (MN-major), core matrices adjacent along the outputs are 128 bytes apart (the
+// descriptor's stride byte offset) and those adjacent along K outputs * 16 bytes (its
+// leading byte offset), and 16-byte accesses stage them.  The bias operand is K-major.
+// One MMA consumes K = 16.
 #include <cuda_bf16.h>
 
 #include <mutex>
@@ -63,17 +65,16 @@ constexpr uint32_t cA = 64, kGroupCols = cA + kHid / 2, cOnes = kGroupCols * kGr
 static_assert(cOnes + 4 * kOnesCols <= kTmemCols, "tensor memory");
 
 // Shared memory (bytes).  B operands are the weights as N x K (K-major).
-constexpr int kB4Rows = 8;                        // W4 rows 0-7 (3 outputs, zero padding)
-constexpr int tB1 = 0;                            // 64 x 32
+constexpr int tB1 = 0;                            // 32 x 64 (inputs x outputs)
 constexpr int tB2 = tB1 + kHid * kIn * 2;         // 64 x 64
 constexpr int tB3 = tB2 + kHid * kHid * 2;        // 64 x 64
-constexpr int tB4 = tB3 + kHid * kHid * 2;        // 8 x 64; the MMA's rows 8-15 re-read rows 0-7
+constexpr int tB4 = tB3 + kHid * kHid * 2;        // 64 x 16 (outputs 3-15 zero)
 // Biases enter the accumulators through one extra MMA per layer: A = a constant
 // "ones" operand, B = the bias operand.  Bias row n holds, at k = 2L and 2L + 1,
 // the bf16 high and low parts of layer L's bias b_L[n] (b - hi rounded again), so
 // the MMA adds hi + lo, b to about 2^-16 relative.  Layer L's ones operand has
 // 1 at k = 2L, 2L + 1 in every row and 0 elsewhere; k = 8-15 read the bias rows again.
-constexpr int tBB = tB4 + kB4Rows * kHid * 2;     // 64 rows x 8 k (16 bytes a row)
+constexpr int tBB = tB4 + kHid * kOutPad * 2;     // 64 rows x 8 k (16 bytes a row)
 // Staging of a tile's own inputs: normal, albedo, few-ray light, direct light, filtered
 // few-ray light (16 bytes a pixel each) and depth moments (8).
 constexpr int sNormal = 0, sAlbedo = 2048, sLight = 4096, sDirect = 6144, sFiltered = 8192, sMoments = 10240;
@@ -110,10 +111,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator (bits 4-5 = 1), BF16 A
-// (bits 7-9 = 1) and B (bits 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
+// (bits 7-9 = 1) and B (bits 10-12 = 1), N >> 3 at bit 17, M >> 4 at bit 24; K-major
+// operands, or MN-major ones with the flags below.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// K runs along the rows of A's, of B's core matrices.
+constexpr uint32_t kARows = 1u << 15, kBRows = 1u << 16;
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -248,13 +252,14 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-// Copies layer weights W [K x N] (row stride ldw, bf16, global) into the N x K
-// K-major core-matrix layout at smem + off (rows n >= nvalid of W4 are the zero padding).
-__device__ __forceinline__ void stage_b(unsigned char* smem, int off, const bf16* __restrict__ w, int K, int N,
-                                        int ldw) {
-  for (int i = threadIdx.x; i < K * N; i += kTcThreads) {
-    const int k = i / N, n = i % N;
-    *reinterpret_cast<bf16*>(smem + off + cm_off(n, k, K)) = w[k * ldw + n];
+// A K x N weight matrix (bf16, row-major, N columns) as core matrices of 8 rows x 8 columns.
+template <int K, int N, int THREADS>
+__device__ __forceinline__ void stage_weights(uint32_t dst, const bf16* __restrict__ w) {
+#pragma unroll
+  for (int i = threadIdx.x; i < K * N / 8; i += THREADS) {
+    const int k = i / (N / 8), c = i % (N / 8);
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(w) + i);
+    st_shared_v4(dst + cm_off(k, 8 * c, N), q.x, q.y, q.z, q.w);
   }
 }
 
@@ -276,8 +281,6 @@ __device__ __forceinline__ bool group_any(int group, bool v) {
 // group's first thread and waits for them; the fence after the wait orders their
 // completion before the accumulator reads.  `bad` is set on a thread whose wait runs
 // out; returns false (on every thread of the group) if an earlier one did.
-// The B operand's row-group stride is K * 16 bytes, or 0 when its N = 16 rows
-// re-read the first 8 (the output layer).
 // `first` runs on the issuing thread after the barrier, before the MMAs.
 template <int K, int N, int L, typename First>
 __device__ __forceinline__ bool run_layer(uint32_t sbase, uint32_t ones, int b_off, uint32_t tmem, uint32_t bar,
@@ -290,11 +293,10 @@ __device__ __forceinline__ bool run_layer(uint32_t sbase, uint32_t ones, int b_o
   if ((threadIdx.x & (kRows - 1)) == 0) {
     first();
     constexpr uint32_t idesc = idesc_bf16(kRows, N);
-    constexpr uint32_t b_sbo = (N == kOutPad) ? 0u : (uint32_t)(K * 16);
     mma_bf16_ts(tmem, ones + kOnesCols * L, smem_desc(sbase + tBB, 0, 128), idesc, 0u);
 #pragma unroll
     for (int j = 0; j < K / 16; j++)
-      mma_bf16_ts(tmem, tmem + cA + 8 * j, smem_desc(sbase + b_off + j * 256, 128, b_sbo), idesc, 1u);
+      mma_bf16_ts(tmem, tmem + cA + 8 * j, smem_desc(sbase + b_off + j * N * 32, N * 16, 128), idesc | kBRows, 1u);
     mma_commit(bar);
   }
   if (!mbar_wait(bar, phase, limit)) bad = true;
@@ -348,10 +350,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   const uint32_t stage = sbase + tStage + group * kStageBytes;
   const unsigned char* stage_p = smem + tStage + group * kStageBytes;
 
-  stage_b(smem, tB1, wb + qW1, kIn, kHid, kHid);
-  stage_b(smem, tB2, wb + qW2, kHid, kHid, kHid);
-  stage_b(smem, tB3, wb + qW3, kHid, kHid, kHid);
-  stage_b(smem, tB4, wb + qW4, kHid, kB4Rows, kOutPad);
+  stage_weights<kIn, kHid, kTcThreads>(sbase + tB1, wb + qW1);
+  stage_weights<kHid, kHid, kTcThreads>(sbase + tB2, wb + qW2);
+  stage_weights<kHid, kHid, kTcThreads>(sbase + tB3, wb + qW3);
+  stage_weights<kHid, kOutPad, kTcThreads>(sbase + tB4, wb + qW4);
   // Bias operand: row n, k = 2L / 2L + 1 = high / low bf16 part of b_L[n].
   for (int i = tid; i < kHid * 8; i += kTcThreads) {
     const int n = i >> 3, k = i & 7, L = k >> 1;
@@ -601,22 +603,11 @@ template <int W> __device__ __forceinline__ Operand along_rows(uint32_t at) { re
 // K/16 MMAs of A (M = 128 x K) and B (N x K) into D; `first` clears D.
 template <int K, int N>
 __device__ __forceinline__ void mma_chain(uint32_t d, const Operand& a, const Operand& b, bool first) {
-  const uint32_t idesc = idesc_bf16(kRows, N) | (a.rows ? 1u << 15 : 0u) | (b.rows ? 1u << 16 : 0u);
+  const uint32_t idesc = idesc_bf16(kRows, N) | (a.rows ? kARows : 0u) | (b.rows ? kBRows : 0u);
 #pragma unroll
   for (int j = 0; j < K / 16; j++)
     mma_bf16(d, smem_desc(a.at + 2 * j * a.k, a.k, a.mn), smem_desc(b.at + 2 * j * b.k, b.k, b.mn), idesc,
              (first && j == 0) ? 0u : 1u);
-}
-
-// A K x N weight matrix (bf16, row-major, N columns) as core matrices of 8 rows x 8 columns.
-template <int K, int N>
-__device__ __forceinline__ void stage_weights(uint32_t dst, const bf16* __restrict__ w) {
-#pragma unroll
-  for (int i = threadIdx.x; i < K * N / 8; i += kTrThreads) {
-    const int k = i / (N / 8), c = i % (N / 8);
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(w) + i);
-    st_shared_v4(dst + cm_off(k, 8 * c, N), q.x, q.y, q.z, q.w);
-  }
 }
 
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
@@ -653,10 +644,10 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   volatile int* fail = reinterpret_cast<volatile int*>(smem + uFail);
   const float* bias = reinterpret_cast<const float*>(smem + uBias);
 
-  stage_weights<kIn, kHid>(sbase + uW1, wb + qW1);
-  stage_weights<kHid, kHid>(sbase + uW2, wb + qW2);
-  stage_weights<kHid, kHid>(sbase + uW3, wb + qW3);
-  stage_weights<kHid, kOutPad>(sbase + uW4, wb + qW4);
+  stage_weights<kIn, kHid, kTrThreads>(sbase + uW1, wb + qW1);
+  stage_weights<kHid, kHid, kTrThreads>(sbase + uW2, wb + qW2);
+  stage_weights<kHid, kHid, kTrThreads>(sbase + uW3, wb + qW3);
+  stage_weights<kHid, kOutPad, kTrThreads>(sbase + uW4, wb + qW4);
   if (tid < 3 * kHid + kOut) {
     const int l = tid >> 6, at = tid & (kHid - 1);
     const int from = (l == 0 ? ob1 : l == 1 ? ob2 : l == 2 ? ob3 : ob4) + at;
