@@ -1,4 +1,4 @@
-"""The bilateral filter where its tiles and its exponential can go wrong, against the
+"""The bilateral filter (and the final gather) where its tiles and its exponential can go wrong, against the
 fp32 oracle bit for bit (the same operations in the same order): images smaller than a
 tile, one row or column past it, odd heights (a thread filters two rows), and depths and
 normals whose weights reach every part of the exponential's range: 1, subnormal, 0, and
@@ -28,3 +28,14 @@ def test_bilateral_equals_the_oracle(gi, oracle, cuda, w, h, kind):
     gi.bilateral(dev(light), dev(moments), dev(normal), out)
     cuda.cuda.synchronize()
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.bilateral(light, moments, normal))
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (5, 3), (2, 9), (32, 16), (33, 17), (31, 15), (70, 34)])
+def test_final_gather_equals_the_oracle(gi, oracle, cuda, w, h):
+    r = np.random.default_rng(w * 100 + h)
+    direct, light, albedo = (r.uniform(-0.1, 2.0, (h, w, 4)).astype(np.float32) for _ in range(3))
+    dev = lambda a: cuda.from_numpy(a).cuda()
+    out = cuda.full((h, w, 4), -7.0, dtype=cuda.float32, device="cuda")
+    gi.final_gather(dev(direct), dev(light), dev(albedo), out)
+    cuda.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), oracle.final_gather(direct, light, albedo))
