@@ -23,6 +23,7 @@
 #include "gi_device.cuh"
 #include "gi_internal.h"
 #include "gi_kernels.h"
+#include "gi_record.h"
 
 namespace gi {
 namespace {
@@ -249,12 +250,6 @@ template <bool TEX> __device__ __forceinline__ MarchSmem<TEX> march_smem(unsigne
   return m;
 }
 
-// Pixels of a march record: every (pattern, sub-image pixel) slot, P^2 ceil(W/P) ceil(H/P).
-__host__ __device__ __forceinline__ size_t record_pixels(const MarchArgs& a) {
-  const size_t P = (size_t)a.pattern;
-  return P * P * (((size_t)a.width + P - 1) / P) * (((size_t)a.height + P - 1) / P);
-}
-
 // The light term of a hit (:254-264): the trilinear light tap at the step's
 // footprint (img0, img1: the light pyramid's two levels), then dl += (light -
 // ambient) * hc, in the order of the restatement (exact) or as fused multiply-adds
@@ -468,7 +463,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
 
   // Records are indexed in the interleaved (pattern, sub-image row, column) order,
   // in which a warp's 32 pixels are consecutive: coalesced stores and loads.
-  const unsigned npix = (unsigned)record_pixels(a);
+  const unsigned npix = (unsigned)record_pixels(a.width, a.height, a.pattern);
   const unsigned rec_idx = ((unsigned)pat * ((a.height + P - 1) / P) + j) * ((a.width + P - 1) / P) + i;
   Light sum{pk(0.0f), 0.0f};
   for (int d = SPLIT > 1 ? (int)threadIdx.y : 0; d < R; d += SPLIT) {
@@ -477,7 +472,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
     // warp, which step together, write and read neighbouring words of one row.  The
     // record is written and read once, larger than L2: streaming (evict-first) stores
     // and loads keep the pyramids the taps read resident in L2 (0.4 % of the frame).
-    float* const rec_rows = REC ? a.rec_hc + (size_t)d * a.rec_steps * npix + rec_idx : nullptr;
+    float* const rec_rows = REC ? a.rec_hc + record_block(d, a.rec_steps, npix) + rec_idx : nullptr;
     const float4 dir4 = s_dir[d];
     const p2 dir = pk(dir4.x, dir4.y);
     // Texture taps: the first step's depth, fetched before the direction's frame.
@@ -585,7 +580,7 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
       return hc;
     };
     auto record = [&](int s, float hc) {
-      if (SPLIT == 1 || inside) __stcs(rec_rows + (size_t)((unsigned)s * npix), hc);
+      if (SPLIT == 1 || inside) __stcs(rec_rows + record_row(s, npix), hc);
       hits |= 1ull << s;
     };
     if constexpr (TEX) {
@@ -708,7 +703,7 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
   const p2 rWH = pk(a.inv_size[0], a.inv_size[1]);
   const p2 centre = pk((float)px + 0.5f, (float)py + 0.5f);
   const size_t out_idx = (size_t)py * a.width + px;
-  const unsigned npix = (unsigned)record_pixels(a);
+  const unsigned npix = (unsigned)record_pixels(a.width, a.height, a.pattern);
   const unsigned rec_idx = ((unsigned)pat * ((a.height + P - 1) / P) + j) * ((a.width + P - 1) / P) + i;
   const float ambient = 0.01f;
   const float rR = rcp_((float)R);
@@ -720,7 +715,7 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
     const float hc0 = __ldcs(a.rec_hc0 + (size_t)d * npix + rec_idx);
     // Bits index the 64-entry table (ReplaySmem): in bounds whatever the mask holds.
     const unsigned long long hits = __ldcs(a.rec_mask + (size_t)d * npix + rec_idx);
-    const float* const rec_rows = a.rec_hc + (size_t)d * a.rec_steps * npix + rec_idx;
+    const float* const rec_rows = a.rec_hc + record_block(d, a.rec_steps, npix) + rec_idx;
     Light dl{pk(ambient * hc0), ambient * hc0};
     // The steps that any lane hit, in order, the lanes together: a step's lanes read
     // neighbouring texels of the same levels.  Bound by L1's data pipe (70 % busy; 90 %
@@ -734,7 +729,7 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
       if (!(hits >> s & 1ull)) continue;
       const TapStep& e = sm.step[s];
       const p2 sp = pmul(padd(centre, pmul(dir, pk(e.off))), rWH);
-      const float hc = __ldcs(rec_rows + (size_t)((unsigned)s * npix));
+      const float hc = __ldcs(rec_rows + record_row(s, npix));
       const bool two = e.delta != 0.0f;
       TapFoot foot;
       if (two) tap_foot2(e, lo_(sp), hi_(sp), foot);
@@ -1302,7 +1297,7 @@ int launch_march(const MarchArgs& a, cudaStream_t stream) {
       return fail(GI_ERR_INVALID_ARGUMENT, "march: a record needs the standard form and its arrays");
     if (march_table_size(a) > a.rec_steps || a.rec_steps > 64)
       return fail(GI_ERR_INVALID_ARGUMENT, "march: record step stride");
-    if (record_pixels(a) >= (1ull << 31) || (size_t)a.dirs * a.rec_steps >= (1ull << 31))
+    if (record_pixels(a.width, a.height, a.pattern) >= (1ull << 31) || (size_t)a.dirs * a.rec_steps >= (1ull << 31))
       return fail(GI_ERR_UNSUPPORTED, "march: record too large for 32-bit indices");
   }
   const TunedLayout t = tuned_layout(a);
@@ -1312,7 +1307,7 @@ int launch_march(const MarchArgs& a, cudaStream_t stream) {
 size_t march_record_bytes(const MarchArgs& a, size_t* hc_bytes, size_t* mask_bytes, size_t* hc0_bytes) {
   const int n_tab = march_table_size(a);
   if (n_tab > 64) return 0;
-  const size_t npix = record_pixels(a), R = (size_t)a.dirs;
+  const size_t npix = record_pixels(a.width, a.height, a.pattern), R = (size_t)a.dirs;
   *hc_bytes = R * (size_t)n_tab * npix * sizeof(float);
   *mask_bytes = R * npix * sizeof(unsigned long long);
   *hc0_bytes = R * npix * sizeof(float);
