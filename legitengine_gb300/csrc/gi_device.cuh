@@ -187,7 +187,10 @@ __device__ __forceinline__ f3 funproject(const Mat4& inv, float sx, float sy, fl
   return mk3(v.x * r, v.y * r, v.z * r);
 }
 // The hardware's approximate division and reciprocal square root without the
-// scaling that subnormal operands would need.
+// scaling that subnormal operands would need: those count as 0.  In the step loop that
+// is a sample within 1e-19 of the pixel's point (its |h|^2) or a view ray as short; with
+// the scaling, whose quotients overflow there in part, frames took 2 to 3 % longer
+// (1283 x 721, R = 12: 1110 against 1139 us).
 __device__ __forceinline__ float div_approx(float a, float b) {
   float r;
   asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
@@ -202,9 +205,12 @@ __device__ __forceinline__ float rsqrt_approx(float a) {
 // atan(t) = t P(t^2), P of degree 8 fitted to atan(t)/t by iteratively reweighted
 // least squares on 6000 Chebyshev nodes of [0, 1] (max error 9.4e-8 rad in fp32,
 // about one ulp of the result; the quotient's approximate division adds ~2 ulp).
+// (0, 0) and two NaNs (a sample of NaN depth) give 0 with y's sign, as the fast
+// precisions always have; the exact precision's angle of two NaNs is NaN, no hit.
 __device__ __forceinline__ float fast_atan2(float y, float x) {
   const float ax = fabsf(x), ay = fabsf(y);
-  const float mx = fmaxf(fmaxf(ax, ay), 1e-37f), mn = fminf(ax, ay);  // (0, 0): t = 0
+  const float mx = fmaxf(fmaxf(ax, ay), 1e-37f);
+  const float mn = fmaxf(fminf(ax, ay), 0.0f);
   const float t = div_approx(mn, mx);
   const float z = t * t;
   float p = 0.0024567246437072754f;
