@@ -243,24 +243,6 @@ __device__ __forceinline__ void lin_setup(float s, int w, int& i0, int& i1, floa
   lin_setup_f(s, (float)w, w, i0, i1, a);
 }
 
-// atan2f_ (gi_math.h), the same bits, with its octant reduction as selects and its
-// special cases (both arguments infinite, or NaN) in one cold branch.
-__device__ __forceinline__ float march_atan2(float y, float x) {
-  const float ax = fabsf(x), ay = fabsf(y);
-  const float num = fminf(ax, ay), den = fmaxf(ax, ay);
-  if (!(num < kInf)) return atan2f_(y, x);
-  float t = den == 0.0f ? 0.0f : num * rcp_(den);
-  float base = 0.0f;
-  if (t > kTanPiO12) {
-    t = div_(t * kSqrt3 - 1.0f, t + kSqrt3);
-    base = kPiO6;
-  }
-  float a = base + atan_core(t);
-  if (ay > ax) a = kPiO2 - a;
-  if (signbit_(x)) a = kPi - a;
-  return copysign_(a, y);
-}
-
 struct Bilin {
   int o00, o10, o01, o11;  // texel indices (y * w + x)
   float w00, w10, w01, w11;

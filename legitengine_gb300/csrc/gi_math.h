@@ -236,6 +236,35 @@ GI_HD float atan2f_(float y, float x) {
   return copysign_(a, y);
 }
 
+// The smaller of two values; NaN if either is.
+GI_HD float min_nan_(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+#else
+  return a != a || b != b ? u2f(0x7fc00000u) : fminf(a, b);
+#endif
+}
+
+// atan2f_, the same bits, with its octant reduction as selects and its special cases
+// (both arguments infinite, or either NaN) in one cold branch.
+GI_HD float march_atan2(float y, float x) {
+  const float ax = fabsf(x), ay = fabsf(y);
+  const float num = min_nan_(ax, ay), den = fmaxf(ax, ay);
+  if (!(num < kInf)) return atan2f_(y, x);
+  float t = den == 0.0f ? 0.0f : num * rcp_(den);
+  float base = 0.0f;
+  if (t > kTanPiO12) {
+    t = div_(t * kSqrt3 - 1.0f, t + kSqrt3);
+    base = kPiO6;
+  }
+  float a = base + atan_core(t);
+  if (ay > ax) a = kPiO2 - a;
+  if (signbit_(x)) a = kPi - a;
+  return copysign_(a, y);
+}
+
 GI_HD void sincos_core(float r, float* s, float* c) {
   float z = r * r;
   float ps = fma_(z, 1.0f / 362880.0f, -1.0f / 5040.0f);
