@@ -187,10 +187,15 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                : "memory");
 }
 
+// The .sync.aligned instructions below are executed by a whole warp together.  A warp
+// that waited lane by lane (mbar_wait) or left one lane's branch need not have come
+// together again, so each has a __syncwarp directly before it.
+
 // 16 consecutive FP32 columns of this thread's accumulator lane; the load and
 // its completion wait are one asm statement, so no use can be scheduled between.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;\n"
@@ -205,6 +210,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // 32 consecutive FP32 columns of this thread's accumulator lane (one load, one wait).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
       "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
@@ -222,11 +228,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // 32-bit columns of this thread's lane written to tensor memory; tmem_st_wait before the
 // barrier that precedes the MMA that reads them.
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  __syncwarp();
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(r[0]),
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
           taddr),
@@ -234,7 +242,25 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st_wait() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// `cols` columns of tensor memory for this CTA, by one warp: their start is stored at
+// `slot` (shared memory); the CTA allocates once.
+__device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n\t"
+      "tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::"r"(slot),
+      "r"(cols)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t start, uint32_t cols) {
+  __syncwarp();
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(start), "r"(cols) : "memory");
+}
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   const bf16 x = __float2bfloat16_rn(a), y = __float2bfloat16_rn(b);
@@ -301,7 +327,6 @@ __device__ __forceinline__ bool run_layer(uint32_t sbase, uint32_t ones, int b_o
   }
   if (!mbar_wait(bar, phase, limit)) bad = true;
   phase ^= 1u;
-  __syncwarp();  // the warp's accumulator loads are one instruction for all its lanes
   fence_after();
   return true;
 }
@@ -372,12 +397,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
     mbar_init(bar, 1);
     mbar_init(sbar, 1);
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + tTmem),
-                 "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 0) tmem_alloc(sbase + tTmem, kTmemCols);
   fence_async_smem();  // the staged operands, for the tensor cores
   fence_before();
   __syncthreads();
@@ -469,7 +489,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
       uint32_t r[kIn / 2];
 #pragma unroll
       for (int k = 0; k < kIn / 2; k++) r[k] = pack_bf16(f[2 * k], f[2 * k + 1]);
-      __syncwarp();
       tmem_st16(lane_addr + cA, r);
     }
     // The head blends candidate estimates as the network saw them (bf16).
@@ -520,10 +539,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_reconstruct_kernel(const __
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(kTmemCols)
-                 : "memory");
+  if (warp == 0) tmem_free(tmem_base, kTmemCols);
 }
 
 // ---- Training on the tensor cores -----------------------------------------
@@ -659,12 +675,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
     mbar_init(grad_bar, 1);
     *fail = 0;
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + uTmem),
-                 "r"(kTrTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 0) tmem_alloc(sbase + uTmem, kTrTmemCols);
   fence_before();
   __syncthreads();
   fence_after();
@@ -868,8 +879,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTrTmemCols) : "memory");
+  if (warp == 0) tmem_free(tmem, kTrTmemCols);
 }
 
 std::mutex g_tc_mutex;
