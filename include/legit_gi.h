@@ -455,11 +455,13 @@ GI_API int gi_mlp_set_loss(gi_mlp* m, int loss);
  * against targets [n x 4]: rgb t_i (divided by scale[i] when scale, device [n],
  * is given) and the pixel's loss weight w_i in channel 3 (a march output carries
  * 1 there).  loss_out (host, optional) receives the batch loss and makes the call
- * synchronous. */
+ * synchronous.  A batch in which a tensor-core wait ran out changes nothing; it is
+ * counted (gi_mlp_tensor_core_errors) and, with loss_out, returns GI_ERR_TIMEOUT. */
 GI_API int gi_mlp_train_step(gi_mlp* m, const void* features, const float* targets, const float* scale, int n,
                              float lr, float* loss_out, void* stream);
 /* Gradient of the batch loss of gi_mlp_train_step with respect to the FP32 parameters (same order as
- * gi_mlp_set_params) into grads_host, without updating; synchronous. */
+ * gi_mlp_set_params) into grads_host, without updating; synchronous.  A tensor-core wait that
+ * runs out is counted and returns GI_ERR_TIMEOUT, with nothing written. */
 GI_API int gi_mlp_gradients(gi_mlp* m, const void* features, const float* targets, const float* scale, int n,
                             float* grads_host, float* loss_host, void* stream);
 /* Allocation-free gradients (this entry point has no counterpart in the
@@ -508,15 +510,16 @@ GI_API int gi_mlp_reconstruct(const gi_mlp* m, int width, int height, int patter
                               const float* depth_moments, const float* normal, const float* albedo,
                               const float* direct, const float* const* indirect_levels, const float* filtered,
                               const float* depth_blur_l2, float* out, void* stream);
-/* Count of tensor-core completion waits in gi_mlp_reconstruct that ran out (each
- * abandons its launch's remaining tiles); 0 in normal operation. */
+/* Count of the tile groups of gi_mlp_reconstruct and gi_mlp_forward and of the CTAs of
+ * gi_mlp_train_step and gi_mlp_gradients that gave up after a tensor-core completion wait
+ * ran out (each abandons its remaining tiles); 0 in normal operation. */
 GI_API int gi_mlp_tensor_core_errors(int* count);
 /* Test hook of the failure path above (no counterpart in the reference):
  * bounds the FIRST tensor-core completion wait of each 128-pixel tile group in
- * later gi_mlp_reconstruct launches to `cycles` SM clock cycles, so that a short
- * bound makes the wait run out: the group records an error
- * (gi_mlp_tensor_core_errors), stops, waits with the full bound for its MMAs in
- * flight, frees its tensor memory and the launch returns.  cycles <= 0 restores
+ * later gi_mlp_reconstruct launches, and of each CTA of training launches, to `cycles`
+ * SM clock cycles, so that a short bound makes the wait run out: the group (the CTA, at
+ * its tile's end) records an error (gi_mlp_tensor_core_errors), stops, waits with the
+ * full bound for its MMAs in flight, frees its tensor memory and the launch returns.  cycles <= 0 restores
  * the default (about 2^31 cycles).  For the current device. */
 GI_API int gi_debug_tensor_core_wait_limit(long long cycles);
 /* 4-channel pixels of listed march tiles, image <-> tile-major arrays. */

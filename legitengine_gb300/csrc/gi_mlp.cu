@@ -232,9 +232,9 @@ __device__ __forceinline__ void relu_backward(const float* dH, const bf16* H, bf
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, bf16* __restrict__ wb, float inv_batch, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
+                            float b2, float eps, float c1, float c2, const int* __restrict__ failed_ctas) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
+  if (i >= kParams || *failed_ctas) return;  // sums of a failed batch are not a gradient
   float gi_ = g[i] * inv_batch;
   if (!isfinite(gi_)) gi_ = 0.0f;  // a non-finite gradient element counts as zero
   const float mi = b1 * m[i] + (1.0f - b1) * gi_;
@@ -595,7 +595,9 @@ int launch_judge(float* learned, const float* plain, int W, int H, int P, const 
 
 struct Mlp {
   float* params = nullptr;
-  float* grads = nullptr;  // gradient sums of a batch, then its loss sum: cleared and read back as one
+  // Gradient sums of a batch, its loss sum and its failed CTAs (an int): cleared and read
+  // back as one.
+  float* grads = nullptr;
   float* m = nullptr;
   float* v = nullptr;
   bf16* wb = nullptr;
@@ -609,8 +611,16 @@ struct Mlp {
     dfree(wb);
   }
   float* loss() const { return grads + kParams; }
-  static constexpr size_t kSumBytes = (kParams + 1) * sizeof(float);
+  int* failed_ctas() const { return reinterpret_cast<int*>(grads + kParams + 1); }
+  static constexpr size_t kSumBytes = (kParams + 2) * sizeof(float);
 };
+
+// GI_OK, or GI_ERR_TIMEOUT where the failed CTAs of a batch (Mlp::failed_ctas, read back) are not 0.
+static int check_batch(const float* failed_ctas, const char* what) {
+  int n;
+  memcpy(&n, failed_ctas, sizeof(n));
+  return n == 0 ? GI_OK : fail(GI_ERR_TIMEOUT, std::string(what) + ": a tensor-core wait ran out");
+}
 
 // gi_mlp_forward: the fused reconstruction kernel on given feature rows (tcgen05).
 int mlp_forward(const Mlp* m, const void* feats, const float* scale, int n, float* out, cudaStream_t s) {
@@ -703,22 +713,27 @@ extern "C" int gi_mlp_train_step(gi_mlp* m, const void* features, const float* t
   Mlp& M = m->impl;
   int e = check_cuda(cudaMemsetAsync(M.grads, 0, Mlp::kSumBytes, s), "gi_mlp_train_step");
   e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss(),
-                              M.loss_kind, s);
+                              M.failed_ctas(), M.loss_kind, s);
   if (e) return e;
   M.step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f - (float)std::pow((double)b1, M.step), c2 = 1.0f - (float)std::pow((double)b2, M.step);
   adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(M.params, M.grads, M.m, M.v, M.wb, 1.0f / (float)n, lr, b1, b2,
-                                                    1e-8f, c1, c2);
+                                                    1e-8f, c1, c2, M.failed_ctas());
   GI_CHECK_LAUNCH("adam_kernel");
   count_launches(1);
   if (loss_out) {
-    float l = 0.0f;
-    e = check_cuda(cudaMemcpyAsync(&l, M.loss(), 4, cudaMemcpyDeviceToHost, s), "gi_mlp_train_step: loss");
+    float l[2] = {0.0f, 0.0f};  // the loss sum and the failed CTAs
+    e = check_cuda(cudaMemcpyAsync(l, M.loss(), sizeof(l), cudaMemcpyDeviceToHost, s), "gi_mlp_train_step: loss");
     if (e) return e;
     e = check_cuda(cudaStreamSynchronize(s), "gi_mlp_train_step: sync");
     if (e) return e;
-    *loss_out = l / (float)(n * kOut);
+    e = check_batch(&l[1], "gi_mlp_train_step");
+    if (e) {
+      M.step--;  // adam_kernel did nothing
+      return e;
+    }
+    *loss_out = l[0] / (float)(n * kOut);
   }
   return GI_OK;
 }
@@ -738,11 +753,13 @@ extern "C" int gi_mlp_gradients(gi_mlp* m, const void* features, const float* ta
   Mlp& M = m->impl;
   int e = check_cuda(cudaMemsetAsync(M.grads, 0, Mlp::kSumBytes, s), "gi_mlp_gradients");
   e = e ? e : launch_train_tc(static_cast<const bf16*>(features), targets, scale, n, M.wb, M.params, M.grads, M.loss(),
-                              M.loss_kind, s);
+                              M.failed_ctas(), M.loss_kind, s);
   if (e) return e;
-  std::vector<float> g(kParams + 1);
+  std::vector<float> g(kParams + 2);
   e = check_cuda(cudaMemcpyAsync(g.data(), M.grads, Mlp::kSumBytes, cudaMemcpyDeviceToHost, s), "gi_mlp_gradients");
   e = e ? e : check_cuda(cudaStreamSynchronize(s), "gi_mlp_gradients");
+  if (e) return e;
+  e = check_batch(&g[kParams + 1], "gi_mlp_gradients");
   if (e) return e;
   for (int i = 0; i < kParams; i++) grads_host[i] = g[i] / (float)n;
   if (loss_host) *loss_host = g[kParams] / (float)(n * kOut);

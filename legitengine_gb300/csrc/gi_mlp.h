@@ -40,15 +40,16 @@ int launch_forward_tc(const __nv_bfloat16* rows, const float* scale, int n, cons
                       const float* params, float* out, cudaStream_t stream);
 // One training batch on the tensor cores (tcgen05): the forward with saved
 // activations, the loss gradient and the backward of every tile of 128 pixels,
-// gradient sums added to `grads` and the summed loss to `loss` (both FP32, the
-// caller zeroes them).  feats: bf16 [n x 32]; targets [n x 4] (rgb, loss weight);
+// gradient sums added to `grads` and the summed loss to `loss` (both FP32), and to
+// `failed_ctas` the CTAs a wait of which ran out, whose sums are left out (the caller
+// zeroes all three).  feats: bf16 [n x 32]; targets [n x 4] (rgb, loss weight);
 // scale: optional [n] exposure scale the rgb targets are divided by.
 int launch_train_tc(const __nv_bfloat16* feats, const float* targets, const float* scale, int n,
-                    const __nv_bfloat16* wb, const float* params, float* grads, float* loss, int loss_kind,
-                    cudaStream_t stream);
+                    const __nv_bfloat16* wb, const float* params, float* grads, float* loss, int* failed_ctas,
+                    int loss_kind, cudaStream_t stream);
 // Number of tensor-core waits that ran out since the library was loaded.
 int reconstruct_errors(int* count);
-// Bound in SM cycles of each tile group's first MMA wait (<= 0: the default).
+// Bound in SM cycles of each tile group's (training: each CTA's) first MMA wait (<= 0: the default).
 int reconstruct_wait_limit(long long cycles);
 int launch_tiles_copy(const float* src, float* dst, int W, int H, int P, const int* tiles, int num_tiles,
                       bool scatter, cudaStream_t stream);

@@ -89,8 +89,8 @@ static_assert(tBB % 128 == 0 && tBar % 8 == 0, "alignment");
 
 __device__ int g_tc_errors;  // waits that ran out (kept across launches)
 constexpr long long kWaitCycles = 1ll << 31;  // ~1 s of SM clocks
-// Bound of each tile group's first MMA-completion wait in a launch; kWaitCycles
-// unless the test hook gi_debug_tensor_core_wait_limit shortened it (so that the
+// Bound of the first MMA-completion wait of each tile group (training: of each CTA) in a
+// launch; kWaitCycles unless the test hook gi_debug_tensor_core_wait_limit shortened it (so that the
 // wait runs out and the error path runs).  Every other wait keeps kWaitCycles.
 __device__ long long g_tc_first_wait_cycles = kWaitCycles;
 
@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
                                                                    const bf16* __restrict__ wb,
                                                                    const float* __restrict__ params,
                                                                    float* __restrict__ grads,
-                                                                   float* __restrict__ loss, int loss_kind) {
+                                                                   float* __restrict__ loss, int* __restrict__ failed_ctas,
+                                                                   int loss_kind) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -659,6 +660,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   const uint32_t layer_bar = sbase + uBar, grad_bar = layer_bar + 8;
   volatile int* fail = reinterpret_cast<volatile int*>(smem + uFail);
   const float* bias = reinterpret_cast<const float*>(smem + uBias);
+  const long long first_limit = g_tc_first_wait_cycles;
 
   stage_weights<kIn, kHid, kTrThreads>(sbase + uW1, wb + qW1);
   stage_weights<kHid, kHid, kTrThreads>(sbase + uW2, wb + qW2);
@@ -689,13 +691,13 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
   // A bounded wait of every thread.  One that runs out is recorded and the tile goes on
   // (with values that are not used), so that the threads stay together; the later
   // waits then return at once.
-  auto wait = [&](uint32_t bar, uint32_t& phase) {
-    if (!*fail && !mbar_wait(bar, phase)) *fail = 1;
+  auto wait = [&](uint32_t bar, uint32_t& phase, long long limit = kWaitCycles) {
+    if (!*fail && !mbar_wait(bar, phase, limit)) *fail = 1;
     phase ^= 1u;
   };
   // Shared-memory writes -> the tensor cores -> `layer` (the layer's accumulator) and
   // `grad` (left running) on thread 0 -> wait for the accumulator.
-  auto mma_round = [&](auto layer, auto grad) {
+  auto mma_round = [&](auto layer, auto grad, long long limit = kWaitCycles) {
     fence_async_smem();
     fence_before();
     __syncthreads();
@@ -705,7 +707,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
       mma_commit(layer_bar);
       grad();
     }
-    wait(layer_bar, layer_phase);
+    wait(layer_bar, layer_phase, limit);
     fence_after();
   };
   auto nothing = [] {};
@@ -770,7 +772,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
       st_shared_v4(sbase + uX + cm_off(row, 16 * half + 8 * c, kIn), x[c].x, x[c].y, x[c].z, x[c].w);
 
     mma_round([&] { mma_chain<kIn, kHid>(tmem + cZ, along_columns<kIn>(sbase + uX), along_rows<kHid>(sbase + uW1), true); },
-              nothing);
+              nothing, first ? first_limit : kWaitCycles);
     forward_epilogue(uH1, bias);
     mma_round([&] { mma_chain<kHid, kHid>(tmem + cZ, along_columns<kHid>(sbase + uH1), along_rows<kHid>(sbase + uW2), true); },
               nothing);
@@ -839,12 +841,18 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(const bf16*
     first = false;
     if (stop) break;
   }
-  if (!first && !mbar_wait(grad_bar, grad_phase)) *fail = 1;  // every product in flight, bounded
+  // Every product in flight, bounded: a tile's commit covers all before it.  After a wait
+  // that ran out the previous tile's may still be open, and is waited for first.
+  if (!first && *fail) (void)mbar_wait(grad_bar, grad_phase ^ 1u);
+  if (!first && !mbar_wait(grad_bar, grad_phase)) *fail = 1;
   fence_before();
   __syncthreads();
   fence_after();
   const bool failed = *fail != 0;
-  if (failed && tid == 0) atomicAdd(&g_tc_errors, 1);
+  if (failed && tid == 0) {  // its sums are left out: the batch is reported as failed
+    atomicAdd(&g_tc_errors, 1);
+    atomicAdd(failed_ctas, 1);
+  }
   if (!failed && !first) {
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if (half == 0 && (tid & 31) == 0) atomicAdd(loss, lsum);
@@ -958,8 +966,8 @@ int launch_forward_tc(const __nv_bfloat16* rows, const float* scale, int n, cons
 }
 
 int launch_train_tc(const __nv_bfloat16* feats, const float* targets, const float* scale, int n,
-                    const __nv_bfloat16* wb, const float* params, float* grads, float* loss, int loss_kind,
-                    cudaStream_t stream) {
+                    const __nv_bfloat16* wb, const float* params, float* grads, float* loss, int* failed_ctas,
+                    int loss_kind, cudaStream_t stream) {
   int dev = 0;
   int e = check_cuda(cudaGetDevice(&dev), "train: device");
   if (e) return e;
@@ -984,7 +992,7 @@ int launch_train_tc(const __nv_bfloat16* feats, const float* targets, const floa
   const int grid = tiles < sms ? tiles : sms;  // one CTA per SM: all 512 tensor-memory columns
   if (grid <= 0) return GI_OK;
   mlp_train_tc_kernel<<<grid, kTrThreads, kSmemTrainTc, stream>>>(feats, targets, scale, n, wb, params, grads,
-                                                                   loss, loss_kind);
+                                                                   loss, failed_ctas, loss_kind);
   GI_CHECK_LAUNCH("mlp_train_tc_kernel");
   count_launches(1);
   return GI_OK;
