@@ -104,7 +104,7 @@ __device__ void cast_mesh(const MeshSet& m, f3 o, f3 d, const float (&iv)[3], Hi
 // |origin - centre|^2 - r^2.  Two 16-byte reads.
 struct __align__(16) PrimTest {
   float a[3];
-  int kind;  // gi_prim_kind, | kFinite
+  int kind;  // gi_prim_kind, | kFinite; -1: no kind that a ray meets
   float b[3];
   float pad;
 };
@@ -115,7 +115,7 @@ __device__ __forceinline__ bool finite(float v) { return v - v == 0.0f; }
 __device__ __forceinline__ PrimTest prim_test(const gi_prim& p, f3 o) {
   PrimTest r;
   const float ov[3] = {o.x, o.y, o.z};
-  r.kind = p.kind;
+  r.kind = p.kind == GI_PRIM_ROOM || p.kind == GI_PRIM_BOX || p.kind == GI_PRIM_SPHERE ? p.kind : -1;
   if (p.kind == GI_PRIM_SPHERE) {
     const f3 oc = sub3(o, mk3(p.a[0], p.a[1], p.a[2]));
     r.a[0] = oc.x;
