@@ -23,6 +23,7 @@
 #include "gi_device.cuh"
 #include "gi_internal.h"
 #include "gi_kernels.h"
+#include "gi_march_split.h"
 #include "gi_record.h"
 
 namespace gi {
@@ -32,8 +33,7 @@ using namespace dev;
 
 constexpr int kMarchTx = kMarchTileSubX;  // sub-image pixels per warp row
 constexpr int kMarchTy = kMarchTileSubY;  // warps per CTA
-constexpr int kSplit = 4;               // direction split: threads per pixel
-constexpr int kSplitMaxDirs = 32;
+constexpr int kSplitMaxDirs = 32;  // direction split (kSplit threads per pixel)
 constexpr int kSplitMinDirs = 4;
 constexpr float kPiRef = 3.1415f;  // indirectLighting.frag:169
 
@@ -1066,18 +1066,7 @@ static bool split_fits(const MarchArgs& a) {
   return !a.deinterleaved && a.depth_ch == 2 && !a.soft && a.dirs >= kSplitMinDirs && a.dirs <= kSplitMaxDirs;
 }
 
-// Whether an untuned frame takes the direction split: four times the threads, each
-// with the pixel's set-up and ceil(R / 4) = n of its directions.  It pays while the
-// one-thread form is too few waves of CTAs (8 an SM) to fill the GPU and hide its
-// latency, and up to more waves the more directions share the set-up and the more
-// evenly they divide.  The line, (1.5 n - 1) waves times the share of the last round of
-// directions that is used, follows a sweep of 200 x 120 to 1920 x 1080 with 4, 5, 8
-// and 16 directions; one-thread form against split, exact march and two-bounce exact
-// frame, in us: R = 8 at 256 x 144 (0.24 waves) 126 / 65 and 203 / 119, at 512 x 512
-// (1.7) 319 / 298 and 511 / 475, at 700 x 500 (2.4) 413 / 413 and 643 / 638, at
-// 1920 x 1080 (13) 1878 / 2046 and 2837 / 3136; R = 16 at 960 x 540 (3.3) 1632 / 1587,
-// at 1280 x 720 (5.9) 2683 / 2648; R = 4 at 320 x 240 (0.6) 66 / 60, at 400 x 300 (1)
-// 79 / 85; R = 5 at 256 x 144 72 / 48, at 320 x 240 84 / 87.
+// Whether an untuned frame takes the direction split (gi_march_split.h).
 static bool split_pays(const MarchArgs& a) {
   if (!split_fits(a)) return false;
   int dev = 0, sms = 0;
@@ -1086,9 +1075,9 @@ static bool split_pays(const MarchArgs& a) {
     (void)cudaGetLastError();
     return false;
   }
-  const int n = (a.dirs + kSplit - 1) / kSplit;
-  const float waves = (float)a.width * (float)a.height / (1024.0f * (float)sms);  // 1024 resident threads an SM
-  return waves < (1.5f * (float)n - 1.0f) * (float)(a.dirs - kSplit * (n - 1)) / (float)kSplit;
+  const int P = a.pattern, sub_w = (a.width + P - 1) / P, sub_h = (a.height + P - 1) / P;
+  const int tiles = ((sub_w + kMarchTx - 1) / kMarchTx) * ((sub_h + kMarchTy - 1) / kMarchTy) * P * P;
+  return split_pays(a.width, a.height, a.dirs, tiles, sms);
 }
 
 // Untuned shapes that do not split: 4 rows (two-bounce texture frame at 1920x1080,
