@@ -4,6 +4,8 @@
 // procedural primitives (boxes and spheres inside a room) that the bounds of a warp's
 // rays meet, then the triangle meshes of a loaded scene, object by object behind a
 // bounds test.
+#include <type_traits>
+
 #include "gi_device.cuh"
 #include "gi_internal.h"
 #include "gi_kernels.h"
@@ -14,9 +16,16 @@ namespace {
 using namespace dev;
 
 constexpr int kTx = 32, kTy = 4;          // direct light: one row of 32 pixels a warp
-constexpr int kCastPix = 2;               // ray casts: pixels a thread, 4 rows apart
-constexpr int kCastX = 32, kCastY = 8 * kCastPix;  // tile of a CTA, in warps of 8 x (4 kCastPix) pixels
-constexpr int kCastThreads = kCastX * kCastY / kCastPix;
+// Ray casts: a CTA's pixels, in warps of 8 x (4 kPixels).  Without meshes a thread takes
+// two pixels, 4 rows apart, which share the bounds of their warp's primitives.  The triangle
+// loops share nothing and would run one after the other, so with meshes it takes one, and a
+// CTA fewer threads, for more CTAs of small images.  G-buffer of 64 objects of 512 triangles
+// at 200 x 120, 640 x 360 and 1920 x 1080: 845, 1126 and 3368 us with two pixels, 585, 732
+// and 2661 with one; of one object of 20000 triangles at 200 x 120 10.7 and 5.2 ms.
+template <bool MESH> struct Cast {
+  static constexpr int kPixels = MESH ? 1 : 2, kThreads = MESH ? 128 : 256;
+  static constexpr int kX = 32, kY = kPixels * kThreads / kX;  // pixels of a CTA
+};
 constexpr int kPrimStage = 256;  // primitives staged per shared-memory batch
 constexpr int kOwnPrims = 4;     // of them that a lane bounds at a time
 
@@ -168,13 +177,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return r;
 }
 
-__device__ __forceinline__ RayBounds ray_bounds(const float (&d)[kCastPix][3]) {
+template <int PIX> __device__ __forceinline__ RayBounds ray_bounds(const float (&d)[PIX][3]) {
   RayBounds r;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     float lo = d[0][k], hi = d[0][k];
 #pragma unroll
-    for (int q = 1; q < kCastPix; q++) {
+    for (int q = 1; q < PIX; q++) {
       lo = min_nan(lo, d[q][k]);
       hi = max_nan(hi, d[q][k]);
     }
@@ -281,11 +290,12 @@ __device__ __forceinline__ float prim_hit(const PrimTest& p, f3 d, const float (
 // bit.  Measured with 64 boxes and 16 spheres: the G-buffer at 1920 x 1080 319 -> 53 us, a
 // shadow map of 1024 x 1024 171 -> 20 us (in index order 87 and 35; one pixel a thread and
 // one primitive a lane at a time 67 and 27).
+template <bool MESH, int PIX>
 __device__ __forceinline__ void cast_rays(const gi_prim* __restrict__ prims, int np, const MeshSet& mesh, f3 o,
-                                          const f3 (&d)[kCastPix], Hit (&h)[kCastPix], PrimTest* s_prims) {
-  float iv[kCastPix][3], dv[kCastPix][3];
+                                          const f3 (&d)[PIX], Hit (&h)[PIX], PrimTest* s_prims) {
+  float iv[PIX][3], dv[PIX][3];
 #pragma unroll
-  for (int q = 0; q < kCastPix; q++) {
+  for (int q = 0; q < PIX; q++) {
     h[q].t = kInf;
     h[q].prim = -1;
     h[q].tri = -1;
@@ -297,13 +307,13 @@ __device__ __forceinline__ void cast_rays(const gi_prim* __restrict__ prims, int
 #pragma unroll
     for (int k = 0; k < 3; k++) iv[q][k] = rcp_(dv[q][k]);
   }
-  const RayBounds bounds = ray_bounds(dv);
+  const RayBounds bounds = ray_bounds<PIX>(dv);
   const int lane = threadIdx.x & 31;
   float farthest = kInf;  // of the warp's hits so far
   for (int base = 0; base < np; base += kPrimStage) {
     const int cnt = min(kPrimStage, np - base);
     __syncthreads();
-    for (int i = threadIdx.x; i < cnt; i += kCastThreads) s_prims[i] = prim_test(prims[base + i], o);
+    for (int i = threadIdx.x; i < cnt; i += Cast<MESH>::kThreads) s_prims[i] = prim_test(prims[base + i], o);
     __syncthreads();
     for (int first = 0; first < cnt; first += 32 * kOwnPrims) {
       // Each lane's primitives, 32 apart; the nearest of them and its place.
@@ -333,7 +343,7 @@ __device__ __forceinline__ void cast_rays(const gi_prim* __restrict__ prims, int
         const bool numbers = bounds.closed && (p.kind & kFinite);
         float far = 0.0f;
 #pragma unroll
-        for (int q = 0; q < kCastPix; q++) {
+        for (int q = 0; q < PIX; q++) {
           const float t = numbers ? prim_hit<true>(p, d[q], iv[q]) : prim_hit<false>(p, d[q], iv[q]);
           if (t > 0.0f && (t < h[q].t || (t == h[q].t && prim < h[q].prim))) {
             h[q].t = t;
@@ -345,8 +355,8 @@ __device__ __forceinline__ void cast_rays(const gi_prim* __restrict__ prims, int
       }
     }
   }
-  if (mesh.num_objects > 0)
-    for (int q = 0; q < kCastPix; q++) cast_mesh(mesh, o, d[q], iv[q], h[q]);
+  if (MESH)
+    for (int q = 0; q < PIX; q++) cast_mesh(mesh, o, d[q], iv[q], h[q]);
 }
 
 // The surface normal at the hit of an analytic primitive.
@@ -367,22 +377,22 @@ __device__ __forceinline__ f3 prim_normal(const gi_prim& g, f3 o, f3 d, float t)
 
 // A thread's pixels and rays.  Pixels past the image take its last row or column (they
 // join the warp's votes) and store nothing.
-struct CastPixels {
-  int x, y[kCastPix];
-  bool live[kCastPix];
-  f3 org, dir[kCastPix];
+template <int PIX> struct CastPixels {
+  int x, y[PIX];
+  bool live[PIX];
+  f3 org, dir[PIX];
 };
-__device__ __forceinline__ CastPixels cast_pixels(const ViewArgs& v) {
-  CastPixels c;
+template <bool MESH, int PIX> __device__ __forceinline__ CastPixels<PIX> cast_pixels(const ViewArgs& v) {
+  CastPixels<PIX> c;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int x = blockIdx.x * kCastX + (w & 3) * 8 + (l & 7);
+  const int x = blockIdx.x * Cast<MESH>::kX + (w & 3) * 8 + (l & 7);
   c.x = min(x, v.width - 1);
   const float sx = div_((float)c.x + 0.5f, (float)v.width);
   const float4 o4 = mat_vec(v.inv_view, 0.0f, 0.0f, 0.0f, 1.0f);
   c.org = mk3(o4.x, o4.y, o4.z);
 #pragma unroll
-  for (int q = 0; q < kCastPix; q++) {
-    const int y = blockIdx.y * kCastY + ((w >> 2) * kCastPix + q) * 4 + (l >> 3);
+  for (int q = 0; q < PIX; q++) {
+    const int y = blockIdx.y * Cast<MESH>::kY + ((w >> 2) * PIX + q) * 4 + (l >> 3);
     c.live[q] = x < v.width && y < v.height;
     c.y[q] = min(y, v.height - 1);
     const float sy = div_((float)c.y[q] + 0.5f, (float)v.height);
@@ -454,32 +464,36 @@ __device__ __forceinline__ void shade(const ViewArgs& v, const gi_prim* __restri
   ndc[i] = project(v.view_proj, hit).z;
 }
 
-__global__ void __launch_bounds__(kCastThreads) gbuffer_kernel(const __grid_constant__ ViewArgs v,
+template <bool MESH>
+__global__ void __launch_bounds__(Cast<MESH>::kThreads) gbuffer_kernel(const __grid_constant__ ViewArgs v,
                                                                const gi_prim* __restrict__ prims, int np, MeshSet mesh,
                                                                float* __restrict__ albedo,
                                                                float* __restrict__ emissive,
                                                                float* __restrict__ normal,
                                                                float* __restrict__ moments, float* __restrict__ ndc) {
   __shared__ PrimTest s_prims[kPrimStage];
-  __shared__ __align__(16) float s_colour[kCastThreads / 32][32][8];  // a warp's surfaces: albedo, emissive
-  const CastPixels c = cast_pixels(v);
-  Hit h[kCastPix];
-  cast_rays(prims, np, mesh, c.org, c.dir, h, s_prims);
+  __shared__ __align__(16) float s_colour[Cast<MESH>::kThreads / 32][32][8];  // a warp's surfaces: albedo, emissive
+  constexpr int PIX = Cast<MESH>::kPixels;
+  const CastPixels<PIX> c = cast_pixels<MESH, PIX>(v);
+  Hit h[PIX];
+  cast_rays<MESH, PIX>(prims, np, mesh, c.org, c.dir, h, s_prims);
 #pragma unroll
-  for (int q = 0; q < kCastPix; q++)
+  for (int q = 0; q < PIX; q++)
     shade(v, prims, np, mesh, c.x, c.y[q], c.live[q], c.org, c.dir[q], h[q], s_colour[threadIdx.x >> 5], albedo, emissive,
           normal, moments, ndc);
 }
 
-__global__ void __launch_bounds__(kCastThreads) shadow_kernel(const __grid_constant__ ViewArgs v,
+template <bool MESH>
+__global__ void __launch_bounds__(Cast<MESH>::kThreads) shadow_kernel(const __grid_constant__ ViewArgs v,
                                                               const gi_prim* __restrict__ prims, int np, MeshSet mesh,
                                                               float* __restrict__ out) {
   __shared__ PrimTest s_prims[kPrimStage];
-  const CastPixels c = cast_pixels(v);
-  Hit h[kCastPix];
-  cast_rays(prims, np, mesh, c.org, c.dir, h, s_prims);
+  constexpr int PIX = Cast<MESH>::kPixels;
+  const CastPixels<PIX> c = cast_pixels<MESH, PIX>(v);
+  Hit h[PIX];
+  cast_rays<MESH, PIX>(prims, np, mesh, c.org, c.dir, h, s_prims);
 #pragma unroll
-  for (int q = 0; q < kCastPix; q++) {
+  for (int q = 0; q < PIX; q++) {
     if (!c.live[q]) continue;
     float z = 1.0f;
     if (h[q].prim >= 0 || h[q].tri >= 0) z = project(v.view_proj, add3(c.org, mul3s(c.dir[q], h[q].t))).z;
@@ -542,7 +556,38 @@ __global__ void __launch_bounds__(kTx* kTy) direct_kernel(const __grid_constant_
 }
 
 dim3 grid2d(int w, int h) { return dim3((w + kTx - 1) / kTx, (h + kTy - 1) / kTy); }
-dim3 cast_grid(int w, int h) { return dim3((w + kCastX - 1) / kCastX, (h + kCastY - 1) / kCastY); }
+// go(mesh, grid, threads) with the launch of a cast with or without meshes.
+template <typename Go> void launch_cast(int w, int h, const MeshSet& mesh, Go go) {
+  auto with = [&](auto m) {
+    using C = Cast<decltype(m)::value>;
+    go(m, dim3((w + C::kX - 1) / C::kX, (h + C::kY - 1) / C::kY), C::kThreads);
+  };
+  if (mesh.num_objects > 0) with(std::true_type{});
+  else with(std::false_type{});
+}
+
+int launch_gbuffer(const gi_view& view, const gi_prim* prims, int np, const MeshSet& mesh, float* albedo,
+                   float* emissive, float* normal, float* moments, float* ndc, cudaStream_t stream) {
+  const ViewArgs v = view_args(view);
+  launch_cast(v.width, v.height, mesh, [&](auto m, dim3 grid, int threads) {
+    gbuffer_kernel<decltype(m)::value><<<grid, threads, 0, stream>>>(v, prims, np, mesh, albedo, emissive, normal,
+                                                                     moments, ndc);
+  });
+  GI_CHECK_LAUNCH("gbuffer_kernel");
+  count_launches(1);
+  return GI_OK;
+}
+
+int launch_shadow(const gi_view& view, const gi_prim* prims, int np, const MeshSet& mesh, float* out,
+                  cudaStream_t stream) {
+  const ViewArgs v = view_args(view);
+  launch_cast(v.width, v.height, mesh, [&](auto m, dim3 grid, int threads) {
+    shadow_kernel<decltype(m)::value><<<grid, threads, 0, stream>>>(v, prims, np, mesh, out);
+  });
+  GI_CHECK_LAUNCH("shadow_kernel");
+  count_launches(1);
+  return GI_OK;
+}
 
 }  // namespace
 }  // namespace gi
@@ -556,12 +601,8 @@ extern "C" int gi_gbuffer(const gi_view* view, const gi_prim* prims, int num_pri
   GI_CHECK_ARG(view->width >= 1 && view->height >= 1, "gi_gbuffer: bad viewport");
   GI_CHECK_ARG(aligned16(albedo) && aligned16(emissive) && aligned16(normal) && aligned16(depth_moments),
                "gi_gbuffer: unaligned buffer");
-  ViewArgs v = view_args(*view);
-  gbuffer_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
-      v, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, albedo, emissive, normal, depth_moments, ndc_depth);
-  GI_CHECK_LAUNCH("gbuffer_kernel");
-  count_launches(1);
-  return GI_OK;
+  return launch_gbuffer(*view, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, albedo, emissive, normal,
+                        depth_moments, ndc_depth, (cudaStream_t)stream);
 }
 
 static int check_mesh(const gi_prim* prims, int num_prims, const gi_mesh_object* objects, int num_objects,
@@ -585,12 +626,8 @@ extern "C" int gi_gbuffer_mesh(const gi_view* view, const gi_prim* prims, int nu
   GI_CHECK_ARG(view->width >= 1 && view->height >= 1, "gi_gbuffer_mesh: bad viewport");
   GI_CHECK_ARG(aligned16(albedo) && aligned16(emissive) && aligned16(normal) && aligned16(depth_moments),
                "gi_gbuffer_mesh: unaligned buffer");
-  ViewArgs v = view_args(*view);
-  gbuffer_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
-      v, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, albedo, emissive, normal, depth_moments, ndc_depth);
-  GI_CHECK_LAUNCH("gbuffer_kernel");
-  count_launches(1);
-  return GI_OK;
+  return launch_gbuffer(*view, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, albedo, emissive, normal,
+                        depth_moments, ndc_depth, (cudaStream_t)stream);
 }
 
 extern "C" int gi_shadow_map_mesh(const gi_view* light_view, const gi_prim* prims, int num_prims,
@@ -600,24 +637,15 @@ extern "C" int gi_shadow_map_mesh(const gi_view* light_view, const gi_prim* prim
   int st = check_mesh(prims, num_prims, objects, num_objects, tris, num_tris, "gi_shadow_map_mesh: bad scene arrays");
   if (st) return st;
   GI_CHECK_ARG(cull == GI_CULL_NONE || cull == GI_CULL_BACK, "gi_shadow_map_mesh: unknown cull mode");
-  ViewArgs v = view_args(*light_view);
-  shadow_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
-      v, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, shadow);
-  GI_CHECK_LAUNCH("shadow_kernel");
-  count_launches(1);
-  return GI_OK;
+  return launch_shadow(*light_view, prims, num_prims, MeshSet{objects, tris, num_objects, cull}, shadow,
+                       (cudaStream_t)stream);
 }
 
 extern "C" int gi_shadow_map(const gi_view* light_view, const gi_prim* prims, int num_prims, float* shadow,
                              void* stream) {
   GI_CHECK_ARG(light_view && prims && shadow, "gi_shadow_map: null");
   GI_CHECK_ARG(num_prims >= 1 && num_prims <= GI_MAX_PRIMS, "gi_shadow_map: bad primitive count");
-  ViewArgs v = view_args(*light_view);
-  shadow_kernel<<<cast_grid(v.width, v.height), kCastThreads, 0, (cudaStream_t)stream>>>(
-      v, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, shadow);
-  GI_CHECK_LAUNCH("shadow_kernel");
-  count_launches(1);
-  return GI_OK;
+  return launch_shadow(*light_view, prims, num_prims, MeshSet{nullptr, nullptr, 0, 0}, shadow, (cudaStream_t)stream);
 }
 
 extern "C" int gi_direct_light(const gi_view* view, const gi_view* light_view, const float* albedo,
