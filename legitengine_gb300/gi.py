@@ -197,28 +197,23 @@ def _torch():
 # up to 20 images, and was bound by building their arguments (an import and a ctypes
 # object each, a stream object a call): 89 us a pass, now 47, about its kernels' time.
 _float32 = None
-_raw_stream = None
+_current_handle = None  # () -> the current stream's handle, once torch's CUDA side is up
 
 
 def _stream() -> int:
     """The current stream's handle."""
-    if _raw_stream is None:
-        return _first_stream()
-    return _raw_stream(_device())
+    return _first_stream() if _current_handle is None else _current_handle()
 
 
 def _first_stream() -> int:
     """Initialises torch's CUDA side, after which the handle can be asked for by itself."""
-    global _raw_stream, _device
+    global _current_handle
     torch = _torch()
     handle = torch.cuda.current_stream().cuda_stream
     raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
     if raw is not None and dev is not None:
-        _raw_stream, _device = raw, dev
+        _current_handle = lambda: raw(dev())  # one assignment: other threads see nothing or all of it
     return handle
-
-
-_device = None
 
 
 def _ptr(t) -> int:
