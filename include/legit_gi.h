@@ -230,11 +230,11 @@ GI_API int gi_march_tiles(const gi_view* view, const gi_march_params* params,
  * `out`) and records the fastest for this march shape (width, height, dirs,
  * step_dirs, step_cap, precision); later gi_march calls of the same shape use it.
  * The layouts, all with the same result bit for bit:
- *   one thread per pixel, CTAs of 2, 4 or 8 rows of 32 pixels (the tile shape
+ *   one thread per pixel, CTAs of 32 x 2, 4 or 8 pixels (the tile shape
  *     of the launch): a warp marches 32 pixels x all `dirs` directions;
  *   four threads per pixel (the direction split; 4 <= dirs <= 32): each thread
  *     marches every fourth direction of its pixel, a warp 32 pixels x
- *     ceil(dirs / 4) directions, CTAs of one 32-pixel row.
+ *     ceil(dirs / 4) directions, CTAs of one warp's 32 pixels.
  * best_rows, best_rays_per_warp (32 x the directions a thread marches) and
  * best_ms (optional, host) receive the choice and its time per launch. */
 GI_API int gi_march_autotune(const gi_view* view, const gi_march_params* params,

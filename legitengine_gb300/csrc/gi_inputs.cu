@@ -1,9 +1,9 @@
 // gi_inputs.cu -- the passes that feed the GI path (SSVGIRenderer.h:61-205):
 // G-buffer, shadow map and direct light.  The reference rasterises meshes; here
-// the scene is ray cast through the pixel centres, one thread per pixel: those of the
+// the scene is ray cast through the pixel centres, two pixels a thread: those of the
 // procedural primitives (boxes and spheres inside a room) that the bounds of a warp's
-// rays meet, then the triangle meshes of a loaded scene, object by object behind a
-// bounds test.
+// rays meet; with the triangle meshes of a loaded scene one pixel a thread, those after
+// the primitives, object by object behind a bounds test.
 #include <type_traits>
 
 #include "gi_device.cuh"

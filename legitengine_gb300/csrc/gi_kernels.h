@@ -66,8 +66,8 @@ struct MarchArgs {
   float* rec_hc;                      // [direction][step][record pixel]: hc of the steps that raised the horizon
   unsigned long long* rec_mask;       // [direction][record pixel]: bit s set = step s raised the horizon
   float* rec_hc0;                     // [direction][record pixel]
-  // (record pixel: the interleaved (pattern, sub-image row, column) index, so that a
-  // warp's 32 pixels are consecutive)
+  // (record pixel: the interleaved (pattern, sub-image row, column) index, in which the
+  // pixels of a warp are a few runs; the offsets are in gi_record.h)
   int rec;                            // 0: march; 1: march and record; 2: replay the record over `light`
   int rec_steps;                      // step stride of rec_hc, >= the step table size (<= 64)
   // Fast standard form only (GI_MARCH_TEXTURE): texture objects over the depth
@@ -105,7 +105,7 @@ class PyramidTexture {
   int w_ = 0, h_ = 0, levels_ = 0, channels_ = 0;
 };
 
-constexpr int kMarchTileSubX = 32;  // sub-image pixels per march CTA along x (one warp row)
+constexpr int kMarchTileSubX = 32;  // sub-image pixels per march CTA along x
 constexpr int kMarchTileSubY = 4;   // sub-image rows per march CTA
 
 int launch_march(const MarchArgs& a, cudaStream_t stream);

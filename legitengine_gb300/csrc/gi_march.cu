@@ -5,11 +5,11 @@
 // (x mod 4, y mod 4) selects the Hammersley offsets (:155-164), and with them
 // the directions and every step offset and mip level of the pixel.  Here a CTA
 // takes pixels of ONE pattern (the interleaved form of LSGIRenderer.h:83-91
-// without materialising deinterleaved copies): blockIdx.z is the pattern, and
-// a warp covers 32 pixels of one row, 4 pixels apart.  All lanes of a warp then
-// march the same directions with the same step offsets, so the per-step tables
-// (offset, mip pair, blend weight) are warp-uniform shared-memory broadcasts,
-// and the taps of neighbouring lanes land on neighbouring texels.
+// without materialising deinterleaved copies): the pattern is blockIdx.x modulo
+// P^2, and a warp covers 8 x 4 pixels of it, P pixels apart (tile_place).  All lanes
+// of a warp then march the same directions with the same step offsets, so the
+// per-step tables (offset, mip pair, blend weight) are warp-uniform shared-memory
+// broadcasts, and the taps of neighbouring lanes land on neighbouring texels.
 //
 // Arithmetic mirrors the restatement exactly (see gi_device.cuh): the output is
 // bit-identical to the fp32 oracle for the same inputs.
@@ -209,12 +209,12 @@ __device__ __forceinline__ float soft_horizon(float dmean, float dsq, f3 rn, f3 
   return max_h - (d * cdf + sigma * pdf);
 }
 
-// Shared-memory tables of one CTA-tile: n_tab steps, R directions and the
-// levels' sizes (float(width >> l), float(height >> l)), laid out in that order
-// in march_smem_bytes(n_tab, R) bytes.  The single-view kernels take exactly that
-// as dynamic shared memory, so the unified L1/shared storage left to L1 does not
-// shrink for the tables' maxima (GI_MAX_STEPS steps, GI_MAX_DIRS directions: 10 KB
-// a CTA, against 0.6 KB for 22 steps and 16 directions).
+// Shared-memory tables of one CTA-tile: n_tab steps and R directions, laid out in
+// that order in march_smem_bytes(n_tab, R) bytes.  The single-view kernels take exactly
+// that as dynamic shared memory, so the unified L1/shared storage left to L1 does not
+// shrink for the tables' maxima (GI_MAX_STEPS steps and GI_MAX_DIRS directions with
+// software taps: 36 KB a CTA; 22 steps and 16 directions: 1.6 KB, with texture taps
+// 0.4 KB).
 template <bool TEX> struct MarchSmem {
   typename StepOf<TEX>::T* step;
   float4* dir;  // cos, sin and their reciprocals (rcp_)
@@ -234,7 +234,7 @@ static_assert(march_smem_bytes<false>(GI_MAX_STEPS, GI_MAX_DIRS) <= 47 * 1024 &&
               "march tables");
 
 // The replay's tables: a record holds at most 64 steps (its step mask), so the
-// replay keeps fixed-size tables for that many (6 KB) -- constant offsets in its
+// replay keeps fixed-size tables for that many (8 KB) -- constant offsets in its
 // per-hit table reads, which the pointer layout above cost it 3 %.
 constexpr int kRecMaxSteps = 64;
 struct ReplaySmem {
@@ -385,11 +385,11 @@ template <int KY, bool TEX> __device__ __forceinline__ int2 tile_place(int tid) 
 // Shared by the full-frame, tile-list and batched kernels; every thread of the
 // CTA calls it (it contains one CTA barrier).
 //
-// SPLIT > 1 (the direction-split form for short tile lists): the CTA takes one
-// warp's pixels of the tile (`row` of its 4 warps), thread (x, s) marches pixel x's directions s, s + SPLIT,
-// ..., stores each direction's term in `contrib` (at most kSplitMaxDirs
-// directions), and after a barrier thread (x, 0) adds the terms in direction
-// order -- the same sum, in the same order, as one thread marching them all.
+// SPLIT > 1 (the direction split, for short tile lists and small frames): the CTA
+// takes one warp's pixels of the tile (`row` of its 4 warps), thread (x, s) marches
+// pixel x's directions s, s + SPLIT, ..., stores each direction's term in `contrib`
+// (at most kSplitMaxDirs directions), and after a barrier thread (x, 0) adds the terms
+// in direction order -- the same sum, in the same order, as one thread marching them all.
 //
 // REC (the standard form only): also record, per pixel and direction, which steps
 // raised the horizon and their horizon contributions hc, plus the direction's
@@ -461,8 +461,8 @@ __device__ __forceinline__ void march_tile(const MarchArgs& a, int n_tab, int pa
   float c0, s0;
   sincosf_(2.0f * 0.0f, &s0, &c0);
 
-  // Records are indexed in the interleaved (pattern, sub-image row, column) order,
-  // in which a warp's 32 pixels are consecutive: coalesced stores and loads.
+  // Records are indexed in the interleaved (pattern, sub-image row, column) order, in
+  // which a warp's pixels are 4 runs of 8 (in tiles of two rows 2 of 16): whole sectors.
   const unsigned npix = (unsigned)record_pixels(a.width, a.height, a.pattern);
   const unsigned rec_idx = ((unsigned)pat * ((a.height + P - 1) / P) + j) * ((a.width + P - 1) / P) + i;
   Light sum{pk(0.0f), 0.0f};

@@ -64,7 +64,8 @@ constexpr int kTcThreads = 128 * kGroups;
 constexpr uint32_t cA = 64, kGroupCols = cA + kHid / 2, cOnes = kGroupCols * kGroups, kOnesCols = 8, kTmemCols = 512;
 static_assert(cOnes + 4 * kOnesCols <= kTmemCols, "tensor memory");
 
-// Shared memory (bytes).  B operands are the weights as N x K (K-major).
+// Shared memory (bytes).  B operands: the weights, inputs x outputs and read MN-major
+// (kBRows); the bias operand alone is K-major.
 constexpr int tB1 = 0;                            // 32 x 64 (inputs x outputs)
 constexpr int tB2 = tB1 + kHid * kIn * 2;         // 64 x 64
 constexpr int tB3 = tB2 + kHid * kHid * 2;        // 64 x 64
