@@ -197,12 +197,13 @@ def _torch():
 # up to 20 images, and was bound by building their arguments (an import and a ctypes
 # object each, a stream object a call): 89 us a pass, now 47, about its kernels' time.
 _float32 = None
-_current_handle = None  # () -> the current stream's handle, once torch's CUDA side is up
+_current_handle = None  # what gives the current stream's handle, once torch's CUDA side is up
 
 
 def _stream() -> int:
     """The current stream's handle."""
-    return _first_stream() if _current_handle is None else _current_handle()
+    current = _current_handle
+    return _first_stream() if current is None else current[0](current[1]())
 
 
 def _first_stream() -> int:
@@ -212,7 +213,7 @@ def _first_stream() -> int:
     handle = torch.cuda.current_stream().cuda_stream
     raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
     if raw is not None and dev is not None:
-        _current_handle = lambda: raw(dev())  # one assignment: other threads see nothing or all of it
+        _current_handle = (raw, dev)  # one assignment: other threads see nothing or all of it
     return handle
 
 
