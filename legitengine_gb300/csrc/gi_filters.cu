@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kTx* kTy) bilateral_fast_kernel(const float* _
 // its other 12 from the pixels before it.  The tile's height keeps the block within 48
 // KB; 8 and 14 rows measured 217 and 209 us against 209 with 12 before the last columns
 // of all rows became one warp's.  3840 x 2160: 315 us with scalar weights per tap, 235
-// with packed ones, 206 shared; bound by shared memory's accesses (85 % busy) now.
+// with packed ones, 206 shared; bound by L1's data pipe (82 % busy, shared memory 70 %) now.
 constexpr int kExY = 6;                        // rows of threads
 constexpr int kExTile = kExY * kBilRows;       // rows of outputs
 constexpr int kExHy = kExTile + 4, kExWy = kExTile + 2;  // rows of the halo, and of weights

@@ -718,7 +718,7 @@ __device__ __forceinline__ void march_replay_tile(const MarchArgs& a, int n_tab,
     const float* const rec_rows = a.rec_hc + record_block(d, a.rec_steps, npix) + rec_idx;
     Light dl{pk(ambient * hc0), ambient * hc0};
     // The steps that any lane hit, in order, the lanes together: a step's lanes read
-    // neighbouring texels of the same levels.  Bound by L1's data pipe (70 % busy; 90 %
+    // neighbouring texels of the same levels.  Bound by L1's data pipe (66 % busy; 90 %
     // with each lane at its own next hit): 1520 -> 1321 us at 1920 x 1080, R = 16.
     // Reading the record a step or a direction ahead gave nothing (1352, 1317 us).
     unsigned long long left = (unsigned long long)__reduce_or_sync(lanes, (unsigned)(hits >> 32)) << 32 |
