@@ -188,9 +188,9 @@ __device__ __forceinline__ f3 funproject(const Mat4& inv, float sx, float sy, fl
 }
 // The hardware's approximate division and reciprocal square root without the
 // scaling that subnormal operands would need: those count as 0.  In the step loop that
-// is a sample within 1e-19 of the pixel's point (its |h|^2) or a view ray as short; with
-// the scaling, whose quotients overflow there in part, frames took 2 to 3 % longer
-// (1283 x 721, R = 12: 1110 against 1139 us).
+// is a sample within 1e-19 of the pixel's point (its |h|^2); with the scaling, whose
+// quotients overflow there in part, frames took 2 to 3 % longer (1283 x 721, R = 12:
+// 1110 against 1139 us).
 __device__ __forceinline__ float div_approx(float a, float b) {
   float r;
   asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));

@@ -14,6 +14,7 @@
 // Arithmetic mirrors the restatement exactly (see gi_device.cuh): the output is
 // bit-identical to the fp32 oracle for the same inputs.
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -1023,6 +1024,9 @@ int PyramidTexture::Pack(const float* const* levels, int src_channels, cudaStrea
 // for the constant part of V.w: that is the fp32 sum m[11] + m[15] that the exact
 // unprojection computes (a cancelling sum for a far plane, 1 / far), so that both
 // precisions scale the far-plane point alike and the fast rays track the exact ones.
+// The step loop uses U's direction and V.w's sign alone, so both are scaled by one power
+// of two, U to about 1: the same bits, and no squared length below the normal range (which
+// the loop's square root counts as 0) for a matrix of any homogeneous scale.
 void set_ray_basis(MarchArgs& a) {
   const float* m = a.inv_view_proj.m;
   const float* iv = a.inv_view.m;
@@ -1033,7 +1037,8 @@ void set_ray_basis(MarchArgs& a) {
   for (int r = 0; r < 4; r++) a.far_col[r] = m[8 + r] * 1.0f + m[12 + r] * 1.0f;
   const double cam[3] = {a.inv_view.m[12], a.inv_view.m[13], a.inv_view.m[14]};
   const float w_far = m[11] + m[15];
-  double U[3][3];  // A, B, C: the ray's constant part and its derivatives in sx, sy
+  double U[3][3], V[3];  // A, B, C: the ray's constant part and its derivatives in sx, sy; of V.w
+  double largest = 0.0;
   for (int part = 0; part < 3; part++) {
     double v[4];
     for (int r = 0; r < 4; r++) {
@@ -1043,9 +1048,15 @@ void set_ray_basis(MarchArgs& a) {
     if (part == 0) v[3] = (double)w_far - (double)m[3] - (double)m[7];
     for (int r = 0; r < 3; r++) {
       U[part][r] = v[r] - cam[r] * v[3];
-      a.ray[4 * part + r] = (float)U[part][r];
+      largest = std::max(largest, std::fabs(U[part][r]));
     }
-    a.ray[4 * part + 3] = (float)v[3];
+    V[part] = v[3];
+  }
+  int exponent = 0;
+  if (largest > 0.0 && std::isfinite(largest)) std::frexp(largest, &exponent);
+  for (int part = 0; part < 3; part++) {
+    for (int r = 0; r < 3; r++) a.ray[4 * part + r] = (float)(U[part][r] = std::ldexp(U[part][r], -exponent));
+    a.ray[4 * part + 3] = (float)std::ldexp(V[part], -exponent);
   }
   // |U|^2 = |A + sx B + sy C|^2 = q0 + sx (q1 + sx q3) + sy (q2 + sx q4 + sy q5).
   auto dot = [&](int i, int j) { return U[i][0] * U[j][0] + U[i][1] * U[j][1] + U[i][2] * U[j][2]; };
